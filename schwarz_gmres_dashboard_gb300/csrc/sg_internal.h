@@ -293,23 +293,51 @@ struct SubInfo {
 // level -- a fixed stride apart in a box subdomain -- fall in distinct banks.
 __host__ __device__ __forceinline__ int tslot(int r, int p) { return p ? r + (r >> p) : r; }
 
+// Level records of the TMA-fed sweep.  Rows of 2, 3 or 4 nonzeros per triangle
+// are stored as row structs (when the preconditioner's rec_rows is set): the
+// row's and the columns' slots (16 bits each), the values, and in the backward
+// sweep the diagonal's reciprocal (FP32, also beside BF16 values; FP64 sweeps
+// hold the reciprocal and the diagonal).  After a level's rows comes one that
+// computes t = 0 in the unused slot: the lanes past the level's end take it.
+// The sizes are multiples of 4 (FP64:
+// 8) bytes whose strides spread a warp over the shared-memory banks, hence
+// the last column: a stride of 32 or 64 bytes would not.
+//   bytes    W = 2     3      4
+//   BF16     12, 16  16, 20  20, 24    (forward, backward)
+//   FP32     16, 20  20, 24  28, 36
+//   FP64     24, 40  40, 48  48, 72
+__host__ __device__ constexpr bool rec_is_rows(int w) { return w >= 2 && w <= 4; }
+__host__ __device__ constexpr int rec_val_off(int w, int sf) {
+    return (2 * (1 + w) + sf - 1) / sf * sf;
+}
+__host__ __device__ constexpr int rec_recip_off(int w, int sf) {
+    return (rec_val_off(w, sf) + w * sf + 3) / 4 * 4;
+}
+__host__ __device__ constexpr int rec_row_bytes(int w, bool back, int sf) {
+    const int b = back ? rec_recip_off(w, sf) + (sf == 8 ? 16 : 4) : rec_recip_off(w, sf);
+    return b % 32 == 0 ? b + (sf == 8 ? 8 : 4) : b;
+}
+
 // One way of streaming the level records through the TMA-fed sweep's
 // shared-memory ring: its size, the largest group of records copied at once,
-// the block size, whether CTAs loop over subdomains (persistent: grid CTAs
-// take subdomains from a work counter, largest first) and the static
-// schedule -- per subdomain (sub: RingSub records as bytes), per level (meta:
-// int4 as four ints), per record group (grp: int2 as two ints).
+// the block size and how many of its threads work on the levels, whether CTAs
+// loop over subdomains (persistent: grid CTAs take subdomains from a work
+// counter, largest first) and the static schedule -- per subdomain (sub:
+// RingSub records as bytes), per pass over a level (ent: int2 as two ints),
+// per record group (grp: int4 as four ints).
 struct RingPlan {
     int R = 1;                 // right-hand sides interleaved in the shared vector
     bool ready = false;
     long long ring_bytes = 0;
     long long gmax = 0;
     int threads = 0;
+    int level_threads = 0;     // the first of them (whole warps) run the level loop
+    int max_ent = 0, max_grp = 0;  // largest counts of one subdomain
     int grid = 0;              // CTAs of a persistent launch (0: one CTA per subdomain)
     std::vector<unsigned char> sub;
-    std::vector<int> meta, grp;
+    std::vector<int> ent, grp;
     DBuf<unsigned char> sub_d;
-    DBuf<int> meta_d, grp_d;
+    DBuf<int> ent_d, grp_d;
     DBuf<unsigned> work;       // persistent launches: next subdomain, CTAs done
 };
 
@@ -339,7 +367,6 @@ struct sg_precond {
     long long fl_total = 0, fu_total = 0;
     int max_n = 0;
     int t_len = 0;       // TMA sweep: largest tslot(n_s, tshift_s) + 1
-    int max_levels = 0;  // largest nlev_f + nlev_b of a subdomain
     long long total_rows = 0;
     bool use_smem = true;
     // level records for the TMA-fed sweep: per level one 16-byte-aligned
@@ -347,6 +374,7 @@ struct sg_precond {
     bool use_rec = false;
     bool use_sf = false;   // sync-free sweep (per-row ready flags)
     int rec_depth = 0;               // 1 when the TMA-fed sweep is set up (0: not used)
+    bool rec_rows = true;            // row structs for levels of width 2 to 4 (rec_layout)
     // how the level records stream through the sweep's shared-memory ring,
     // for one right-hand side at a time (ring1) and for four interleaved ones
     // (ring4, planned when a batched solve first asks for it)
@@ -405,3 +433,20 @@ struct sg_precond {
     sg::PinnedBuf<double> h_in, h_out;  // n doubles each (FP32 data uses the front)
     sg::PinnedBuf<HostCtl> h_ctl;
 };
+
+namespace sg {
+// bytes of a factor value in the level records
+inline int rec_value_bytes(const sg_precond* pc) {
+    return pc->opts.sweep_dtype == SG_FP64 ? 8 : (pc->opts.factor_dtype == SG_BF16 ? 2 : 4);
+}
+// bytes of the record of a level of c rows, w nonzeros each
+inline long long rec_level_bytes(const sg_precond* pc, int w, bool back, int c) {
+    const int sf = rec_value_bytes(pc);
+    if (pc->rec_rows && rec_is_rows(w))
+        return ((long long)(c + 1) * rec_row_bytes(w, back, sf) + 15) & ~15ll;
+    const long long C = (c + 7) & ~7;
+    return C * (2 + w * (2 + sf) + (back ? sf : 0));
+}
+// places the level records of every subdomain (setup.cpp)
+void rec_layout(sg_precond* pc, bool row_structs);
+}  // namespace sg

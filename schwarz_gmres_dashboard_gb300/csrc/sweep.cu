@@ -7,11 +7,14 @@
 // run level by level: rows of one level are independent and a __syncthreads
 // separates levels.
 //
-// A level's factor data is one contiguous, 16-byte-aligned record
+// A level's factor data is one contiguous, 16-byte-aligned record.  Rows with
+// 2, 3 or 4 nonzeros per triangle (the 5-, 7- and 9-point stencils) are row
+// structs [row slot, w column slots u16 | w values (| reciprocal diagonal)];
+// other widths are stored by component,
 //   [row slot u16 x C][column slot u16 x C x w][value x C x w](diagonal x C)
-// (C = rows rounded up to 8; a slot is the row's place in the shared-memory
+// (C = rows rounded up to 8).  A slot is the row's place in the shared-memory
 // vector, tslot, whose per-subdomain padding keeps the rows of a level in
-// distinct banks).  A subdomain's records form one stream (forward levels,
+// distinct banks.  A subdomain's records form one stream (forward levels,
 // then backward) that flows through a shared-memory byte ring in groups of
 // whole levels: the block's last thread copies a group with one
 // cp.async.bulk tracked by an mbarrier, as far ahead as the ring allows (at
@@ -99,44 +102,9 @@ __device__ __forceinline__ void sts(uint32_t a, double v) {
     asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
-// The rows of one level record with W nonzeros per row (W fixed: the 5-, 7-
-// and 9-point stencils give 2, 3 and 4).  Record at shared address R:
-//   rows u16[C] | columns u16[W][C] | values TF[W][C] | (diagonal TF[C]).
-// A row computes acc = t[r]; acc -= v_k t[c_k] for k = 0..W-1 in order;
-// backward: acc /= d -- every load of the row issued before the first
-// multiply-add.  Row and column entries are shared-memory slots of t
-// (tslot); padding entries hold the slot of row n, where t is 0, and value 0.
-template <int W, bool BACK, class TS, class TF, bool EXACT>
-__device__ __forceinline__ void level_rows_w(uint32_t tb, uint32_t R, int C, int c, int nthreads) {
-    constexpr uint32_t SF = sizeof(TF), ST = sizeof(TS);
-    const uint32_t cstride = 2u * (uint32_t)C;
-    const uint32_t vbase = R + cstride * (uint32_t)(1 + W);
-    const uint32_t vstride = SF * (uint32_t)C;
-    for (int q = threadIdx.x; q < c; q += nthreads) {
-        const uint32_t rq = R + 2u * (uint32_t)q;
-        const uint32_t vq = vbase + SF * (uint32_t)q;
-        const uint32_t r = lds_u16(rq);
-        uint32_t ck[W];
-        TF vk[W];
-#pragma unroll
-        for (int k = 0; k < W; ++k) ck[k] = lds_u16(rq + cstride * (uint32_t)(k + 1));
-#pragma unroll
-        for (int k = 0; k < W; ++k) vk[k] = lds<TF>(vq + vstride * (uint32_t)k);
-        TF dg{};
-        if (BACK) dg = lds<TF>(vq + vstride * (uint32_t)W);
-        TS acc = lds<TS>(tb + ST * r);
-        TS xk[W];
-#pragma unroll
-        for (int k = 0; k < W; ++k) xk[k] = lds<TS>(tb + ST * ck[k]);
-#pragma unroll
-        for (int k = 0; k < W; ++k) acc = sub_mul<TS, EXACT>(acc, Load<TS>::f(vk[k]), xk[k]);
-        if (BACK) acc = div_diag(acc, Load<TS>::f(dg));
-        sts(tb + ST * r, acc);
-    }
-}
-
-// Any width w: the same row computation through generic pointers, the loads
-// of four nonzeros at a time.
+// Records stored by component, any width w: a row computes acc = t[r]; acc -=
+// v_k t[c_k] for k = 0..w-1 in order; backward: acc /= d.  The loads of four
+// nonzeros at a time.
 template <class TS, class TF, bool EXACT>
 __device__ __forceinline__ void level_rows_any(TS* t, const unsigned char* R, int C, int c,
                                                int w, bool back, int nthreads) {
@@ -167,32 +135,68 @@ __device__ __forceinline__ void level_rows_any(TS* t, const unsigned char* R, in
     }
 }
 
-// One level: the fixed-width row code for w = 2, 3, 4, else the generic one
-// (t / t_s: the subdomain vector as generic pointer / shared address; R /
-// R_s: the level record likewise).
-template <class TS, class TF, bool EXACT>
-__device__ __forceinline__ void level_rows(TS* t, uint32_t t_s, const unsigned char* R,
-                                           uint32_t R_s, int C, int c, int w, bool back,
-                                           int nthreads) {
-    switch (w) {
-    case 2:
-        if (back) level_rows_w<2, true, TS, TF, EXACT>(t_s, R_s, C, c, nthreads);
-        else level_rows_w<2, false, TS, TF, EXACT>(t_s, R_s, C, c, nthreads);
-        return;
-    case 3:
-        if (back) level_rows_w<3, true, TS, TF, EXACT>(t_s, R_s, C, c, nthreads);
-        else level_rows_w<3, false, TS, TF, EXACT>(t_s, R_s, C, c, nthreads);
-        return;
-    case 4:
-        if (back) level_rows_w<4, true, TS, TF, EXACT>(t_s, R_s, C, c, nthreads);
-        else level_rows_w<4, false, TS, TF, EXACT>(t_s, R_s, C, c, nthreads);
-        return;
-    default:
-        level_rows_any<TS, TF, EXACT>(t, R, C, c, w, back, nthreads);
+// Factored local CSR (FP64, reference layout) -> level records of type TF.
+template <class TF>
+__device__ __forceinline__ void put_recip(unsigned char* p, double d);
+template <>
+__device__ __forceinline__ void put_recip<double>(unsigned char* p, double d) {
+    reinterpret_cast<double*>(p)[0] = 1.0 / d;
+    reinterpret_cast<double*>(p)[1] = d;
+}
+template <>
+__device__ __forceinline__ void put_recip<float>(unsigned char* p, double d) {
+    *reinterpret_cast<float*>(p) = 1.0f / to_factor<float>(d);
+}
+template <>
+__device__ __forceinline__ void put_recip<uint16_t>(unsigned char* p, double d) {
+    *reinterpret_cast<float*>(p) = 1.0f / bf16_to_f(to_factor<uint16_t>(d));
+}
+
+// One level's record: the c rows of perm, then padding (component records up
+// to C rows; row structs: the row that computes 0 in the unused slot).
+template <class TF, bool BACK>
+__device__ __forceinline__ void pack_level(const SubInfo& inf, const int* rp, const int* ci,
+                                           const int* dg, const double* v, const uint16_t* perm,
+                                           int c, int C, int w, bool rows, unsigned char* R) {
+    constexpr int SF = (int)sizeof(TF);
+    const uint16_t zero = (uint16_t)tslot(inf.n, inf.tshift);
+    const int rb = rec_row_bytes(w, BACK, SF), vo = rec_val_off(w, SF);
+    uint16_t* rr = reinterpret_cast<uint16_t*>(R);
+    uint16_t* cc = rr + C;
+    TF* vv = reinterpret_cast<TF*>(cc + (size_t)C * w);
+    for (int q = threadIdx.x; q < (rows ? c + 1 : C); q += blockDim.x) {
+        const int r = q < c ? perm[q] : 0;
+        unsigned char* P = R + (size_t)q * rb;
+        auto col = [&](int k) -> uint16_t& {
+            return rows ? reinterpret_cast<uint16_t*>(P)[1 + k] : cc[(size_t)k * C + q];
+        };
+        auto val = [&](int k) -> TF& {
+            return rows ? reinterpret_cast<TF*>(P + vo)[k] : vv[(size_t)k * C + q];
+        };
+        (rows ? reinterpret_cast<uint16_t*>(P)[0] : rr[q]) =
+            q < c ? (uint16_t)tslot(r, inf.tshift) : (rows ? zero : (uint16_t)0);
+        int k = 0;
+        if (q < c) {
+            for (int e = BACK ? dg[r] + 1 : rp[r]; e < rp[r + 1] && k < w; ++e) {
+                const int cl = ci[e];
+                if (!BACK && cl >= r) break;
+                col(k) = (uint16_t)tslot(cl, inf.tshift);
+                val(k) = to_factor<TF>(v[e]);
+                ++k;
+            }
+        }
+        for (; k < w; ++k) {
+            col(k) = zero;
+            val(k) = to_factor<TF>(0.0);
+        }
+        if (BACK) {
+            const double d = q < c ? v[dg[r]] : 1.0;
+            if (rows) put_recip<TF>(P + rec_recip_off(w, SF), d);
+            else (vv + (size_t)C * w)[q] = to_factor<TF>(d);
+        }
     }
 }
 
-// Factored local CSR (FP64, reference layout) -> level records of type TF.
 template <class TF>
 __global__ void __launch_bounds__(256)
 k_pack_rec(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
@@ -201,68 +205,22 @@ k_pack_rec(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
            const uint16_t* __restrict__ perm_b, const int* __restrict__ lev_f,
            const int* __restrict__ lev_b, const long long* __restrict__ off_f,
            const long long* __restrict__ off_b, const int* __restrict__ rows_f,
-           const int* __restrict__ rows_b, unsigned char* rec) {
+           const int* __restrict__ rows_b, int row_structs, unsigned char* rec) {
     const SubInfo inf = info[blockIdx.x];
     const int* rp = lrp + inf.csr_row_off;
     const int* ci = lci + inf.csr_nz_off;
     const double* v = lu + inf.csr_nz_off;
     const int* dg = ldiag + inf.row_off;
+    const bool sf = row_structs && rec_is_rows(inf.wl), sb = row_structs && rec_is_rows(inf.wu);
     for (int l = 0; l < inf.nlev_f; ++l) {
-        const int p0 = lev_f[inf.lev_off_f + l], c = lev_f[inf.lev_off_f + l + 1] - p0;
-        const int C = rows_f[inf.lev_off_f + l];
-        unsigned char* R = rec + off_f[inf.lev_off_f + l];
-        uint16_t* rr = reinterpret_cast<uint16_t*>(R);
-        uint16_t* cc = rr + C;
-        TF* vv = reinterpret_cast<TF*>(cc + (size_t)C * inf.wl);
-        for (int q = threadIdx.x; q < C; q += blockDim.x) {
-            int k = 0;
-            if (q < c) {
-                const int r = perm_f[inf.row_off + p0 + q];
-                rr[q] = (uint16_t)tslot(r, inf.tshift);
-                for (int e = rp[r]; e < rp[r + 1] && k < inf.wl; ++e) {
-                    const int col = ci[e];
-                    if (col >= r) break;
-                    cc[(size_t)k * C + q] = (uint16_t)tslot(col, inf.tshift);
-                    vv[(size_t)k * C + q] = to_factor<TF>(v[e]);
-                    ++k;
-                }
-            } else {
-                rr[q] = 0;
-            }
-            for (; k < inf.wl; ++k) {
-                cc[(size_t)k * C + q] = (uint16_t)tslot(inf.n, inf.tshift);
-                vv[(size_t)k * C + q] = to_factor<TF>(0.0);
-            }
-        }
+        const int i = inf.lev_off_f + l, p0 = lev_f[i];
+        pack_level<TF, false>(inf, rp, ci, dg, v, perm_f + inf.row_off + p0, lev_f[i + 1] - p0,
+                              rows_f[i], inf.wl, sf, rec + off_f[i]);
     }
     for (int l = 0; l < inf.nlev_b; ++l) {
-        const int p0 = lev_b[inf.lev_off_b + l], c = lev_b[inf.lev_off_b + l + 1] - p0;
-        const int C = rows_b[inf.lev_off_b + l];
-        unsigned char* R = rec + off_b[inf.lev_off_b + l];
-        uint16_t* rr = reinterpret_cast<uint16_t*>(R);
-        uint16_t* cc = rr + C;
-        TF* vv = reinterpret_cast<TF*>(cc + (size_t)C * inf.wu);
-        TF* dd = vv + (size_t)C * inf.wu;
-        for (int q = threadIdx.x; q < C; q += blockDim.x) {
-            int k = 0;
-            if (q < c) {
-                const int r = perm_b[inf.row_off + p0 + q];
-                rr[q] = (uint16_t)tslot(r, inf.tshift);
-                for (int e = dg[r] + 1; e < rp[r + 1] && k < inf.wu; ++e) {
-                    cc[(size_t)k * C + q] = (uint16_t)tslot(ci[e], inf.tshift);
-                    vv[(size_t)k * C + q] = to_factor<TF>(v[e]);
-                    ++k;
-                }
-                dd[q] = to_factor<TF>(v[dg[r]]);
-            } else {
-                rr[q] = 0;
-                dd[q] = to_factor<TF>(1.0);
-            }
-            for (; k < inf.wu; ++k) {
-                cc[(size_t)k * C + q] = (uint16_t)tslot(inf.n, inf.tshift);
-                vv[(size_t)k * C + q] = to_factor<TF>(0.0);
-            }
-        }
+        const int i = inf.lev_off_b + l, p0 = lev_b[i];
+        pack_level<TF, true>(inf, rp, ci, dg, v, perm_b + inf.row_off + p0, lev_b[i + 1] - p0,
+                             rows_b[i], inf.wu, sb, rec + off_b[i]);
     }
 }
 
@@ -295,14 +253,13 @@ struct FVec<4> {
     }
 };
 
-// W > 0: rows with W nonzeros per triangle; W = 0: any width w
-template <int W, bool BACK, class TF, int R>
+// the component-wise records of any width w for R right-hand sides
+template <bool BACK, class TF, int R>
 __device__ __forceinline__ void level_rows_mr(uint32_t tb, uint32_t Rr, int C, int c, int w,
                                               int nthreads) {
     constexpr uint32_t SF = sizeof(TF), ST = 4u * R;
-    const int ww = W > 0 ? W : w;
     const uint32_t cstride = 2u * (uint32_t)C;
-    const uint32_t vbase = Rr + cstride * (uint32_t)(1 + ww);
+    const uint32_t vbase = Rr + cstride * (uint32_t)(1 + w);
     const uint32_t vstride = SF * (uint32_t)C;
     for (int q = threadIdx.x; q < c; q += nthreads) {
         const uint32_t rq = Rr + 2u * (uint32_t)q;
@@ -310,39 +267,91 @@ __device__ __forceinline__ void level_rows_mr(uint32_t tb, uint32_t Rr, int C, i
         const uint32_t r = lds_u16(rq);
         float acc[R];
         FVec<R>::ld(tb + ST * r, acc);
-        if constexpr (W > 0) {
-            uint32_t ck[W];
-            TF vk[W];
+        for (int k = 0; k < w; ++k) {
+            const uint32_t ci = lds_u16(rq + cstride * (uint32_t)(k + 1));
+            const float v = Load<float>::f(lds<TF>(vq + vstride * (uint32_t)k));
+            float xv[R];
+            FVec<R>::ld(tb + ST * ci, xv);
 #pragma unroll
-            for (int k = 0; k < W; ++k) ck[k] = lds_u16(rq + cstride * (uint32_t)(k + 1));
-#pragma unroll
-            for (int k = 0; k < W; ++k) vk[k] = lds<TF>(vq + vstride * (uint32_t)k);
-            float xk[W][R];
-#pragma unroll
-            for (int k = 0; k < W; ++k) FVec<R>::ld(tb + ST * ck[k], xk[k]);
-#pragma unroll
-            for (int k = 0; k < W; ++k) {
-                const float v = Load<float>::f(vk[k]);
-#pragma unroll
-                for (int i = 0; i < R; ++i) acc[i] = fmaf(-v, xk[k][i], acc[i]);
-            }
-        } else {
-            for (int k = 0; k < ww; ++k) {
-                const uint32_t ci = lds_u16(rq + cstride * (uint32_t)(k + 1));
-                const float v = Load<float>::f(lds<TF>(vq + vstride * (uint32_t)k));
-                float xv[R];
-                FVec<R>::ld(tb + ST * ci, xv);
-#pragma unroll
-                for (int i = 0; i < R; ++i) acc[i] = fmaf(-v, xv[i], acc[i]);
-            }
+            for (int i = 0; i < R; ++i) acc[i] = fmaf(-v, xv[i], acc[i]);
         }
         if (BACK) {
-            const float rd = 1.0f / Load<float>::f(lds<TF>(vq + vstride * (uint32_t)ww));
+            const float rd = 1.0f / Load<float>::f(lds<TF>(vq + vstride * (uint32_t)w));
 #pragma unroll
             for (int i = 0; i < R; ++i) acc[i] = acc[i] * rd;
         }
         FVec<R>::st(tb + ST * r, acc);
     }
+}
+
+// ---- row structs.  One struct of RB bytes holds everything a row reads
+// besides the vector; its words are loaded together (16, 8 or 4 bytes at a
+// time, whichever RB allows; every RB is conflict-free across a warp).
+template <int W, bool BACK, class TF>
+struct RowRec {
+    static constexpr int SF = (int)sizeof(TF);
+    static constexpr int RB = rec_row_bytes(W, BACK, SF);
+    static constexpr int VO = rec_val_off(W, SF);
+    static constexpr int DO = rec_recip_off(W, SF);
+    static constexpr int NW = (BACK ? DO + (SF == 8 ? 16 : 4) : VO + W * SF + 3) / 4;  // words read
+    uint32_t w[(NW + 3) / 4 * 4];
+
+    __device__ __forceinline__ void load(uint32_t a) {
+        if constexpr (RB % 16 == 0) {
+#pragma unroll
+            for (int i = 0; i < NW; i += 4)
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(w[i]), "=r"(w[i + 1]), "=r"(w[i + 2]), "=r"(w[i + 3])
+                             : "r"(a + 4u * i)
+                             : "memory");
+        } else if constexpr (RB % 8 == 0) {
+#pragma unroll
+            for (int i = 0; i < NW; i += 2)
+                asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];"
+                             : "=r"(w[i]), "=r"(w[i + 1])
+                             : "r"(a + 4u * i)
+                             : "memory");
+        } else {
+#pragma unroll
+            for (int i = 0; i < NW; ++i)
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[i]) : "r"(a + 4u * i) : "memory");
+        }
+    }
+    // slot k: the row (0) or column k - 1
+    __device__ __forceinline__ uint32_t slot(int k) const {
+        return (k & 1) ? w[k / 2] >> 16 : w[k / 2] & 0xffffu;
+    }
+    template <class TS>
+    __device__ __forceinline__ TS value(int k) const {
+        if constexpr (SF == 2) {
+            const int h = VO / 2 + k;
+            return (TS)__uint_as_float((h & 1) ? w[h / 2] & 0xffff0000u : w[h / 2] << 16);
+        } else if constexpr (SF == 4) {
+            return (TS)__uint_as_float(w[VO / 4 + k]);
+        } else {
+            return (TS)__hiloint2double((int)w[VO / 4 + 2 * k + 1], (int)w[VO / 4 + 2 * k]);
+        }
+    }
+    // FP64 sweeps: i = 0 the reciprocal, 1 the diagonal itself
+    template <class TS>
+    __device__ __forceinline__ TS recip(int i) const {
+        if constexpr (SF == 8)
+            return (TS)__hiloint2double((int)w[DO / 4 + 2 * i + 1], (int)w[DO / 4 + 2 * i]);
+        else
+            return (TS)__uint_as_float(w[DO / 4]);
+    }
+};
+
+// R vector elements of one slot
+template <class TS, int R>
+__device__ __forceinline__ void slot_ld(uint32_t a, TS (&v)[R]) {
+    if constexpr (R > 1) FVec<R>::ld(a, v);
+    else v[0] = lds<TS>(a);
+}
+template <class TS, int R>
+__device__ __forceinline__ void slot_st(uint32_t a, const TS (&v)[R]) {
+    if constexpr (R > 1) FVec<R>::st(a, v);
+    else sts(a, v[0]);
 }
 
 // ---- the gather and the restricted scatter of the TMA-fed sweep.  Rows are
@@ -444,16 +453,17 @@ __device__ __forceinline__ void scatter_ilp(const TS* t, TO* __restrict__ y, lon
 
 // Static schedule of one subdomain's record stream through the ring: the
 // stream (forward records, then backward, contiguous from `base` in the
-// packed array) is cut into groups of whole levels, each copied by one
-// cp.async.bulk into a fixed ring position and tracked by mbarrier
-// (group % RING_NBAR).  Per level (int4): x = rows | padded rows << 16, y =
-// the record's byte offset in the ring, z = the group whose copy the level
-// waits for (its first level; -1 otherwise), w = the groups that may have
-// been issued once the level is done.  Per group (int2): x = stream offset,
-// y = bytes / 16 | ring position / 16 << 16.
+// packed array) is cut into groups of whole levels of one direction, each
+// copied by one cp.async.bulk into a fixed ring position and tracked by
+// mbarrier (group % RING_NBAR).  Per group (int4): x = stream offset, y =
+// bytes / 16 | ring position / 16 << 16, z = its first entry, w = the groups
+// that may have been issued once it is done.  Per entry (int2), one pass over
+// at most the level threads' number of rows (component records: one entry a
+// level): x = rows left of the level | 0x10000 when a barrier follows, y = the
+// record's byte offset in the ring.  An entry of no rows ends a group.
 struct RingSub {
     long long base;
-    int meta_off, grp_off, ngrp, ninit;
+    int ent_off, grp_off, nent, ngrp, ngrp_f, ninit;  // groups [0, ngrp_f) are forward
 };
 constexpr int RING_LOG_NBAR = 5;
 constexpr int RING_NBAR = 1 << RING_LOG_NBAR;
@@ -463,8 +473,8 @@ struct RecArgs {
     const int* order;
     const int* dofs;
     const RingSub* ring;
-    const int4* meta;
-    const int2* grp;
+    const int2* ent;
+    const int4* grp;
     const unsigned char* rec;
     const int* ownloc;
     const int* owned;
@@ -473,9 +483,11 @@ struct RecArgs {
     int nparts;
     int nc;
     int a0pre;       // 1: the coarse row a0inv[s] is prefetched into shared memory
+    int row_structs; // 1: levels of width 2 to 4 are row structs
     int ring_bytes;  // bytes of the record ring
     int t_len;       // slots of the subdomain vector region (largest tslot(n) + 1)
-    int max_levels;  // largest nlev_f + nlev_b over the subdomains
+    int max_ent, max_grp;  // largest counts of schedule entries and groups
+    int level_threads;     // threads of the level loop
     long long ldx, ldy;  // distance between right-hand sides (R > 1)
     int* err;
     // optional per-subdomain switches, one array of nparts per right-hand
@@ -505,20 +517,18 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 }
 
 // The ring side of the level loop.  Set-up has checked that every group is
-// issued (after the level its schedule names) before its first level waits
+// issued (after the group its schedule names) before its first level waits
 // for it, and that a group re-arms an mbarrier or overwrites ring bytes only
 // after every thread has observed, and finished with, the group before it.
 //
-// A wait that gives up marks the thread (bad: it computes no more rows) and
-// the block: the shared word fail takes the failing level + 1.  Every thread
-// reads it when it next opens a group and acts only on a failure at an
-// earlier level -- written before a barrier it has passed, so all threads
-// see it and leave at the same level, while a failure being recorded at the
-// current level by a faster thread is left for the next group -- and once
-// more after the last level.
+// A wait that gives up marks the thread (bad: it computes no more rows and
+// waits for no further group) and the block (the shared word fail); a thread
+// that finds the word set before a wait does the same without waiting.  All
+// threads still pass every level's barrier, and the block gives up together
+// after the last one.  No thread reads a group that it has not seen land.
 struct RecRing {
     const unsigned char* src;
-    const int2* grp;       // shared memory
+    const int4* grp;       // shared memory
     volatile int* fail;    // shared memory
     uint32_t bars_s, ring_s;
     long long budget;
@@ -537,10 +547,10 @@ struct RecRing {
         return (uint32_t)((gbase + j) >> RING_LOG_NBAR) & 1u;
     }
     __device__ __forceinline__ void issue_to(int limit) {
-        if (issued >= limit) return;
+        if (issued >= limit || *fail != 0) return;
         fence_proxy_async();  // the ring bytes it overwrites were read by the generic proxy
         do {
-            const int2 gi = grp[issued];
+            const int4 gi = grp[issued];
             const uint32_t bytes = ((uint32_t)gi.y & 0xffffu) << 4;
             const uint32_t pos = ((uint32_t)gi.y >> 16) << 4;
             if (!(wait_test == 1 && issued == 0)) {
@@ -549,15 +559,18 @@ struct RecRing {
             }
         } while (++issued < limit);
     }
-    // the first try costs one mbarrier probe; the bounded loop (which reads
-    // the clock) runs only when the copy has not landed yet
-    __device__ __forceinline__ void wait_group(int j, int level) {
-        const uint32_t par = parity(j);
-        if (mbar_try(bar(j), par) || mbar_wait(bar(j), par, budget)) {
+    // whether group j has landed (one probe, no wait)
+    __device__ __forceinline__ bool landed(int j) const { return mbar_try(bar(j), parity(j)); }
+    // this thread's first access to group j: the first try costs one mbarrier
+    // probe; the bounded loop (which reads the clock) runs only when the copy
+    // has not landed yet
+    __device__ __forceinline__ void open(int j) {
+        if (bad) return;
+        if (*fail == 0 && (landed(j) || mbar_wait(bar(j), parity(j), budget))) {
             observed = j + 1;
         } else {
             bad = true;
-            *fail = level + 1;
+            *fail = 1;
         }
     }
     // the block leaves after a wait gave up: the producer waits (full budget
@@ -575,54 +588,121 @@ struct RecRing {
     }
 };
 
-// One sweep direction: levels [g0, g1), rows with W nonzeros per triangle
-// (W = 0: any width w).  Per level: the wait for the level's group when it
-// opens one, the rows, one barrier, then the producer issues the groups the
-// schedule allows.  The next level's metadata loads while this one
-// computes.  Returns false when the block leaves because a group did not
-// arrive within the wait budget.
-template <int W, bool BACK, class TS, class TF, bool EXACT, int R>
-__device__ __forceinline__ bool level_loop(const int4* meta, int g0, int g1, int T, int w,
-                                           RecRing& ring, TS* t, uint32_t t_s,
-                                           unsigned char* ring_g, int NC, int* err) {
-    if (g0 >= g1) return true;
-    int4 md = meta[g0];
-    for (int g = g0; g < g1; ++g) {
-        int4 mn = md;
-        if (g + 1 < T) mn = meta[g + 1];
-        if (md.z >= 0) {
-            const int f = *ring.fail;
-            if (f != 0 && f <= g) {  // a wait at an earlier level gave up
-                ring.drain(err);
-                return false;
+// barrier among the NC level threads
+__device__ __forceinline__ void level_sync(int NC) {
+    asm volatile("bar.sync 1, %0;" ::"r"(NC) : "memory");
+}
+
+// One sweep direction over component-wise records: groups [j0, j1), any
+// width w.  Per group the wait for its copy, then per level the rows and one
+// barrier, then the producer issues the groups the schedule allows.
+template <bool BACK, class TS, class TF, bool EXACT, int R>
+__device__ __forceinline__ void level_loop_any(const int2* ent, int j0, int j1, int w,
+                                               RecRing& ring, TS* t, uint32_t t_s,
+                                               unsigned char* ring_g, int NC) {
+    for (int j = j0; j < j1; ++j) {
+        ring.open(j);
+        const int e1 = ring.grp[j + 1].z - 1;
+        for (int e = ring.grp[j].z; e < e1; ++e) {
+            const int2 md = ent[e];
+            if (!ring.bad) {
+                const int c = md.x & 0xffff, C = (c + 7) & ~7;
+                if constexpr (R > 1)
+                    level_rows_mr<BACK, TF, R>(t_s, ring.ring_s + (uint32_t)md.y, C, c, w, NC);
+                else
+                    level_rows_any<TS, TF, EXACT>(t, ring_g + md.y, C, c, w, BACK, NC);
             }
-            ring.wait_group(md.z, g);
+            level_sync(NC);
         }
-        if (!ring.bad) {
-            const int c = md.x & 0xffff, C = (int)((unsigned)md.x >> 16);
-            if constexpr (R > 1)
-                level_rows_mr<W, BACK, TF, R>(t_s, ring.ring_s + (uint32_t)md.y, C, c, w, NC);
-            else if constexpr (W > 0)
-                level_rows_w<W, BACK, TS, TF, EXACT>(t_s, ring.ring_s + (uint32_t)md.y, C, c, NC);
-            else
-                level_rows_any<TS, TF, EXACT>(t, ring_g + md.y, C, c, w, BACK, NC);
-        }
-        __syncthreads();
-        if (ring.producer) ring.issue_to(md.w);
-        md = mn;
+        if (ring.producer) ring.issue_to(ring.grp[j].w);
     }
-    return true;
+}
+
+// One sweep direction over row structs of W nonzeros, groups [j0, j1).  The
+// time of a level is a chain of latencies -- shared loads, multiply-adds, the
+// barrier (a dependent FP64 multiply-add takes ~75 cycles here, a division
+// ~560) -- so everything that does not depend on the previous level is taken
+// out of it, and the loop over a group's levels is straight-line predicated
+// code (a divergent branch or an inner loop costs 40 to 80 cycles a level):
+//  * a thread loads the struct of its next row before the barrier, between
+//    the loads of this level's vector elements and their first use;
+//  * the diagonal comes as its reciprocal (exact FP64 sweeps divide);
+//  * the lanes past a level's end take the row that computes 0 in the unused
+//    slot, so no store is conditional within a warp;
+//  * a level of more than NC rows is several entries of the schedule.
+// Cycles per level in isolation, component records with the row's loads after
+// the barrier -> this loop: 51 x 51 FP32 223 -> 104, 15^3 FP32 288 -> 165;
+// 51 x 51 FP64 354 forward, 995 backward -> 214, 270; 14^3 FP64 481, 1159 ->
+// 414, 519.  Warps without rows still take the predicated FP64 instructions'
+// slots of the narrow FP64 pipe, which is why FP64 sweeps run their levels on
+// few warps (270 cycles with 2 warps, 507 with 8).
+template <int W, bool BACK, class TS, class TF, bool EXACT, int R>
+__device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecRing& ring,
+                                           uint32_t t_s, int NC) {
+    using Row = RowRec<W, BACK, TF>;
+    constexpr uint32_t ST = (uint32_t)(sizeof(TS) * R);
+    const int tid = threadIdx.x;
+    for (int j = j0; j < j1; ++j) {
+        ring.open(j);
+        const int wid = ring.bad ? 1 << 30 : (tid & ~31);  // first row of this warp
+        int e = ring.grp[j].z;
+        const int e1 = ring.grp[j + 1].z - 1;
+        int2 md = ent[e], mn = ent[e + 1];
+        int c = md.x & 0xffff, sync = md.x >> 16;
+        uint32_t a = ring.ring_s + (uint32_t)(md.y + Row::RB * min(tid, c));
+        bool on = wid < c;
+        Row row;
+        if (on) row.load(a);
+        for (; e < e1; ++e) {
+            const bool cur = on;
+            const int f = sync;
+            uint32_t ar = 0;
+            TS xk[W][R], acc[R], vk[W], rd = (TS)1;
+            if (cur) {
+                ar = t_s + ST * row.slot(0);
+#pragma unroll
+                for (int k = 0; k < W; ++k) slot_ld<TS, R>(t_s + ST * row.slot(k + 1), xk[k]);
+                slot_ld<TS, R>(ar, acc);
+#pragma unroll
+                for (int k = 0; k < W; ++k) vk[k] = row.template value<TS>(k);
+                if (BACK) rd = row.template recip<TS>(EXACT ? 1 : 0);
+            }
+            md = mn;
+            c = md.x & 0xffff;
+            sync = md.x >> 16;
+            a = ring.ring_s + (uint32_t)(md.y + Row::RB * min(tid, c));
+            on = wid < c;
+            mn = ent[e + 2];
+            if (on) row.load(a);
+            if (cur) {
+#pragma unroll
+                for (int k = 0; k < W; ++k)
+#pragma unroll
+                    for (int i = 0; i < R; ++i)
+                        acc[i] = sub_mul<TS, EXACT>(acc[i], vk[k], xk[k][i]);
+                if (BACK) {
+#pragma unroll
+                    for (int i = 0; i < R; ++i)
+                        acc[i] = (EXACT && sizeof(TS) == 8) ? acc[i] / rd : acc[i] * rd;
+                }
+                slot_st<TS, R>(ar, acc);
+            }
+            if (f) level_sync(NC);
+        }
+        if (ring.producer) ring.issue_to(ring.grp[j].w);
+    }
 }
 
 template <bool BACK, class TS, class TF, bool EXACT, int R>
-__device__ __forceinline__ bool level_loop_w(const int4* meta, int g0, int g1, int T, int w,
+__device__ __forceinline__ void level_loop_w(const int2* ent, int j0, int j1, int w, bool rows,
                                              RecRing& ring, TS* t, uint32_t t_s,
-                                             unsigned char* ring_g, int NC, int* err) {
-    switch (w) {
-    case 2: return level_loop<2, BACK, TS, TF, EXACT, R>(meta, g0, g1, T, w, ring, t, t_s, ring_g, NC, err);
-    case 3: return level_loop<3, BACK, TS, TF, EXACT, R>(meta, g0, g1, T, w, ring, t, t_s, ring_g, NC, err);
-    case 4: return level_loop<4, BACK, TS, TF, EXACT, R>(meta, g0, g1, T, w, ring, t, t_s, ring_g, NC, err);
-    default: return level_loop<0, BACK, TS, TF, EXACT, R>(meta, g0, g1, T, w, ring, t, t_s, ring_g, NC, err);
+                                             unsigned char* ring_g, int NC) {
+    switch (rows ? w : 0) {
+    case 2: return level_loop<2, BACK, TS, TF, EXACT, R>(ent, j0, j1, ring, t_s, NC);
+    case 3: return level_loop<3, BACK, TS, TF, EXACT, R>(ent, j0, j1, ring, t_s, NC);
+    case 4: return level_loop<4, BACK, TS, TF, EXACT, R>(ent, j0, j1, ring, t_s, NC);
+    default:
+        return level_loop_any<BACK, TS, TF, EXACT, R>(ent, j0, j1, w, ring, t, t_s, ring_g, NC);
     }
 }
 
@@ -631,8 +711,8 @@ struct SweepSmem {
     unsigned char* raw;   // RING_NBAR mbarriers, then the ring
     unsigned char* ring;  // ring_bytes
     void* t;              // t_len slots of R elements
-    int4* meta;           // max_levels
-    int2* grp;            // max_levels
+    int4* grp;            // max_grp + 1
+    int2* ent;            // max_ent
     double* a0row;        // nc (a0pre)
 };
 
@@ -654,11 +734,10 @@ __device__ __forceinline__ bool sweep_one(const RecArgs& a, int s, const TI* __r
     const SubInfo inf = a.info[s];
     const RingSub rs = a.ring[s];
     const int n = inf.n;
-    const int nf = inf.nlev_f, T = inf.nlev_f + inf.nlev_b;
     // the schedule, staged once (the level loop touches global memory only
     // through the ring)
-    for (int g = threadIdx.x; g < T; g += NC) sm.meta[g] = a.meta[rs.meta_off + g];
-    for (int j = threadIdx.x; j < rs.ngrp; j += NC) sm.grp[j] = a.grp[rs.grp_off + j];
+    for (int e = threadIdx.x; e < rs.nent; e += NC) sm.ent[e] = a.ent[rs.ent_off + e];
+    for (int j = threadIdx.x; j <= rs.ngrp; j += NC) sm.grp[j] = a.grp[rs.grp_off + j];
 
     RecRing ring;
     ring.src = a.rec + rs.base;
@@ -672,11 +751,12 @@ __device__ __forceinline__ bool sweep_one(const RecArgs& a, int s, const TI* __r
     ring.observed = 0;
     ring.bad = false;
     ring.wait_test = a.wait_test;
-    // the producer is the block's last thread: levels rarely have rows for
-    // it, so its copies overlap the other threads' work.  The mbarriers are
+    // the producer is the last of the level threads: levels rarely have rows
+    // for it, so its copies overlap the other threads' work.  The mbarriers are
     // initialised with the CTA's first subdomain; later ones continue their
     // phases (every group of the previous subdomain was issued and observed).
-    ring.producer = threadIdx.x == blockDim.x - 1;
+    const int LT = a.level_threads;
+    ring.producer = (int)threadIdx.x == LT - 1;
     if (ring.producer) {
         if (first)
             for (int i = 0; i < RING_NBAR; ++i) mbar_init(ring.bars_s + 8u * (uint32_t)i, 1);
@@ -724,13 +804,14 @@ __device__ __forceinline__ bool sweep_one(const RecArgs& a, int s, const TI* __r
     // the level loop -- the latency chain of the sweep -- one direction at a
     // time, specialised on the row width
     const uint32_t t_s = smem_u32(t);
-    if (!level_loop_w<false, TS, TF, EXACT, R>(sm.meta, 0, nf, T, inf.wl, ring, t, t_s, sm.ring,
-                                               NC, a.err))
-        return false;
-    if (!level_loop_w<true, TS, TF, EXACT, R>(sm.meta, nf, T, T, inf.wu, ring, t, t_s, sm.ring,
-                                              NC, a.err))
-        return false;
-    if (s_fail) {  // a wait in the last group gave up (read after the last level's barrier)
+    if ((int)threadIdx.x < LT) {
+        level_loop_w<false, TS, TF, EXACT, R>(sm.ent, 0, rs.ngrp_f, inf.wl, a.row_structs != 0,
+                                              ring, t, t_s, sm.ring, LT);
+        level_loop_w<true, TS, TF, EXACT, R>(sm.ent, rs.ngrp_f, rs.ngrp, inf.wu,
+                                             a.row_structs != 0, ring, t, t_s, sm.ring, LT);
+    }
+    __syncthreads();
+    if (s_fail) {  // a wait gave up
         ring.drain(a.err);
         return false;
     }
@@ -791,12 +872,21 @@ __device__ __forceinline__ bool sweep_one(const RecArgs& a, int s, const TI* __r
     return true;
 }
 
+// The same as a call of its own, for CTAs that loop over subdomains: inlined
+// there, values hoisted out of that loop spill inside the level loops.
+template <class TI, class TO, class TS, class TF, bool EXACT, int R>
+__device__ __noinline__ bool sweep_one_call(const RecArgs& a, int s, const TI* __restrict__ x,
+                                            TO* __restrict__ y, int mode, int coarse,
+                                            const SweepSmem& sm, int& gbase, bool first) {
+    return sweep_one<TI, TO, TS, TF, EXACT, R>(a, s, x, y, mode, coarse, sm, gbase, first);
+}
+
 // mode 0: RAS (owned rows written), 1: ASM (all rows added atomically).  One
 // subdomain per CTA, or (PERSIST) CTAs looping over subdomains taken largest
 // first from a work counter.
 template <class TI, class TO, class TS, class TF, bool EXACT, int R, bool PERSIST>
 __global__ void __launch_bounds__(SW_T, 2)
-k_sweep_tma(RecArgs a, const TI* __restrict__ x, TO* __restrict__ y, int mode, int coarse,
+k_sweep_tma(const __grid_constant__ RecArgs a, const TI* __restrict__ x, TO* __restrict__ y, int mode, int coarse,
             const int* __restrict__ active) {
     if (active && *active == 0) return;
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -805,10 +895,10 @@ k_sweep_tma(RecArgs a, const TI* __restrict__ x, TO* __restrict__ y, int mode, i
     sm.raw = smraw;
     sm.ring = smraw + HDR;
     sm.t = sm.ring + a.ring_bytes;
-    sm.meta = reinterpret_cast<int4*>(reinterpret_cast<unsigned char*>(sm.t) +
-                                      (((size_t)a.t_len * R * sizeof(TS) + 15) & ~(size_t)15));
-    sm.grp = reinterpret_cast<int2*>(sm.meta + a.max_levels);
-    sm.a0row = reinterpret_cast<double*>(sm.grp + a.max_levels);
+    sm.grp = reinterpret_cast<int4*>(reinterpret_cast<unsigned char*>(sm.t) +
+                                     (((size_t)a.t_len * R * sizeof(TS) + 15) & ~(size_t)15));
+    sm.ent = reinterpret_cast<int2*>(sm.grp + a.max_grp + 1);
+    sm.a0row = reinterpret_cast<double*>(sm.ent + a.max_ent);
     auto on = [&](int s) {
         if (!a.sub_on) return true;
         bool v = false;
@@ -832,7 +922,8 @@ k_sweep_tma(RecArgs a, const TI* __restrict__ x, TO* __restrict__ y, int mode, i
             if (idx >= a.nparts) break;
             const int s = a.order[idx];
             if (!on(s)) continue;
-            if (!sweep_one<TI, TO, TS, TF, EXACT, R>(a, s, x, y, mode, coarse, sm, gbase, first))
+            if (!sweep_one_call<TI, TO, TS, TF, EXACT, R>(a, s, x, y, mode, coarse, sm, gbase,
+                                                          first))
                 return;
             first = false;
         }
@@ -854,8 +945,8 @@ RecArgs rec_args(sg_precond* pc, const RingPlan& plan, bool fuse) {
     a.order = pc->order.p;
     a.dofs = pc->dofs.p;
     a.ring = reinterpret_cast<const RingSub*>(plan.sub_d.p);
-    a.meta = reinterpret_cast<const int4*>(plan.meta_d.p);
-    a.grp = reinterpret_cast<const int2*>(plan.grp_d.p);
+    a.ent = reinterpret_cast<const int2*>(plan.ent_d.p);
+    a.grp = reinterpret_cast<const int4*>(plan.grp_d.p);
     a.rec = pc->rec_d.p;
     a.ownloc = pc->ownloc_d.p;
     a.owned = pc->owned_d.p;
@@ -864,9 +955,12 @@ RecArgs rec_args(sg_precond* pc, const RingPlan& plan, bool fuse) {
     a.nparts = pc->nparts;
     a.nc = pc->nc;
     a.a0pre = sweep_a0_prefetch(pc) ? 1 : 0;
+    a.row_structs = pc->rec_rows ? 1 : 0;
     a.ring_bytes = (int)plan.ring_bytes;
     a.t_len = pc->t_len;
-    a.max_levels = pc->max_levels;
+    a.max_ent = plan.max_ent;
+    a.max_grp = plan.max_grp;
+    a.level_threads = plan.level_threads;
     a.ldx = 0;
     a.ldy = 0;
     a.err = pc->err_d.p;
@@ -886,16 +980,17 @@ bool sweep_a0_prefetch(const sg_precond* pc) {
 }
 
 // dynamic shared memory of the sweep: the mbarriers, the record ring, the
-// subdomain vector (R elements per slot), per-level and per-group schedule
-// entries, the coarse row
-size_t sweep_smem_for(const sg_precond* pc, long long ring_bytes, int R) {
+// subdomain vector (R elements per slot), the schedule's groups and entries,
+// the coarse row
+size_t sweep_smem_for(const sg_precond* pc, const RingPlan& plan, long long ring_bytes) {
     const size_t ts = pc->opts.sweep_dtype == SG_FP64 ? 8 : 4;
-    const size_t tbytes = ((size_t)pc->t_len * ts * R + 15) & ~(size_t)15;
+    const size_t tbytes = ((size_t)pc->t_len * ts * plan.R + 15) & ~(size_t)15;
     const size_t a0 = sweep_a0_prefetch(pc) ? (size_t)pc->nparts * 8 : 0;
-    return RING_NBAR * 8 + (size_t)ring_bytes + tbytes + (size_t)pc->max_levels * (16 + 8) + a0;
+    return RING_NBAR * 8 + (size_t)ring_bytes + tbytes + ((size_t)plan.max_grp + 1) * 16 +
+           (size_t)plan.max_ent * 8 + a0;
 }
 size_t sweep_smem(const sg_precond* pc, const RingPlan& plan) {
-    return sweep_smem_for(pc, plan.ring_bytes, plan.R);
+    return sweep_smem_for(pc, plan, plan.ring_bytes);
 }
 
 template <class TI, class TO, class TS, class TF, bool EXACT, int R>
@@ -940,108 +1035,127 @@ void launch_tma(sg_precond* pc, const RingPlan& plan, const TI* x, TO* y, int mo
 }  // namespace
 
 // Builds the static ring schedule of every subdomain (see RingSub) into
-// `plan` for a ring of ring_bytes and groups of at most gmax bytes (a larger
-// level is a group of its own).  Groups are placed one after another and
-// start over at the ring's beginning when they would cross its end.  Group
-// j may be issued after the last level of every earlier group whose ring
-// bytes it overwrites and of group j - RING_NBAR (its mbarrier's previous
-// user); the schedule is feasible when that is always before group j's
-// first level.  Returns false (plan unchanged) when it is not.
-static bool ring_schedule(const sg_precond* pc, RingPlan& plan, long long ring_bytes,
-                          long long gmax) {
-    const long long sf = pc->opts.sweep_dtype == SG_FP64 ? 8
-                         : (pc->opts.factor_dtype == SG_BF16 ? 2 : 4);
+// `plan` for level loops of nlt threads, groups of at most gmax bytes (a
+// larger level is a group of its own) and the ring that `budget` bytes of
+// dynamic shared memory leave.  Groups are placed one after another and start
+// over at the ring's beginning when they would cross its end.  Group j may be
+// issued after the last level of every earlier group whose ring bytes it
+// overwrites and of group j - RING_NBAR (its mbarrier's previous user); the
+// schedule is feasible when that is always before group j's first level.
+// Returns false when it is not.
+static bool ring_schedule(const sg_precond* pc, RingPlan& plan, long long budget, long long gmax,
+                          int nlt) {
+    const int sf = rec_value_bytes(pc);
     std::vector<RingSub> subs((size_t)pc->nparts);
-    std::vector<int> meta, grp;  // int4 / int2 entries as ints
-    std::vector<long long> rel, gstart, gbytes, gpos;
-    std::vector<int> B, cnt, padded, gfirst, glast, ia;
+    std::vector<int> ent, grp;  // int2 / int4 entries as ints
+    struct Group {
+        int first, last;  // levels
+        long long start, bytes, pos;
+    };
+    std::vector<Group> groups;  // of all subdomains
+    int max_ent = 0, max_grp = 0;
     for (int s = 0; s < pc->nparts; ++s) {
         const SubInfo& inf = pc->h_info[s];
         const int nf = inf.nlev_f, T = inf.nlev_f + inf.nlev_b;
-        rel.resize(T);
-        B.resize(T);
-        cnt.resize(T);
-        padded.resize(T);
-        for (int g = 0; g < T; ++g) {
-            if (g < nf) {
-                const int i = inf.lev_off_f + g;
-                rel[g] = pc->h_rec_off_f[i];
-                padded[g] = pc->h_rec_rows_f[i];
-                cnt[g] = pc->h_lev_ptr_f[i + 1] - pc->h_lev_ptr_f[i];
-                B[g] = (int)(padded[g] * (2 + inf.wl * (2 + sf)));
-            } else {
-                const int i = inf.lev_off_b + (g - nf);
-                rel[g] = pc->h_rec_off_b[i];
-                padded[g] = pc->h_rec_rows_b[i];
-                cnt[g] = pc->h_lev_ptr_b[i + 1] - pc->h_lev_ptr_b[i];
-                B[g] = (int)(padded[g] * (2 + inf.wu * (2 + sf) + sf));
-            }
-        }
         RingSub& r = subs[s];
-        r.base = T > 0 ? rel[0] : 0;
-        r.meta_off = (int)(meta.size() / 4);
-        r.grp_off = (int)(grp.size() / 2);
-        for (int g = 0; g < T; ++g) rel[g] -= r.base;
-        // groups of whole levels
-        gfirst.clear();
-        glast.clear();
-        gstart.clear();
-        gbytes.clear();
+        r.base = nf > 0 ? pc->h_rec_off_f[inf.lev_off_f]
+                        : (T > 0 ? pc->h_rec_off_b[inf.lev_off_b] : 0);
+        const size_t g0 = groups.size();
+        r.ngrp_f = 0;
+        int nent = 0;
         for (int g = 0; g < T; ++g) {
-            if (gfirst.empty() || gbytes.back() + B[g] > gmax) {
-                gfirst.push_back(g);
-                glast.push_back(g);
-                gstart.push_back(rel[g]);
-                gbytes.push_back(B[g]);
+            const bool back = g >= nf;
+            const int i = back ? inf.lev_off_b + (g - nf) : inf.lev_off_f + g;
+            const std::vector<int>& lp = back ? pc->h_lev_ptr_b : pc->h_lev_ptr_f;
+            const int c = lp[i + 1] - lp[i], w = back ? inf.wu : inf.wl;
+            const long long rel = (back ? pc->h_rec_off_b[i] : pc->h_rec_off_f[i]) - r.base;
+            const long long B = rec_level_bytes(pc, w, back, c);
+            if (groups.size() == g0 || g == nf || groups.back().bytes + B > gmax) {
+                groups.push_back({g, g, rel, B, 0});
+                ++nent;  // the entry that ends it
+                if (!back) ++r.ngrp_f;
             } else {
-                glast.back() = g;
-                gbytes.back() = rel[g] + B[g] - gstart.back();
+                groups.back().last = g;
+                groups.back().bytes = rel + B - groups.back().start;
             }
+            nent += pc->rec_rows && rec_is_rows(w) ? (c + nlt - 1) / nlt : 1;
         }
-        const int G = (int)gfirst.size();
-        gpos.assign(G, 0);
+        r.ngrp = (int)(groups.size() - g0);
+        r.nent = nent + 1;  // the loop reads one entry past the last
+        max_ent = std::max(max_ent, r.nent);
+        max_grp = std::max(max_grp, r.ngrp);
+    }
+    plan.max_ent = max_ent;
+    plan.max_grp = max_grp;
+    plan.level_threads = nlt;
+    const long long ring = (budget - (long long)sweep_smem_for(pc, plan, 0)) & ~15ll;
+    if (ring < pc->rec_stage_bytes) return false;
+    std::vector<int> ia;
+    size_t gbase = 0;
+    for (int s = 0; s < pc->nparts; ++s) {
+        const SubInfo& inf = pc->h_info[s];
+        const int nf = inf.nlev_f;
+        RingSub& r = subs[s];
+        const int G = r.ngrp;
+        Group* gr = groups.data() + gbase;
+        gbase += (size_t)G;
         long long pos = 0;
         for (int j = 0; j < G; ++j) {
-            if (gbytes[j] > ring_bytes || gbytes[j] >= (1ll << 20)) return false;
-            if (pos + gbytes[j] > ring_bytes) pos = 0;
-            gpos[j] = pos;
-            pos += gbytes[j];
+            if (gr[j].bytes > ring || gr[j].bytes >= (1ll << 20)) return false;
+            if (pos + gr[j].bytes > ring) pos = 0;
+            gr[j].pos = pos;
+            pos += gr[j].bytes;
         }
+        // ia[j]: the group after which group j may be issued (-1: at once)
         ia.assign(G, -1);
         int run = -1;
         for (int j = 0; j < G; ++j) {
             int v = -1;
             for (int i = std::max(0, j - RING_NBAR); i < j; ++i)
-                if (gpos[i] < gpos[j] + gbytes[j] && gpos[j] < gpos[i] + gbytes[i])
-                    v = std::max(v, glast[i]);
-            if (j >= RING_NBAR) v = std::max(v, glast[j - RING_NBAR]);
+                if (gr[i].pos < gr[j].pos + gr[j].bytes && gr[j].pos < gr[i].pos + gr[i].bytes)
+                    v = i;
+            if (j >= RING_NBAR) v = std::max(v, j - RING_NBAR);
             run = std::max(run, v);
-            if (run >= gfirst[j]) return false;  // would wait for a copy not yet issued
             ia[j] = run;
         }
-        int ninit = 0;
-        while (ninit < G && ia[ninit] < 0) ++ninit;
-        r.ngrp = G;
-        r.ninit = ninit;
-        int jg = 0, ji = 0;
-        for (int g = 0; g < T; ++g) {
-            while (jg + 1 < G && gfirst[jg + 1] <= g) ++jg;
-            while (ji < G && ia[ji] <= g) ++ji;
-            meta.push_back(cnt[g] | (padded[g] << 16));
-            meta.push_back((int)(gpos[jg] + rel[g] - gstart[jg]));
-            meta.push_back(gfirst[jg] == g ? jg : -1);
-            meta.push_back(ji);
-        }
+        r.ninit = 0;
+        while (r.ninit < G && ia[r.ninit] < 0) ++r.ninit;
+        r.ent_off = (int)(ent.size() / 2);
+        r.grp_off = (int)(grp.size() / 4);
+        int ji = 0, ne = 0;
         for (int j = 0; j < G; ++j) {
-            grp.push_back((int)gstart[j]);
-            grp.push_back((int)((gbytes[j] >> 4) | ((gpos[j] >> 4) << 16)));
+            while (ji < G && ia[ji] <= j) ++ji;
+            grp.push_back((int)gr[j].start);
+            grp.push_back((int)((gr[j].bytes >> 4) | ((gr[j].pos >> 4) << 16)));
+            grp.push_back(ne);
+            grp.push_back(ji);
+            for (int g = gr[j].first; g <= gr[j].last; ++g) {
+                const bool back = g >= nf;
+                const int i = back ? inf.lev_off_b + (g - nf) : inf.lev_off_f + g;
+                const std::vector<int>& lp = back ? pc->h_lev_ptr_b : pc->h_lev_ptr_f;
+                const int c = lp[i + 1] - lp[i], w = back ? inf.wu : inf.wl;
+                const long long rel = (back ? pc->h_rec_off_b[i] : pc->h_rec_off_f[i]) - r.base;
+                const int at = (int)(gr[j].pos + rel - gr[j].start);
+                const bool rows = pc->rec_rows && rec_is_rows(w);
+                const int step = rows ? nlt : c, rb = rec_row_bytes(w, back, sf);
+                for (int q = 0; q < c; q += step, ++ne) {
+                    ent.push_back((c - q) | (q + step >= c ? 0x10000 : 0));
+                    ent.push_back(at + (rows ? q * rb : 0));
+                }
+            }
+            ent.push_back(0);
+            ent.push_back(0);
+            ++ne;
         }
+        ent.push_back(0);
+        ent.push_back(0);
+        for (int v : {0, 0, ne, G}) grp.push_back(v);
     }
     plan.sub.assign(reinterpret_cast<const unsigned char*>(subs.data()),
                     reinterpret_cast<const unsigned char*>(subs.data() + subs.size()));
-    plan.meta.swap(meta);
+    plan.ent.swap(ent);
     plan.grp.swap(grp);
-    plan.ring_bytes = ring_bytes;
+    plan.ring_bytes = ring;
     plan.gmax = gmax;
     return true;
 }
@@ -1049,7 +1163,7 @@ static bool ring_schedule(const sg_precond* pc, RingPlan& plan, long long ring_b
 static void ring_upload(sg_precond* pc, RingPlan& plan) {
     cudaStream_t st = pc->ctx->stream;
     plan.sub_d.upload(plan.sub, st);
-    plan.meta_d.upload(plan.meta, st);
+    plan.ent_d.upload(plan.ent, st);
     plan.grp_d.upload(plan.grp, st);
 }
 
@@ -1065,10 +1179,30 @@ static int sweep_occupancy(sg_precond* pc, const RingPlan& plan, K kern) {
     return per_sm;
 }
 
-// Sizes a plan's ring (what the shared memory of the CTAs that must share an
-// SM leaves) and lists the record-group sizes whose schedule is feasible
-// for it (the schedule of the last one is left in `plan`).
-static std::vector<long long> ring_size(sg_precond* pc, RingPlan& plan) {
+// Block sizes to time, and how many of the threads run the level loop.  FP64
+// levels run on few warps (see level_loop) while the whole block gathers and
+// scatters; opts.reserved[1] forces one size for both.  One- and two-warp CTAs
+// are not timed: on the 2D subdomains of the batched workload (~20 rows per
+// level) they measured slower than 128 threads (the gather, scatter and
+// record stream lose more than the cheaper barrier gains).
+struct BlockShape {
+    int threads, level_threads;
+};
+static std::vector<BlockShape> block_shapes(const sg_precond* pc) {
+    const int forced = pc->opts.reserved[1];
+    if (forced > 0) return {{forced, forced}};
+    if (pc->opts.sweep_dtype == SG_FP64) return {{384, 384}, {256, 256}, {256, 128}, {256, 64}};
+    return {{512, 512}, {384, 384}, {256, 256}, {128, 128}};
+}
+
+// The dynamic shared memory a plan's CTAs may use (what the CTAs that must
+// share an SM leave each other) and the record-group sizes whose schedule is
+// feasible in it.
+struct RingFit {
+    long long budget = 0;
+    std::vector<long long> gmax;
+};
+static RingFit ring_size(sg_precond* pc, RingPlan& plan) {
     sg_ctx* ctx = pc->ctx;
     int max_smem = 0, sm_smem = 0;
     SG_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin,
@@ -1080,31 +1214,35 @@ static std::vector<long long> ring_size(sg_precond* pc, RingPlan& plan) {
     // subdomains than that run persistent or in waves)
     int want = (pc->nparts + ctx->num_sms - 1) / ctx->num_sms;
     if (want > 4) want = 4;
-    // group size: opts.reserved[3] when set, else timed among 8 and 16 KB
-    // (never below the largest record)
-    std::vector<long long> gcand;
-    if (pc->opts.reserved[3] > 0) gcand.push_back(pc->opts.reserved[3]);
-    else gcand = {8192, 16384};
-    std::vector<long long> gok;
-    for (int per_sm = want < 1 ? 1 : want; per_sm >= 1 && gok.empty(); --per_sm) {
-        const long long budget = std::min<long long>((long long)sm_smem / per_sm - static_smem - 1024,
-                                                     (long long)max_smem - static_smem);
-        const long long ring = (budget - (long long)sweep_smem_for(pc, 0, plan.R)) & ~15ll;
-        if (ring < pc->rec_stage_bytes) continue;
+    const int nlt = block_shapes(pc).front().level_threads;  // the fewest entries
+    RingFit fit;
+    for (int per_sm = want < 1 ? 1 : want; per_sm >= 1 && fit.gmax.empty(); --per_sm) {
+        fit.budget = std::min<long long>((long long)sm_smem / per_sm - static_smem - 1024,
+                                         (long long)max_smem - static_smem);
+        // group size: opts.reserved[3] when set, else timed among two sizes
+        // (never below the largest record): 8 and 16 KB, or 16 and 32 KB where
+        // the ring holds four of them -- each group costs the level loop ~160
+        // cycles, and the first one delays the first level
+        plan.max_ent = plan.max_grp = 0;
+        const long long room = fit.budget - (long long)sweep_smem_for(pc, plan, 0);
+        std::vector<long long> gcand = {8192, 16384};
+        if (room >= 131072) gcand = {16384, 32768};
+        if (pc->opts.reserved[3] > 0) gcand = {pc->opts.reserved[3]};
         for (long long target : gcand) {
             for (long long gmax : {target, target / 2, target / 4}) {
                 if (gmax < pc->rec_stage_bytes) gmax = pc->rec_stage_bytes;
-                if (ring_schedule(pc, plan, ring, gmax)) {
-                    if (std::find(gok.begin(), gok.end(), gmax) == gok.end()) gok.push_back(gmax);
+                if (ring_schedule(pc, plan, fit.budget, gmax, nlt)) {
+                    if (std::find(fit.gmax.begin(), fit.gmax.end(), gmax) == fit.gmax.end())
+                        fit.gmax.push_back(gmax);
                     break;
                 }
             }
         }
     }
-    return gok;
+    return fit;
 }
 
-void tune_plan(sg_precond* pc, RingPlan& plan, const std::vector<long long>& gmax_list);
+void tune_plan(sg_precond* pc, RingPlan& plan, const RingFit& fit);
 
 // Packs the level records in the configured factor type, plans the
 // one-vector ring and times its block size, record-group size and launch
@@ -1113,19 +1251,26 @@ void rec_setup_device(sg_precond* pc) {
     if (!pc->use_rec) return;
     sg_ctx* ctx = pc->ctx;
     cudaStream_t st = ctx->stream;
-    if (pc->rec_stage_bytes % 16 != 0 || pc->rec_total % 16 != 0)
-        fail(SG_ERR_INTERNAL, "level records are not 16-byte multiples");
     RingPlan& plan = pc->ring1;
     plan.R = 1;
     plan.ready = false;
     pc->ring4.ready = false;  // a new set-up plans the four-vector ring again when asked
-    const std::vector<long long> gok = ring_size(pc, plan);
-    if (gok.empty() || (pc->opts.reserved[0] & 1)) {
+    // records of row structs, unless their rings do not fit beside the vector
+    // of a subdomain near the shared-memory limit (component records are
+    // smaller)
+    rec_layout(pc, true);
+    RingFit fit = ring_size(pc, plan);
+    if (fit.gmax.empty()) {
+        rec_layout(pc, false);
+        fit = ring_size(pc, plan);
+    }
+    if (fit.gmax.empty() || (pc->opts.reserved[0] & 1)) {
         pc->use_rec = false;
         return;
     }
+    if (pc->rec_stage_bytes % 16 != 0 || pc->rec_total % 16 != 0)
+        fail(SG_ERR_INTERNAL, "level records are not 16-byte multiples");
     pc->rec_depth = 1;
-    ring_upload(pc, plan);
     pc->rec_off_f_d.upload(pc->h_rec_off_f, st);
     pc->rec_off_b_d.upload(pc->h_rec_off_b, st);
     pc->rec_rows_f_d.upload(pc->h_rec_rows_f, st);
@@ -1139,7 +1284,7 @@ void rec_setup_device(sg_precond* pc) {
     k_pack_rec<TF><<<pc->nparts, 256, 0, st>>>(                                            \
         pc->info.p, pc->lrp_d.p, pc->lci_d.p, pc->ldiag_d.p, pc->lu_d.p, pf, pb,            \
         pc->lev_ptr_f.p, pc->lev_ptr_b.p, pc->rec_off_f_d.p, pc->rec_off_b_d.p,             \
-        pc->rec_rows_f_d.p, pc->rec_rows_b_d.p, pc->rec_d.p)
+        pc->rec_rows_f_d.p, pc->rec_rows_b_d.p, pc->rec_rows ? 1 : 0, pc->rec_d.p)
     if (pc->opts.sweep_dtype == SG_FP64) SG_PACK(double);
     else if (pc->opts.factor_dtype == SG_BF16) SG_PACK(uint16_t);
     else SG_PACK(float);
@@ -1149,7 +1294,7 @@ void rec_setup_device(sg_precond* pc) {
     // and launch shape.  Levels of a 3D subdomain hold ~100+ rows, those of a
     // small 2D one ~20: a 512-thread block then idles at every level
     // barrier, while narrower blocks let more subdomains run at once.
-    tune_plan(pc, plan, gok);
+    tune_plan(pc, plan, fit);
     pc->sweep_threads = plan.threads;
     // two-level: the coarse restriction runs inside the sweep when every
     // subdomain's CTA can be resident at once (a cooperative launch)
@@ -1176,11 +1321,10 @@ bool sweep_fuses_restrict(const sg_precond* pc) {
 }
 
 // Times the sweep (RAS mode, no coarse term, zero input; R interleaved
-// vectors) for every record-group size in gmax_list, 128, 256, 384 and 512
-// threads per CTA (or the forced block size) and, when there are more
+// vectors) for every record-group size of the fit, every block shape and, when there are more
 // subdomains than resident CTAs, one CTA per subdomain against a persistent
 // grid; keeps the fastest.
-void tune_plan(sg_precond* pc, RingPlan& plan, const std::vector<long long>& gmax_list) {
+void tune_plan(sg_precond* pc, RingPlan& plan, const RingFit& fit) {
     sg_ctx* ctx = pc->ctx;
     cudaStream_t st = ctx->stream;
     const int R = plan.R;
@@ -1221,19 +1365,14 @@ void tune_plan(sg_precond* pc, RingPlan& plan, const std::vector<long long>& gma
     SG_CUDA(cudaEventCreate(&e0));
     SG_CUDA(cudaEventCreate(&e1));
     float best = -1.f;
-    int best_nt = SW_T, best_grid = 0;
-    long long best_g = gmax_list.front();
-    // one- and two-warp CTAs (reserved[1] = 32 or 64) are not timed: on the
-    // 2D subdomains of the batched workload (~20 rows per level) they
-    // measured slower than 128 threads (the gather, scatter and record
-    // stream lose more than the cheaper barrier gains)
-    std::vector<int> threads = {512, 384, 256, 128};
-    if (pc->opts.reserved[1] > 0) threads = {pc->opts.reserved[1]};
-    for (long long gmax : gmax_list) {
-        if (!ring_schedule(pc, plan, plan.ring_bytes, gmax)) continue;
-        ring_upload(pc, plan);
-        for (int nt : threads) {
-            plan.threads = nt;
+    BlockShape best_sh{SW_T, SW_T};
+    int best_grid = 0;
+    long long best_g = fit.gmax.front();
+    for (long long gmax : fit.gmax) {
+        for (const BlockShape& sh : block_shapes(pc)) {
+            if (!ring_schedule(pc, plan, fit.budget, gmax, sh.level_threads)) continue;
+            ring_upload(pc, plan);
+            plan.threads = sh.threads;
             plan.grid = 0;
             const int per_sm = occupancy();
             if (per_sm < 1) continue;
@@ -1266,7 +1405,7 @@ void tune_plan(sg_precond* pc, RingPlan& plan, const std::vector<long long>& gma
                 }
                 if (best < 0.f || ms < best) {
                     best = ms;
-                    best_nt = nt;
+                    best_sh = sh;
                     best_g = gmax;
                     best_grid = grid;
                 }
@@ -1276,9 +1415,9 @@ void tune_plan(sg_precond* pc, RingPlan& plan, const std::vector<long long>& gma
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (best < 0.f) fail(SG_ERR_INTERNAL, "no sweep configuration fits the GPU");
-    plan.threads = best_nt;
+    plan.threads = best_sh.threads;
     plan.grid = best_grid;
-    if (!ring_schedule(pc, plan, plan.ring_bytes, best_g)) fail(SG_ERR_INTERNAL, "ring schedule lost");
+    if (!ring_schedule(pc, plan, fit.budget, best_g, best_sh.level_threads)) fail(SG_ERR_INTERNAL, "ring schedule lost");
     ring_upload(pc, plan);
     plan.ready = true;
 }
@@ -1309,11 +1448,11 @@ bool sweep_plan4(sg_precond* pc) {
     RingPlan& plan = pc->ring4;
     if (plan.ready) return true;
     plan.R = 4;
-    const std::vector<long long> gok = ring_size(pc, plan);
-    if (gok.empty()) return false;
+    const RingFit fit = ring_size(pc, plan);
+    if (fit.gmax.empty()) return false;
     const int* keep = pc->sub_on;
     pc->sub_on = nullptr;
-    tune_plan(pc, plan, gok);
+    tune_plan(pc, plan, fit);
     pc->sub_on = keep;
     return true;
 }
@@ -1408,15 +1547,13 @@ static long long plan_check(sg_precond* pc, const RingPlan& plan, int plant) {
     std::vector<unsigned char> rec((size_t)pc->rec_total);
     SG_CUDA(cudaMemcpyAsync(rec.data(), pc->rec_d.p, rec.size(), cudaMemcpyDeviceToHost, st));
     SG_CUDA(cudaStreamSynchronize(st));
-    const long long sf = pc->opts.sweep_dtype == SG_FP64 ? 8
-                         : (pc->opts.factor_dtype == SG_BF16 ? 2 : 4);
+    const int sf = rec_value_bytes(pc);
     const RingSub* subs = reinterpret_cast<const RingSub*>(plan.sub.data());
-    const int* meta = plan.meta.data();
+    const int* ent = plan.ent.data();
     const int* grp = plan.grp.data();
     long long bad = 0;
     bool planted = false;
     std::vector<char> done;
-    std::vector<int> last_level, first_level;
     for (int s = 0; s < pc->nparts; ++s) {
         const SubInfo& inf = pc->h_info[s];
         const RingSub& r = subs[s];
@@ -1435,90 +1572,110 @@ static long long plan_check(sg_precond* pc, const RingPlan& plan, int plant) {
                 const int c = dir == 0 ? pc->h_lev_ptr_f[i + 1] - pc->h_lev_ptr_f[i]
                                        : pc->h_lev_ptr_b[i + 1] - pc->h_lev_ptr_b[i];
                 const int C = dir == 0 ? pc->h_rec_rows_f[i] : pc->h_rec_rows_b[i];
+                const int nq = pc->rec_rows && rec_is_rows(w) ? c + 1 : c;
                 const long long off = dir == 0 ? pc->h_rec_off_f[i] : pc->h_rec_off_b[i];
-                const long long bytes = (long long)C * (2 + w * (2 + sf) + (dir ? sf : 0));
+                const long long bytes = rec_level_bytes(pc, w, dir != 0, c);
                 if (C % 8 || c > C || off < 0 || off + bytes > pc->rec_total) {
                     ++bad;
                     continue;
                 }
-                uint16_t* rows = reinterpret_cast<uint16_t*>(rec.data() + off);
-                uint16_t* cols = rows + C;
+                // slot k of row q: the row itself (0) or its column k - 1
+                const bool rows_rec = pc->rec_rows && rec_is_rows(w);
+                const int rb = rec_row_bytes(w, dir != 0, sf);
+                auto slot = [&](int q, int k) -> uint16_t& {
+                    unsigned char* R = rec.data() + off;
+                    return rows_rec ? reinterpret_cast<uint16_t*>(R + (size_t)q * rb)[k]
+                                    : reinterpret_cast<uint16_t*>(R)[(size_t)k * C + q];
+                };
                 if (plant && !planted && l > 0 && c > 0 && w > 0) {
-                    cols[0] = (uint16_t)rows[0];  // a row reading itself: not yet computed
+                    slot(0, 1) = slot(0, 0);  // a row reading itself: not yet computed
                     planted = true;
                 }
-                for (int q = 0; q < c; ++q) {
-                    const int rs = rows[q];
+                for (int q = 0; q < nq; ++q) {
+                    const int rs = slot(q, 0);
+                    if (q == c) {  // the row past the end: the unused slot only
+                        for (int k = 0; k <= w; ++k)
+                            if (slot(q, k) != zero_slot) ++bad;
+                        continue;
+                    }
                     if (rs >= zero_slot || !real[rs]) {
                         ++bad;
                         continue;
                     }
                     for (int k = 0; k < w; ++k) {
-                        const int cs = cols[(size_t)k * C + q];
+                        const int cs = slot(q, k + 1);
                         if (cs > zero_slot) ++bad;
                         else if (cs != zero_slot && (!real[cs] || !done[cs])) ++bad;
                     }
                 }
                 for (int q = 0; q < c; ++q)
-                    if (rows[q] < zero_slot) done[rows[q]] = 1;
+                    if (slot(q, 0) < zero_slot) done[slot(q, 0)] = 1;
             }
         }
         // ---- ring schedule: simulate the producer and the level loop
         const int G = r.ngrp;
-        last_level.assign(G, -1);
-        first_level.assign(G, -1);
-        int cur = -1;
-        for (int g = 0; g < T; ++g) {
-            const int* m = meta + 4 * ((size_t)r.meta_off + g);
-            if (m[2] >= 0) {
-                if (m[2] != cur + 1) ++bad;  // groups open in order
-                cur = m[2];
-                first_level[cur] = g;
-            }
-            if (cur < 0 || cur >= G) {
-                ++bad;
-                break;
-            }
-            last_level[cur] = g;
-        }
-        int issued = r.ninit;
-        if (issued > G) ++bad;
-        for (int g = 0; g < T && cur >= 0; ++g) {
-            const int* m = meta + 4 * ((size_t)r.meta_off + g);
-            int j = 0;
-            while (j + 1 < G && first_level[j + 1] >= 0 && first_level[j + 1] <= g) ++j;
-            const int c = m[0] & 0xffff, C = (int)((unsigned)m[0] >> 16);
-            const bool back = g >= nf;
-            const int i = back ? inf.lev_off_b + (g - nf) : inf.lev_off_f + g;
-            const long long B = (long long)C * (back ? 2 + inf.wu * (2 + sf) + sf : 2 + inf.wl * (2 + sf));
-            const long long rel = (back ? pc->h_rec_off_b[i] : pc->h_rec_off_f[i]) - r.base;
-            const int* gj = grp + 2 * ((size_t)r.grp_off + j);
+        int issued = r.ninit, e = 0, g = 0;  // groups issued, entry, level
+        if (issued > G || r.ngrp_f > G) ++bad;
+        for (int j = 0; j < G; ++j) {
+            const int* gj = grp + 4 * ((size_t)r.grp_off + j);
             const long long gstart = (unsigned)gj[0];
             const long long gbytes = (long long)(((unsigned)gj[1] & 0xffffu) << 4);
             const long long gpos = (long long)(((unsigned)gj[1] >> 16) << 4);
-            if (c != (back ? pc->h_lev_ptr_b[i + 1] - pc->h_lev_ptr_b[i]
-                           : pc->h_lev_ptr_f[i + 1] - pc->h_lev_ptr_f[i]))
+            if (j >= issued) ++bad;  // waits for a copy not yet issued
+            if (gj[2] != e || gpos + gbytes > plan.ring_bytes) ++bad;
+            const int e1 = gj[4 + 2] - 1;  // the entry that ends it
+            if (e1 >= r.nent || e1 < e) {
                 ++bad;
-            if (m[1] < gpos || m[1] + B > gpos + gbytes || m[1] + B > plan.ring_bytes) ++bad;
-            if (rel - gstart != m[1] - gpos) ++bad;  // the ring copy holds this record
-            if (m[2] >= 0 && m[2] >= issued) ++bad;  // waits for a copy not yet issued
-            // issue after the level: what the new groups overwrite must be done
-            for (int k = issued; k < m[3] && k < G; ++k) {
-                const int* gk = grp + 2 * ((size_t)r.grp_off + k);
+                break;
+            }
+            while (e < e1 && g < T) {
+                const bool back = g >= nf;
+                if (back != (j >= r.ngrp_f)) ++bad;
+                const int i = back ? inf.lev_off_b + (g - nf) : inf.lev_off_f + g;
+                const int w = back ? inf.wu : inf.wl;
+                const int c = back ? pc->h_lev_ptr_b[i + 1] - pc->h_lev_ptr_b[i]
+                                   : pc->h_lev_ptr_f[i + 1] - pc->h_lev_ptr_f[i];
+                const long long B = rec_level_bytes(pc, w, back, c);
+                const long long rel = (back ? pc->h_rec_off_b[i] : pc->h_rec_off_f[i]) - r.base;
+                const bool rows = pc->rec_rows && rec_is_rows(w);
+                const int step = rows ? plan.level_threads : c, rb = rec_row_bytes(w, back, sf);
+                // the ring copy holds the whole record, in this group's bytes
+                const long long at = gpos + rel - gstart;
+                if (rel < gstart || rel + B > gstart + gbytes) ++bad;
+                for (int q = 0; q < c && e < e1; q += step, ++e) {
+                    const int* m = ent + 2 * ((size_t)r.ent_off + e);
+                    if ((m[0] & 0xffff) != c - q || (m[0] >> 16) != (q + step >= c ? 1 : 0) ||
+                        m[1] != at + (rows ? (long long)q * rb : 0))
+                        ++bad;
+                }
+                ++g;
+            }
+            if (e != e1 || ent[2 * ((size_t)r.ent_off + e1)] != 0) ++bad;
+            e = e1 + 1;
+            // issued after group j: what the new groups overwrite must be done
+            for (int k = issued; k < gj[3] && k < G; ++k) {
+                const int* gk = grp + 4 * ((size_t)r.grp_off + k);
                 const long long kb = (long long)(((unsigned)gk[1] & 0xffffu) << 4);
                 const long long kp = (long long)(((unsigned)gk[1] >> 16) << 4);
-                for (int q = 0; q < k; ++q) {
-                    if (last_level[q] <= g) continue;  // finished: its bytes are free
-                    const int* gq = grp + 2 * ((size_t)r.grp_off + q);
+                for (int q = j + 1; q < k; ++q) {
+                    const int* gq = grp + 4 * ((size_t)r.grp_off + q);
                     const long long qb = (long long)(((unsigned)gq[1] & 0xffffu) << 4);
                     const long long qp = (long long)(((unsigned)gq[1] >> 16) << 4);
                     if (kp < qp + qb && qp < kp + kb) ++bad;
                 }
-                if (k >= RING_NBAR && last_level[k - RING_NBAR] > g) ++bad;
+                if (k >= RING_NBAR && k - RING_NBAR > j) ++bad;
             }
-            if (m[3] > issued) issued = m[3];
+            if (gj[3] > issued) issued = gj[3];
         }
-        if (issued != G && T > 0) ++bad;  // every group issued by the end
+        if (g != T || (issued != G && T > 0)) ++bad;  // every level, every group
+        // groups issued at once never overlap each other
+        for (int k = 0; k < r.ninit && k < G; ++k)
+            for (int q = 0; q < k; ++q) {
+                const int *gk = grp + 4 * ((size_t)r.grp_off + k), *gq = grp + 4 * ((size_t)r.grp_off + q);
+                const long long kb = (long long)(((unsigned)gk[1] & 0xffffu) << 4), kp = (long long)(((unsigned)gk[1] >> 16) << 4);
+                const long long qb = (long long)(((unsigned)gq[1] & 0xffffu) << 4), qp = (long long)(((unsigned)gq[1] >> 16) << 4);
+                if (kp < qp + qb && qp < kp + kb) ++bad;
+            }
     }
     if (plant && !planted) ++bad;  // nothing to corrupt: report it as found
     return bad;

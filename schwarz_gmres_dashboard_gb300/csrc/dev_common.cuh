@@ -377,4 +377,107 @@ __device__ __forceinline__ bool last_block_reduce(double* partials, unsigned* co
     return true;
 }
 
+// ----------------------------------------------------- cluster-level reductions
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the double at shared address `p` of the cluster's CTA `rank`
+__device__ __forceinline__ double ld_cluster(const double* p, unsigned rank) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    uint32_t r;
+    double v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(r) : "memory");
+    return v;
+}
+
+// Grid-level completion of a reduction of nv <= 32 block sums (bs, shared and
+// visible to the block) by kernels launched in clusters of at most 8 blocks of
+// at least 8 warps.  The FP64 pipe of one SM adds two values a cycle, so a
+// last block that added every block's sums by itself was the longest part of
+// a reduction (608 blocks x 30 sums: 15 us); here the clusters' first blocks add
+// their own cluster's sums through distributed shared memory, and the last of
+// them to arrive adds one set per cluster, a lane per value and a warp per
+// eighth of the clusters (148 clusters of 4 x 30: under 5 us).  Orders are fixed: cluster
+// rank, then cluster index within a warp, then warps.  Returns true in that
+// block, with the totals in `out`; no block waits for a block of another
+// cluster.  One cluster needs no global memory at all.
+constexpr int CL_MAX = 8;   // largest cluster; also the warps that add the clusters' sums
+constexpr int CL_SIZE = 4;  // of a grid of several clusters
+__device__ __forceinline__ bool cluster_reduce(double* partials, unsigned* counter,
+                                               const double* bs, int nv, double* out) {
+    __shared__ unsigned s_ticket;
+    __shared__ double scr[CL_MAX][32];
+    const unsigned rank = cluster_rank(), nr = cluster_size();
+    const unsigned cid = blockIdx.x / nr, nc = gridDim.x / nr;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (nr > 1) {
+        cluster_arrive();
+        cluster_wait();
+    }
+    if (rank == 0 && warp == 0 && lane < nv) {
+        double v[CL_MAX];
+#pragma unroll
+        for (int r = 0; r < CL_MAX; ++r) v[r] = r < (int)nr ? ld_cluster(bs + lane, r) : 0.0;
+        const double t = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        if (nc == 1) out[lane] = t;
+        else partials[(size_t)cid * nv + lane] = t;
+    }
+    __syncwarp();
+    if (nr > 1) {
+        cluster_arrive();
+        if (rank != 0) {  // its shared memory is read until here
+            cluster_wait();
+            return false;
+        }
+    }
+    if (nc == 1) {
+        __syncthreads();
+        return true;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_ticket = atomicAdd(counter, 1u);
+    __syncthreads();
+    if (s_ticket != nc - 1) return false;
+    __threadfence();
+    if (warp < CL_MAX) {
+        double a = 0.0;
+        for (unsigned c0 = warp; c0 < nc; c0 += 4 * CL_MAX) {
+            double v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const unsigned c = c0 + q * CL_MAX;
+                v[q] = c < nc && lane < nv ? __ldcg(&partials[(size_t)c * nv + lane]) : 0.0;
+            }
+            a += (v[0] + v[1]) + (v[2] + v[3]);
+        }
+        scr[warp][lane] = a;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double v[CL_MAX];
+#pragma unroll
+        for (int r = 0; r < CL_MAX; ++r) v[r] = scr[r][lane];
+        if (lane < nv)
+            out[lane] = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        if (lane == 0) *counter = 0u;
+    }
+    __syncthreads();
+    return true;
+}
+
 }  // namespace sg

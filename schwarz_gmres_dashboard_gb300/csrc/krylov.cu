@@ -11,10 +11,16 @@
 //   A  h1 = V^T w                          (dot products, one pass)
 //   B  w' = w - V h1 ; h2 = V^T w'          (update and second dots, one pass)
 //   C  w'' = w' - V h2 ; ||w''||           (update and norm, one pass)
-// Every pass reduces per block, and the last block to finish sums the block
-// partials in block order; after pass C it also writes the Hessenberg column,
-// applies the Givens rotations (same formulas as src/core/gmres.cpp:9-30)
-// and tests convergence, so no value travels to the host inside a cycle.
+// Every pass reduces per block, per cluster, and in the last cluster to finish
+// (cluster_reduce); after the last pass that block also writes the Hessenberg
+// column, applies the Givens rotations (the reference's, src/core/
+// gmres.cpp:9-30) and tests convergence, so no value travels to the host
+// inside a cycle.  These ends of a pass are chains of FP64 operations on one
+// SM (~75 cycles each when dependent, ~400-560 for a root or a quotient), so
+// they are arranged for depth: matrix-vector products take a lane per row and
+// four sums per lane, the earlier rotations run as a parallel prefix.
+#include <algorithm>
+
 #include "dev_common.cuh"
 #include "kernels.h"
 
@@ -25,30 +31,23 @@ namespace {
 constexpr int KT = 256;    // threads of the Krylov kernels
 constexpr int BS_T = 256;  // threads of the back substitution (loads; one warp solves)
 
-// Givens rotation of src/core/gmres.cpp:9-30
-__device__ void rot_compute(double& c, double& s, double a, double b) {
+// Givens rotation of src/core/gmres.cpp:9-30 (1 / sqrt(1 + t^2) as one rsqrt:
+// one rounding less)
+__device__ __forceinline__ void rot_compute(double& c, double& s, double a, double b) {
     if (fabs(b) < 1e-30) {
         c = 1.0;
         s = 0.0;
-    } else if (fabs(b) > fabs(a)) {
-        const double t = -a / b;
-        s = 1.0 / sqrt(1.0 + t * t);
-        c = s * t;
-    } else {
-        const double t = -b / a;
-        c = 1.0 / sqrt(1.0 + t * t);
-        s = c * t;
+        return;
     }
-}
-__device__ void rot_apply(double c, double s, double& h1, double& h2) {
-    const double t1 = c * h1 - s * h2;
-    const double t2 = s * h1 + c * h2;
-    h1 = t1;
-    h2 = t2;
+    const bool big = fabs(b) > fabs(a);
+    const double t = -(big ? a : b) / (big ? b : a);
+    const double r = rsqrt(1.0 + t * t);
+    c = big ? r * t : r;
+    s = big ? r : r * t;
 }
 
-// State the serial end of an Arnoldi step reads, brought to shared memory
-// (and, for thread 0, registers) in one round of loads: the column h(0..j),
+// State the end of an Arnoldi step reads, brought to shared memory in one round
+// of loads: the column h(0..j),
 // the earlier rotations, g(j..j+1) and the stopping-test scalars.
 struct FinalizeIn {
     double hc[SG_MMAX + 2], csv[SG_MMAX], snv[SG_MMAX], gv[2];
@@ -56,88 +55,131 @@ struct FinalizeIn {
     int tol_kind, hist_len, total_iter;
 };
 
-// all threads of the block: loads everything but hc (the caller's column)
+// global -> shared without a register in between: the issuing warp goes on
+template <class T>
+__device__ __forceinline__ void cp_async(T* dst, const T* src) {
+    static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async sizes");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"((int)sizeof(T))
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// all threads of the block: starts to load everything but hc (the caller's
+// column); the caller waits (cp_async_wait, then a barrier)
 __device__ __forceinline__ void finalize_load(FinalizeIn& f, const SolveState* st, int j) {
     for (int i = threadIdx.x; i < j; i += blockDim.x) {
-        f.csv[i] = st->cs[i];
-        f.snv[i] = st->sn[i];
+        cp_async(&f.csv[i], &st->cs[i]);
+        cp_async(&f.snv[i], &st->sn[i]);
     }
     if (threadIdx.x == 0) {
-        f.gv[0] = st->g[j];
-        f.gv[1] = st->g[j + 1];
-        f.tol = st->tol;
-        f.bnorm = st->bnorm;
-        f.est_scale = st->est_scale;
-        f.tol_kind = st->tol_kind;
-        f.hist_len = st->hist_len;
-        f.total_iter = st->total_iter;
+        cp_async(&f.gv[0], &st->g[j]);
+        cp_async(&f.gv[1], &st->g[j + 1]);
+        cp_async(&f.tol, &st->tol);
+        cp_async(&f.bnorm, &st->bnorm);
+        cp_async(&f.est_scale, &st->est_scale);
+        cp_async(&f.tol_kind, &st->tol_kind);
+        cp_async(&f.hist_len, &st->hist_len);
+        cp_async(&f.total_iter, &st->total_iter);
     }
 }
 
-// Thread 0: completes Arnoldi step j from f (hc[0..j] holds the column) and
-// ss = ||w''||^2: normalisation, Givens rotations, residual estimate and
-// stopping test.  Returns the new vector's scale 1/||w''|| when the cycle
-// goes on, 0 when it stops here (breakdown, convergence, last step).
-__device__ double finalize_core(SolveState* st, FinalizeIn& f, int j, int m, double ss,
-                                double* hist, int hist_cap) {
-    const int ld = m + 1;
-    double* hc = f.hc;
-    const double nrm = sqrt(ss);
-    double* Hc = st->H + (size_t)j * ld;
-    hc[j + 1] = nrm;
-    if (!(nrm >= 1e-30)) {
-        // breakdown (src/core/gmres.cpp:297-300): this column is used as is
-        for (int i = 0; i <= j + 1; ++i) Hc[i] = hc[i];
-        if (!isfinite(nrm)) {
+// One warp: the column's earlier rotations.  Rotation i maps the carried entry
+// a_i (a_0 = h_0) to a_{i+1} = s_i a_i + c_i h_{i+1} and leaves r_i = c_i a_i -
+// s_i h_{i+1}: the carried entries are a prefix of affine maps, formed in five
+// steps for 32 rotations instead of one after another.  Writes r_0..r_{j-1}
+// to H's column j and returns a_j.
+__device__ double rotate_column(SolveState* st, const FinalizeIn& f, int j, int m) {
+    const int lane = threadIdx.x & 31;
+    const double* hc = f.hc;
+    double* Hc = st->H + (size_t)j * (m + 1);
+    double a = hc[0];
+    for (int i0 = 0; i0 < j; i0 += 32) {
+        const int i = i0 + lane;
+        const bool in = i < j;
+        const double c = in ? f.csv[i] : 1.0, sn = in ? f.snv[i] : 0.0, hn = in ? hc[i + 1] : 0.0;
+        double A = in ? sn : 1.0, B = in ? c * hn : 0.0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double pA = __shfl_up_sync(0xffffffffu, A, o);
+            const double pB = __shfl_up_sync(0xffffffffu, B, o);
+            if (lane >= o) {
+                B = fma(A, pB, B);
+                A *= pA;
+            }
+        }
+        const double next = fma(A, a, B);
+        double cur = __shfl_up_sync(0xffffffffu, next, 1);
+        if (lane == 0) cur = a;
+        if (in) Hc[i] = fma(c, cur, -(sn * hn));
+        a = __shfl_sync(0xffffffffu, next, 31);
+    }
+    return a;
+}
+
+// The same warp: completes Arnoldi step j from a = rotate_column and ss =
+// ||w''||^2: normalisation, the new rotation, residual estimate and stopping
+// test.  Returns the new vector's scale 1/||w''|| when the cycle goes on, 0
+// when it stops here (breakdown, convergence, last step); nrm = ||w''||.
+__device__ double finalize_warp(SolveState* st, const FinalizeIn& f, int j, int m, double a,
+                                double ss, double* hist, int hist_cap, double& nrm) {
+    const int lane = threadIdx.x & 31;
+    double* Hc = st->H + (size_t)j * (m + 1);
+    if (!(ss >= 1e-60)) {
+        // breakdown, ||w''|| < 1e-30 (src/core/gmres.cpp:297-300): this column is used as is
+        nrm = sqrt(ss);
+        __syncwarp();
+        for (int i = lane; i <= j + 1; i += 32) Hc[i] = i <= j ? f.hc[i] : nrm;
+        if (lane == 0) {
+            if (!isfinite(nrm)) {
+                st->nonfinite = 1;
+                st->done = 1;
+            }
+            st->breakdown = 1;
+            st->kcount = j + 1;
+            st->cycle_active = 0;
+        }
+        return 0.0;
+    }
+    const double vs = rsqrt(ss);
+    nrm = ss * vs;
+    double c, sn;
+    rot_compute(c, sn, a, nrm);
+    const double g0 = f.gv[0], g1 = f.gv[1];
+    const double gj = c * g0 - sn * g1, gn = sn * g0 + c * g1;
+    const double res = fabs(gn);
+    // the stopping tests: the reference's rule, or the estimated true residual
+    // (which the restart verifies in FP64)
+    const bool conv = f.tol_kind == SG_TOL_REF_ABS && res < f.tol;
+    const bool bad = !isfinite(res);
+    const bool stop = conv || bad || j + 1 >= m ||
+                      (f.tol_kind == SG_TOL_TRUE_REL && res * f.est_scale <= 0.5 * f.tol * f.bnorm);
+    if (lane == 0) {
+        st->vscale[j + 1] = vs;
+        Hc[j] = c * a - sn * nrm;
+        Hc[j + 1] = sn * a + c * nrm;
+        st->cs[j] = c;
+        st->sn[j] = sn;
+        st->g[j] = gj;
+        st->g[j + 1] = gn;
+        if (hist && f.hist_len < hist_cap) hist[f.hist_len] = res;
+        st->hist_len = f.hist_len + 1;
+        st->last_res = res;
+        st->total_iter = f.total_iter + 1;
+        st->kcount = j + 1;
+        st->j = j + 1;
+        if (conv) {
+            st->converged = 1;
+            st->done = 1;
+        }
+        if (bad) {
             st->nonfinite = 1;
             st->done = 1;
         }
-        st->breakdown = 1;
-        st->kcount = j + 1;
-        st->cycle_active = 0;
-        return 0.0;
+        if (stop) st->cycle_active = 0;
     }
-    const double vs = 1.0 / nrm;
-    st->vscale[j + 1] = vs;
-    for (int i = 0; i < j; ++i) rot_apply(f.csv[i], f.snv[i], hc[i], hc[i + 1]);
-    double c, sn;
-    rot_compute(c, sn, hc[j], hc[j + 1]);
-    rot_apply(c, sn, hc[j], hc[j + 1]);
-    rot_apply(c, sn, f.gv[0], f.gv[1]);
-    st->cs[j] = c;
-    st->sn[j] = sn;
-    st->g[j] = f.gv[0];
-    st->g[j + 1] = f.gv[1];
-    for (int i = 0; i <= j + 1; ++i) Hc[i] = hc[i];
-    const double res = fabs(f.gv[1]);
-    if (hist && f.hist_len < hist_cap) hist[f.hist_len] = res;
-    st->hist_len = f.hist_len + 1;
-    st->last_res = res;
-    st->total_iter = f.total_iter + 1;
-    st->kcount = j + 1;
-    st->j = j + 1;
-    bool stop = false;
-    if (f.tol_kind == SG_TOL_REF_ABS) {
-        if (res < f.tol) {
-            st->converged = 1;
-            st->done = 1;
-            stop = true;
-        }
-    } else if (f.tol_kind == SG_TOL_TRUE_REL) {
-        // estimated true residual; the restart verifies it in FP64
-        if (res * f.est_scale <= 0.5 * f.tol * f.bnorm) stop = true;
-    }
-    if (!isfinite(res)) {
-        st->nonfinite = 1;
-        st->done = 1;
-        stop = true;
-    }
-    if (j + 1 >= m) stop = true;
-    if (stop) {
-        st->cycle_active = 0;
-        return 0.0;
-    }
-    return vs;
+    return stop ? 0.0 : vs;
 }
 
 // Completes Arnoldi step j once ||w''||^2 is known (all threads of the last
@@ -145,10 +187,15 @@ __device__ double finalize_core(SolveState* st, FinalizeIn& f, int j, int m, dou
 __device__ void arnoldi_finalize(SolveState* st, int j, int m, double ss, double* hist,
                                  int hist_cap) {
     __shared__ FinalizeIn f;
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) f.hc[i] = st->hsum[i];
+    for (int i = threadIdx.x; i <= j; i += blockDim.x) cp_async(&f.hc[i], &st->hsum[i]);
     finalize_load(f, st, j);
+    cp_async_wait();
     __syncthreads();
-    if (threadIdx.x == 0) finalize_core(st, f, j, m, ss, hist, hist_cap);
+    if (threadIdx.x < 32) {
+        double nrm;
+        const double a = rotate_column(st, f, j, m);
+        finalize_warp(st, f, j, m, a, ss, hist, hist_cap, nrm);
+    }
 }
 
 template <class T>
@@ -195,18 +242,39 @@ __device__ __forceinline__ void vstore<float>(float* p, const float (&o)[4]) {
 // with few vectors still keeps every warp loading.
 constexpr int KW = KT / 32;  // warps per block
 constexpr int KPW = 4;       // basis vectors per warp
+constexpr int DOTS_PER_SM = 4, UPD_PER_SM = 3;  // resident blocks of the two passes
 
-// warps per tile group: the fewest that hold kc vectors at KPW per warp
-__device__ __forceinline__ int warps_per_tile(int kc) {
-    return kc <= KPW ? 1 : (kc <= 2 * KPW ? 2 : (kc <= 4 * KPW ? 4 : 8));
+// warps per tile group (the kernels' NWG): the fewest that hold kc vectors at
+// KPW per warp
+int warps_per_tile(int kc) { return kc <= KPW ? 1 : (kc <= 2 * KPW ? 2 : (kc <= 4 * KPW ? 4 : 8)); }
+
+// acc + a . b, one multiply-add per element (FP64 ones are the scarce resource)
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+template <class TV>
+__device__ __forceinline__ TV dotv(const TV (&a)[Vec<TV>::N], const TV (&b)[Vec<TV>::N], TV acc) {
+#pragma unroll
+    for (int e = 0; e < Vec<TV>::N; ++e) acc = fma_t(a[e], b[e], acc);
+    return acc;
 }
 
+// the warp sums of four values at once: each of the first two exchanges halves
+// the values a lane holds (6 additions a lane instead of 20); the sum of value
+// (lane >> 3) is in every lane of that eighth
 template <class TV>
-__device__ __forceinline__ TV dotv(const TV (&a)[Vec<TV>::N], const TV (&b)[Vec<TV>::N]) {
-    TV s = (TV)0;
-#pragma unroll
-    for (int e = 0; e < Vec<TV>::N; ++e) s += a[e] * b[e];
-    return s;
+__device__ __forceinline__ TV warp_sum4(const TV (&v)[KPW]) {
+    static_assert(KPW == 4, "two halvings");
+    const int lane = threadIdx.x & 31;
+    const bool h1 = lane & 16, h2 = lane & 8;
+    TV a = h1 ? v[2] : v[0], b = h1 ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, h1 ? v[0] : v[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, h1 ? v[1] : v[3], 16);
+    TV r = h2 ? b : a;
+    r += __shfl_xor_sync(0xffffffffu, h2 ? a : b, 8);
+    r += __shfl_xor_sync(0xffffffffu, r, 4);
+    r += __shfl_xor_sync(0xffffffffu, r, 2);
+    r += __shfl_xor_sync(0xffffffffu, r, 1);
+    return r;
 }
 
 // per-warp accumulators -> block sums bs[k] (k < kc): the warp trees run in
@@ -216,11 +284,8 @@ template <class TV>
 __device__ __forceinline__ void group_sums(const TV (&acc)[KPW], int kc, int nwg, double* bs) {
     __shared__ double red[KW][KPW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < KPW; ++q) {
-        const double v = (double)warp_sum(acc[q]);
-        if (lane == 0) red[warp][q] = v;
-    }
+    const double v = (double)warp_sum4<TV>(acc);
+    if ((lane & 7) == 0) red[warp][lane >> 3] = v;
     __syncthreads();
     if ((int)threadIdx.x < kc) {
         const int k = threadIdx.x, slot = k % nwg, q = k / nwg;
@@ -256,121 +321,133 @@ __device__ __forceinline__ void group_sync(int grp, int nwg) {
 //      stored as raw_{j+1} with its pending correction c = h2 / ||w''||.
 // In exact arithmetic this is CGS2; the stored vectors are never rewritten.
 
-// the leading n x n block of the column-major SG_LAGM matrix M into
-// shared memory (upper triangle only when `upper`)
-__device__ __forceinline__ void stage_lag(double (*dst)[SG_LAGM + 1], const double* M, int n,
-                                          int ncol, bool upper) {
-    for (int idx = threadIdx.x; idx < n * ncol; idx += blockDim.x) {
-        const int i = idx % n, k = idx / n;
-        dst[i][k] = (!upper || i <= k) ? M[i + k * SG_LAGM] : 0.0;
+// What the ends of the two passes read from the state.  The first block of
+// every cluster starts to copy it when the kernel starts (cp.async, waited
+// for at the end: none of it changes during the kernel), so the block that
+// gets there last finds it in shared memory.  T and H keep their zeros below
+// the (sub)diagonal, so whole rows are summed.
+struct LagIn {
+    double T[SG_LAGM][SG_LAGM + 1];   // T(l, i) at [i][l]
+    double Tt[SG_LAGM][SG_LAGM + 1];  // T(l, i) at [l][i]
+    double H[SG_LAGM][SG_LAGM + 1];   // pass A: the unrotated Hessenberg, H(i, k) at [k][i]
+    double c[SG_LAGM];                // pass A: the pending correction
+    FinalizeIn f;                     // pass B
+};
+__device__ __forceinline__ void lag_prefetch(LagIn& in, const SolveState* st, int j, bool pass_b) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = warp; i <= j; i += KT / 32) {
+        if (lane <= j) {
+            cp_async(&in.T[i][lane], &st->lagT[lane + i * SG_LAGM]);
+            cp_async(&in.Tt[lane][i], &st->lagT[lane + i * SG_LAGM]);
+        }
+        if (!pass_b && i < j && lane <= j) cp_async(&in.H[i][lane], &st->lagH[lane + i * SG_LAGM]);
+    }
+    if (pass_b) {
+        for (int i = threadIdx.x; i <= j; i += KT) cp_async(&in.f.hc[i], &st->hsum[i]);
+        finalize_load(in.f, st, j);
+    } else if (warp == 0 && lane < j) {
+        cp_async(&in.c[lane], &st->lagc[lane]);
     }
 }
 
-// what the pass A epilogue reads from the state (T, the lagged Hessenberg
-// block, the pending correction), loaded by the last block with its partials
-struct LagAIn {
-    double Ts[SG_LAGM][SG_LAGM + 1], Hs[SG_LAGM][SG_LAGM + 1];
-    double cs[SG_LAGM];
-};
-__device__ __forceinline__ void lagged_a_load(LagAIn& in, const SolveState* st, int j) {
-    const int n1 = j + 1;
-    stage_lag(in.Ts, st->lagT, n1, n1, true);
-    stage_lag(in.Hs, st->lagH, n1, j, false);
-    for (int i = threadIdx.x; i < j; i += blockDim.x) in.cs[i] = st->lagc[i];
+// sum_k M[k][lane] x[k] over k < n (one warp; a lane per row, four sums each)
+__device__ __forceinline__ double lag_rows(const double (*M)[SG_LAGM + 1], const double* x,
+                                           int n) {
+    const int lane = threadIdx.x & 31;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    int k = 0;
+    for (; k + 4 <= n; k += 4) {
+        s0 = fma(M[k][lane], x[k], s0);
+        s1 = fma(M[k + 1][lane], x[k + 1], s1);
+        s2 = fma(M[k + 2][lane], x[k + 2], s2);
+        s3 = fma(M[k + 3][lane], x[k + 3], s3);
+    }
+    if (k < n) s0 = fma(M[k][lane], x[k], s0);
+    if (k + 1 < n) s1 = fma(M[k + 1][lane], x[k + 1], s1);
+    if (k + 2 < n) s2 = fma(M[k + 2][lane], x[k + 2], s2);
+    return (s0 + s1) + (s2 + s3);
 }
-
-// pass A epilogue (all threads of the last block; d = tot[0..j], `in` loaded
-// and visible): p = T^T d, hsum = p - g, update coefficients u = T p
-__device__ void lagged_pass_a(SolveState* st, int j, const double* d, const LagAIn& in) {
+// pass A's end (all threads of the last block; d = tot[0..j]): p = T^T d,
+// hsum = p - g with g = H c, update coefficients u = T p
+__device__ void lagged_pass_a(SolveState* st, int j, const double* d, const LagIn& in) {
     __shared__ double p_s[SG_LAGM];
-    const auto& Ts = in.Ts;
-    const auto& Hs = in.Hs;
-    const double* cs = in.cs;
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) {
-        double s = 0.0;
-        for (int l = 0; l <= i; ++l) s += Ts[l][i] * d[l];
-        p_s[i] = s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double g = 0.0;
+    if (warp == 0) {
+        const double p = lag_rows(in.Tt, d, j + 1);
+        if (lane <= j) p_s[lane] = p;
+    } else if (warp == 1) {
+        if (lane <= j) g = lag_rows(in.H, in.c, j);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) {
-        double g = 0.0;
-        for (int k = (i > 0 ? i - 1 : 0); k < j; ++k) g += Hs[i][k] * cs[k];
-        st->h[i] = p_s[i];
-        st->hsum[i] = p_s[i] - g;
-        double u = 0.0;
-        for (int k = i; k <= j; ++k) u += Ts[i][k] * p_s[k];
-        st->cfu[i] = u;
-    }
-    __syncthreads();
+    if (lane > j) return;
+    if (warp == 0) st->cfu[lane] = lag_rows(in.T, p_s, j + 1);
+    if (warp == 1) st->hsum[lane] = p_s[lane] - g;
 }
 
-// pass B epilogue (all threads of the last block; r = tot[0..j], ss =
-// ||w'||^2).  Everything it reads from the state (T, the column's pass A
-// part, the rotations, g, the stopping-test scalars) is loaded by
-// lagged_b_load with the partials; the step's end runs on thread 0 from
-// shared memory.
-struct LagBIn {
-    double Ts[SG_LAGM][SG_LAGM + 1];
-    FinalizeIn f;
-};
-__device__ __forceinline__ void lagged_b_load(LagBIn& in, const SolveState* st, int j) {
-    const int n1 = j + 1;
-    stage_lag(in.Ts, st->lagT, n1, n1, true);
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) in.f.hc[i] = st->hsum[i];
-    finalize_load(in.f, st, j);
-}
-
+// pass B's end (all threads of the last block; r = tot[0..j], ss =
+// ||w'||^2): h2 = T^T r, the column hsum + h2, its rotations (warp 0), the new
+// norm (warp 2), the step's end (warp 0), the new vector's pending correction
+// and T column (warp 1)
 __device__ void lagged_pass_b(SolveState* st, int j, int m, const double* r, double ss,
-                              double* hist, int hist_cap, LagBIn& in) {
-    __shared__ double h2_s[SG_LAGM], c_s[SG_LAGM];
-    __shared__ double s_vs;
-    const auto& Ts = in.Ts;
-    FinalizeIn& f = in.f;
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) {
-        double s = 0.0;
-        for (int l = 0; l <= i; ++l) s += Ts[l][i] * r[l];
-        h2_s[i] = s;
-        const double hs = f.hc[i] + s;  // the Hessenberg column
-        f.hc[i] = hs;
-        st->hsum[i] = hs;
-        st->lagH[i + j * SG_LAGM] = hs;
+                              double* hist, int hist_cap, LagIn& in) {
+    __shared__ double h2_s[SG_LAGM];
+    __shared__ double s_vs, s_n2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double a = 0.0, tc = 0.0;
+    if (warp == 0) {
+        const double h2 = lag_rows(in.Tt, r, j + 1);
+        if (lane <= j) {
+            h2_s[lane] = h2;
+            const double hs = in.f.hc[lane] + h2;  // the Hessenberg column
+            in.f.hc[lane] = hs;
+            st->hsum[lane] = hs;
+            st->lagH[lane + j * SG_LAGM] = hs;
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double nrm2 = ss;
-        for (int i = 0; i <= j; ++i) nrm2 -= h2_s[i] * h2_s[i];
+    if (warp == 0) {
+        a = rotate_column(st, in.f, j, m);
+    } else if (warp == 1) {
+        if (lane <= j) tc = lag_rows(in.T, h2_s, j + 1);
+    } else if (warp == 2) {
+        const double h2 = lane <= j ? h2_s[lane] : 0.0;
+        double nrm2 = ss - warp_sum(h2 * h2);
         if (!(nrm2 > 0.0)) nrm2 = isfinite(nrm2) ? 0.0 : nrm2;
-        st->lagH[j + 1 + j * SG_LAGM] = sqrt(nrm2);
-        const double vs = finalize_core(st, f, j, m, nrm2, hist, hist_cap);
-        s_vs = j + 1 < SG_LAGM ? vs : 0.0;
+        if (lane == 0) s_n2 = nrm2;
     }
     __syncthreads();
-    // the pending correction of the new stored vector
+    if (warp == 0) {
+        double nrm;
+        const double vs = finalize_warp(st, in.f, j, m, a, s_n2, hist, hist_cap, nrm);
+        if (lane == 0) {
+            st->lagH[j + 1 + j * SG_LAGM] = nrm;
+            s_vs = j + 1 < SG_LAGM ? vs : 0.0;
+        }
+    }
+    __syncthreads();
     const double vs = s_vs;
-    if (vs == 0.0) return;
-    for (int k = threadIdx.x; k <= j; k += blockDim.x) {
-        c_s[k] = h2_s[k] * vs;
-        st->lagc[k] = c_s[k];
-    }
-    if (threadIdx.x == 0) st->lagT[(j + 1) + (j + 1) * SG_LAGM] = vs;
-    __syncthreads();
-    // T(:, j+1) = T(j+1,j+1) e_{j+1} - T(:, 0..j) c
-    for (int l = threadIdx.x; l <= j; l += blockDim.x) {
-        double s = 0.0;
-        for (int k = l; k <= j; ++k) s += Ts[l][k] * c_s[k];
-        st->lagT[l + (j + 1) * SG_LAGM] = -s;
+    if (vs == 0.0 || warp != 1) return;
+    // T(:, j+1) = T(j+1,j+1) e_{j+1} - T(:, 0..j) c with c = h2 vs
+    if (lane <= j) {
+        st->lagc[lane] = h2_s[lane] * vs;
+        st->lagT[lane + (j + 1) * SG_LAGM] = -tc * vs;
+    } else if (lane == j + 1) {
+        st->lagT[lane + (j + 1) * SG_LAGM] = vs;
     }
 }
 
-template <class TV>
-__global__ void __launch_bounds__(KT)
+template <class TV, int NWG>
+__global__ void __launch_bounds__(KT, DOTS_PER_SM)
 k_dots(const TV* __restrict__ raw, size_t ldv, int n, int k0, int kc, const TV* __restrict__ w,
        SolveState* st, int second, int lagged, double* partials, unsigned* counter) {
     if (!st->cycle_active) return;
     constexpr int VN = Vec<TV>::N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwg = warps_per_tile(kc), ngrp = KW / nwg;
+    constexpr int nwg = NWG, ngrp = KW / NWG;
     const int grp = warp / nwg, slot = warp % nwg;
+    __shared__ LagIn lag_in;
+    if (lagged && cluster_rank() == 0) lag_prefetch(lag_in, st, kc - 1, false);
     TV acc[KPW];
 #pragma unroll
     for (int q = 0; q < KPW; ++q) acc[q] = (TV)0;
@@ -396,8 +473,8 @@ k_dots(const TV* __restrict__ raw, size_t ldv, int n, int k0, int kc, const TV* 
         for (int q = 0; q < KPW; ++q) {
             const int k = slot + nwg * q;
             if (k < kc) {
-                acc[q] += dotv<TV>(v0[q], w0);
-                acc[q] += dotv<TV>(v1[q], w1);
+                acc[q] = dotv<TV>(v0[q], w0, acc[q]);
+                acc[q] = dotv<TV>(v1[q], w1, acc[q]);
             }
         }
     }
@@ -410,7 +487,7 @@ k_dots(const TV* __restrict__ raw, size_t ldv, int n, int k0, int kc, const TV* 
             if (k < kc) {
                 TV vv[VN];
                 vload<TV>(raw + (size_t)(k0 + k) * ldv + (size_t)u * VN, vv);
-                acc[q] += dotv<TV>(vv, wv);
+                acc[q] = dotv<TV>(vv, wv, acc[q]);
             }
         }
     }
@@ -425,20 +502,17 @@ k_dots(const TV* __restrict__ raw, size_t ldv, int n, int k0, int kc, const TV* 
         }
     }
     __shared__ double bs[KW * KPW], tot[KW * KPW];
-    __shared__ LagAIn lag_in;
     group_sums<TV>(acc, kc, nwg, bs);
-    if (last_block_reduce(partials, counter, bs, kc, tot, [&] {
-            if (lagged) lagged_a_load(lag_in, st, kc - 1);
-        })) {
-        if (lagged) {
-            lagged_pass_a(st, kc - 1, tot, lag_in);
-            return;
-        }
-        for (int k = threadIdx.x; k < kc; k += blockDim.x) {
-            const double h = st->vscale[k0 + k] * tot[k];
-            st->h[k0 + k] = h;
-            st->hsum[k0 + k] = second ? st->hsum[k0 + k] + h : h;
-        }
+    if (lagged) cp_async_wait();
+    if (!cluster_reduce(partials, counter, bs, kc, tot)) return;
+    if (lagged) {
+        lagged_pass_a(st, kc - 1, tot, lag_in);
+        return;
+    }
+    for (int k = threadIdx.x; k < kc; k += blockDim.x) {
+        const double h = st->vscale[k0 + k] * tot[k];
+        st->h[k0 + k] = h;
+        st->hsum[k0 + k] = second ? st->hsum[k0 + k] + h : h;
     }
 }
 
@@ -446,11 +520,11 @@ k_dots(const TV* __restrict__ raw, size_t ldv, int n, int k0, int kc, const TV* 
 // Each warp of a tile group forms the update of its own vectors for the
 // tile.  A one-warp group holds every vector: w' = w - share directly.  In a
 // larger group the shares meet in shared memory, the group's threads each
-// form w' = w - (sum of the shares, in warp order) for some elements of the
+// form w' = w - (sum of the shares) for some elements of the
 // tile (and store them), and every warp dots w' with the vector values it
 // still holds.
-template <class TV>
-__global__ void __launch_bounds__(KT)
+template <class TV, int NWG>
+__global__ void __launch_bounds__(KT, UPD_PER_SM)
 k_upd_dots(const TV* __restrict__ raw, size_t ldv, int n, int nk, TV* __restrict__ w,
            SolveState* st, double* partials, unsigned* counter, int lagged, int m,
            double* hist, int hist_cap) {
@@ -458,15 +532,14 @@ k_upd_dots(const TV* __restrict__ raw, size_t ldv, int n, int nk, TV* __restrict
     constexpr int VN = Vec<TV>::N;
     constexpr int TE = 32 * VN;  // elements of a tile
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwg = warps_per_tile(nk), ngrp = KW / nwg;
+    constexpr int nwg = NWG, ngrp = KW / NWG;
     const int grp = warp / nwg, slot = warp % nwg;
-    const int gsz = nwg * 32, gt = slot * 32 + lane;  // threads of the group, rank
+    constexpr int gsz = nwg * 32;  // threads of the group
+    const int gt = slot * 32 + lane;
     __shared__ TV cf[KW * KPW];
     __shared__ TV upd[KW][TE];
     __shared__ TV wsh[KW / 2][TE];
-    for (int k = threadIdx.x; k < nk; k += blockDim.x)
-        cf[k] = lagged ? (TV)st->cfu[k] : (TV)(st->h[k] * st->vscale[k]);
-    __syncthreads();
+    __shared__ LagIn lag_in;
     TV ss = (TV)0;  // ||w'||^2 (lagged): slot 0 of each group counts its elements
     TV acc[KPW];
 #pragma unroll
@@ -511,7 +584,12 @@ k_upd_dots(const TV* __restrict__ raw, size_t ldv, int n, int nk, TV* __restrict
     };
     const int gstride = gridDim.x * ngrp;
     int tile = blockIdx.x * ngrp + grp;
+    // the first tile's loads, the coefficients' and the end's all in flight at once
     if (tile < ntiles) load_tile(tile, vv, we);
+    if (lagged && cluster_rank() == 0) lag_prefetch(lag_in, st, nk - 1, true);
+    for (int k = threadIdx.x; k < nk; k += blockDim.x)
+        cf[k] = lagged ? (TV)st->cfu[k] : (TV)(st->h[k] * st->vscale[k]);
+    __syncthreads();
     for (; tile < ntiles; tile += gstride) {
         const int next = tile + gstride;
         if (next < ntiles) load_tile(next, nv, nwe);
@@ -540,14 +618,19 @@ k_upd_dots(const TV* __restrict__ raw, size_t ldv, int n, int nk, TV* __restrict
 #pragma unroll
             for (int e = 0; e < VN; ++e) upd[warp][lane * VN + e] = part[e];
             group_sync(grp, nwg);
-            // w' = w - (sum of the shares, in warp order), once per element
+            // w' = w - (sum of the shares), once per element
 #pragma unroll
             for (int r = 0; r < VN; ++r) {
                 const int t = gt + r * gsz;
                 if (t < TE) {
-                    TV sum = (TV)0;
-                    for (int g = 0; g < nwg; ++g) sum += upd[grp * nwg + g][t];
-                    const TV x = we[r] - sum;
+                    TV sh[nwg];  // added pairwise: three deep for eight warps
+#pragma unroll
+                    for (int g = 0; g < nwg; ++g) sh[g] = upd[grp * nwg + g][t];
+#pragma unroll
+                    for (int o = 1; o < nwg; o *= 2)
+#pragma unroll
+                        for (int g = 0; g < nwg; g += 2 * o) sh[g] += sh[g + o];
+                    const TV x = we[r] - sh[0];
                     wsh[grp][t] = x;
                     const int i = ptile * TE + t;
                     if (i < nfull) w[i] = x;
@@ -563,10 +646,7 @@ k_upd_dots(const TV* __restrict__ raw, size_t ldv, int n, int nk, TV* __restrict
         }
 #pragma unroll
         for (int q = 0; q < KPW; ++q) {
-            TV d = (TV)0;
-#pragma unroll
-            for (int e = 0; e < VN; ++e) d += vv[q][e] * wn[e];
-            acc[q] += d;
+            acc[q] = dotv<TV>(vv[q], wn, acc[q]);
         }
 #pragma unroll
         for (int q = 0; q < KPW; ++q)
@@ -595,27 +675,28 @@ k_upd_dots(const TV* __restrict__ raw, size_t ldv, int n, int nk, TV* __restrict
             }
         }
     }
-    __shared__ double bs[KW * KPW + 1], tot[KW * KPW + 1];
+    __shared__ double bs[KW * KPW], tot[KW * KPW];
     group_sums<TV>(acc, nk, nwg, bs);
     if (lagged) {
-        // block sum of ||w'||^2 next to the dots
+        // block sum of ||w'||^2 next to the dots (nk < SG_LAGM)
         __shared__ double red_ss[KW];
-        const double v = (double)warp_sum(ss);
-        if (lane == 0) red_ss[warp] = v;
+        if (slot == 0 || warp == 0) {
+            const double v = (double)warp_sum(ss);
+            if (lane == 0) red_ss[warp] = v;
+        }
         __syncthreads();
         if (threadIdx.x == 0) {
             double t = red_ss[0];
-            for (int g = 1; g < KW; ++g) t += red_ss[g];
+            for (int g = 1; g < ngrp; ++g) t += red_ss[g * nwg];
             bs[nk] = t;
         }
+        cp_async_wait();
         __syncthreads();
-        __shared__ LagBIn lag_in;
-        if (last_block_reduce(partials, counter, bs, nk + 1, tot,
-                              [&] { lagged_b_load(lag_in, st, nk - 1); }))
+        if (cluster_reduce(partials, counter, bs, nk + 1, tot))
             lagged_pass_b(st, nk - 1, m, tot, tot[nk], hist, hist_cap, lag_in);
         return;
     }
-    if (last_block_reduce(partials, counter, bs, nk, tot)) {
+    if (cluster_reduce(partials, counter, bs, nk, tot)) {
         for (int k = threadIdx.x; k < nk; k += blockDim.x) {
             const double h = st->vscale[k] * tot[k];
             st->h[k] = h;
@@ -689,7 +770,7 @@ k_upd_norm(const TV* __restrict__ raw, size_t ldv, int n, int j, int m, TV* __re
     __shared__ double bs[1], tot[1];
     TV v1[1] = {ss};
     block_sum_multi<1>(v1, 1, red, bs);
-    if (last_block_reduce(partials, counter, bs, 1, tot))
+    if (cluster_reduce(partials, counter, bs, 1, tot))
         arnoldi_finalize(st, j, m, tot[0], hist, hist_cap);
 }
 
@@ -716,7 +797,7 @@ k_cycle_init(const TV* __restrict__ raw0, int n, SolveState* st, int m, int flex
     __shared__ double bs[1], tot[1];
     TV v1[1] = {ss};
     block_sum_multi<1>(v1, 1, red, bs);
-    if (!last_block_reduce(partials, counter, bs, 1, tot)) return;
+    if (!cluster_reduce(partials, counter, bs, 1, tot)) return;
     const int ld = m + 1;
     for (int i = threadIdx.x; i < ld * m; i += blockDim.x) st->H[i] = 0.0;
     for (int i = threadIdx.x; i <= m; i += blockDim.x) st->g[i] = 0.0;
@@ -898,14 +979,77 @@ int kgrid(sg_ctx* ctx, int n, int per_sm) {
     return need < 1 ? 1 : (int)need;
 }
 
+// Launches a reducing kernel over `need` blocks of work in clusters.  Up to 32
+// blocks' worth runs as one cluster of up to eight blocks (its reduction stays
+// in shared memory; up to four rounds of tiles cost less than the global
+// round trip); a larger grid has clusters of four (two passes at 128^3 FP32
+// take 70.8, 66.3, 63.6 and 64.3 us with clusters of 1, 2, 4 and 8), at most
+// as many as are resident at once (the GPU's processor groups do not divide
+// evenly, and a second wave of a few clusters would double the time: 84 us).
+template <class... P, class... A>
+void launch_clusters(sg_ctx* ctx, long long need, void (*kern)(P...), A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(KT);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CL_SIZE;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (need <= 4 * CL_MAX) {
+        unsigned c = 1;
+        while (c < need && c < CL_MAX) c *= 2;
+        at[0].val.clusterDim.x = c;
+        cfg.gridDim = dim3(c);
+    } else {
+        int& cap = ctx->max_clusters[reinterpret_cast<const void*>(kern)];
+        cfg.gridDim = dim3(CL_SIZE);
+        if (cap == 0) {
+            SG_CUDA(cudaOccupancyMaxActiveClusters(&cap, kern, &cfg));
+            if (cap < 1) fail(SG_ERR_INTERNAL, "a reduction's clusters do not fit this GPU");
+        }
+        const long long ncl = (need + CL_SIZE - 1) / CL_SIZE;
+        cfg.gridDim = dim3((unsigned)(CL_SIZE * std::min<long long>(ncl, cap)));
+    }
+    SG_CUDA(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+    count_launch(ctx);
+}
+
+// blocks that give every tile group of a pass over nk vectors one tile
+template <class TV>
+long long tile_blocks(int n, int nk) {
+    const long long tiles = ((long long)n / Vec<TV>::N + 31) / 32;
+    return (tiles * warps_per_tile(nk) + KW - 1) / KW;
+}
+
 }  // namespace
 
 template <class TV>
 void launch_cycle_init(sg_ctx* ctx, const TV* raw0, int n, SolveState* st, int m, bool flexible) {
-    k_cycle_init<TV><<<kgrid(ctx, (n + 3) / 4, 4), KT, 0, ctx->stream>>>(
-        raw0, n, st, m, flexible ? 1 : 0, ctx->partials.p, ctx->counter.p);
-    SG_CUDA(cudaGetLastError());
-    count_launch(ctx);
+    launch_clusters(ctx, n / (4 * KT) + 1, k_cycle_init<TV>, raw0, n, st, m,
+                    flexible ? 1 : 0, ctx->partials.p, ctx->counter.p);
+}
+
+// the kernel for nk vectors
+template <class TV>
+static auto dots_kernel(int nk) {
+    switch (warps_per_tile(nk)) {
+    case 1: return k_dots<TV, 1>;
+    case 2: return k_dots<TV, 2>;
+    case 4: return k_dots<TV, 4>;
+    default: return k_dots<TV, 8>;
+    }
+}
+template <class TV>
+static auto upd_dots_kernel(int nk) {
+    switch (warps_per_tile(nk)) {
+    case 1: return k_upd_dots<TV, 1>;
+    case 2: return k_upd_dots<TV, 2>;
+    case 4: return k_upd_dots<TV, 4>;
+    default: return k_upd_dots<TV, 8>;
+    }
 }
 
 template <class TV>
@@ -913,10 +1057,8 @@ static void dots_any(sg_ctx* ctx, const TV* raw, size_t ldv, int n, int nk, cons
                      SolveState* st, int second, int lagged = 0) {
     for (int k0 = 0; k0 < nk; k0 += KW * KPW) {
         const int kc = nk - k0 < KW * KPW ? nk - k0 : KW * KPW;
-        k_dots<TV><<<kgrid(ctx, (n + 3) / 4 * 8, 4), KT, 0, ctx->stream>>>(
-            raw, ldv, n, k0, kc, w, st, second, lagged, ctx->partials.p, ctx->counter.p);
-        SG_CUDA(cudaGetLastError());
-        count_launch(ctx);
+        launch_clusters(ctx, tile_blocks<TV>(n, kc), dots_kernel<TV>(kc), raw, ldv, n,
+                        k0, kc, w, st, second, lagged, ctx->partials.p, ctx->counter.p);
     }
 }
 
@@ -929,21 +1071,17 @@ void launch_cgs2(sg_ctx* ctx, TV* raw, size_t ldv, int n, int j, int m, SolveSta
         // two passes (see lagged_pass_a / lagged_pass_b); m < SG_LAGM <= 32
         if (m >= SG_LAGM || nk > KW * KPW) fail(SG_ERR_INTERNAL, "lagged CGS2 needs m < %d", SG_LAGM);
         dots_any<TV>(ctx, raw, ldv, n, nk, w, st, 0, 1);
-        k_upd_dots<TV><<<kgrid(ctx, (n + 3) / 4 * 8, 3), KT, 0, ctx->stream>>>(
-            raw, ldv, n, nk, w, st, ctx->partials.p, ctx->counter.p, 1, m, ctx->hist_d,
-            ctx->hist_cap);
-        SG_CUDA(cudaGetLastError());
-        count_launch(ctx);
+        launch_clusters(ctx, tile_blocks<TV>(n, nk), upd_dots_kernel<TV>(nk), raw, ldv,
+                        n, nk, w, st, ctx->partials.p, ctx->counter.p, 1, m, ctx->hist_d,
+                        ctx->hist_cap);
         return;
     }
     // pass A
     dots_any<TV>(ctx, raw, ldv, n, nk, w, st, 0);
     // pass B
     if (nk <= KW * KPW) {
-        k_upd_dots<TV><<<kgrid(ctx, (n + 3) / 4 * 8, 3), KT, 0, ctx->stream>>>(
-            raw, ldv, n, nk, w, st, ctx->partials.p, ctx->counter.p, 0, m, nullptr, 0);
-        SG_CUDA(cudaGetLastError());
-        count_launch(ctx);
+        launch_clusters(ctx, tile_blocks<TV>(n, nk), upd_dots_kernel<TV>(nk), raw, ldv,
+                        n, nk, w, st, ctx->partials.p, ctx->counter.p, 0, m, (double*)nullptr, 0);
     } else {
         k_upd<TV><<<kgrid(ctx, n, 4), KT, 0, ctx->stream>>>(raw, ldv, n, nk, w, st);
         SG_CUDA(cudaGetLastError());
@@ -951,10 +1089,8 @@ void launch_cgs2(sg_ctx* ctx, TV* raw, size_t ldv, int n, int j, int m, SolveSta
         dots_any<TV>(ctx, raw, ldv, n, nk, w, st, 1);
     }
     // pass C
-    k_upd_norm<TV><<<kgrid(ctx, n / Vec<TV>::N + 1, 4), KT, 0, ctx->stream>>>(
-        raw, ldv, n, j, m, w, st, ctx->partials.p, ctx->counter.p, ctx->hist_d, ctx->hist_cap);
-    SG_CUDA(cudaGetLastError());
-    count_launch(ctx);
+    launch_clusters(ctx, n / (Vec<TV>::N * KT) + 1, k_upd_norm<TV>, raw, ldv,
+                    n, j, m, w, st, ctx->partials.p, ctx->counter.p, ctx->hist_d, ctx->hist_cap);
 }
 
 void launch_backsolve(sg_ctx* ctx, SolveState* st, int m) {

@@ -6,6 +6,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -193,6 +194,8 @@ struct sg_ctx {
     // reduction scratch shared by the kernels of this context (one stream)
     sg::DBuf<double> partials;
     sg::DBuf<unsigned int> counter;
+    // clusters of a reducing kernel that this device holds at once, by kernel
+    std::map<const void*, int> max_clusters;
     // residual history of the running solve (device)
     sg::DBuf<double> hist;
     double* hist_d = nullptr;

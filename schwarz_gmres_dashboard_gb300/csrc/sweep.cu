@@ -342,6 +342,28 @@ struct RowRec {
     }
 };
 
+// a / d rounded to nearest from y = 1 / d rounded to nearest: two corrected
+// quotients (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990).  a y is within two units in the last
+// place, the first correction makes it faithful, and the last residual, exact
+// in one fused multiply-add, rounds the quotient correctly -- five dependent
+// operations where the division takes the time of seven and twice the FP64
+// slots.  Outside the exponents where no residual can lose bits (and for
+// infinities and NaN) the division itself; a zero keeps the sign of a y.
+__device__ __noinline__ double div_plain(double a, double d) { return a / d; }
+__device__ __forceinline__ double div_recip(double a, double d, double y) {
+    const int ha = __double2hiint(a);
+    const int ea = (ha >> 20) & 0x7ff, ed = (__double2hiint(d) >> 20) & 0x7ff;
+    const bool zero = ((ha << 1) | __double2loint(a)) == 0;  // also the lanes past a level's end
+    const double q0 = a * y;
+    double q = fma(fma(-q0, d, a), y, q0);
+    q = fma(fma(-q, d, a), y, q);
+    if (zero) q = q0;
+    const bool safe = (unsigned)(ea - 423) <= 1200u && (unsigned)(ed - 723) <= 600u;
+    if (!safe && !zero) q = div_plain(a, d);  // a call: inlined, it would run for every row
+    return q;
+}
+
 // R vector elements of one slot
 template <class TS, int R>
 __device__ __forceinline__ void slot_ld(uint32_t a, TS (&v)[R]) {
@@ -626,7 +648,8 @@ __device__ __forceinline__ void level_loop_any(const int2* ent, int j0, int j1, 
 // code (a divergent branch or an inner loop costs 40 to 80 cycles a level):
 //  * a thread loads the struct of its next row before the barrier, between
 //    the loads of this level's vector elements and their first use;
-//  * the diagonal comes as its reciprocal (exact FP64 sweeps divide);
+//  * the diagonal comes as its reciprocal (exact FP64 sweeps round the
+//    quotient correctly with it, div_recip);
 //  * the lanes past a level's end take the row that computes 0 in the unused
 //    slot, so no store is conditional within a warp;
 //  * a level of more than NC rows is several entries of the schedule.
@@ -634,9 +657,12 @@ __device__ __forceinline__ void level_loop_any(const int2* ent, int j0, int j1, 
 // the barrier -> this loop: 51 x 51 FP32 223 -> 104, 15^3 FP32 288 -> 165;
 // 51 x 51 FP64 354 forward, 995 backward -> 214, 270; 14^3 FP64 481, 1159 ->
 // 414, 519.  Warps without rows still take the predicated FP64 instructions'
-// slots of the narrow FP64 pipe, which is why FP64 sweeps run their levels on
-// few warps (270 cycles with 2 warps, 507 with 8).
-template <int W, bool BACK, class TS, class TF, bool EXACT, int R>
+// slots of the narrow FP64 pipe, so FP64 sweeps either run their levels on few
+// warps (270 cycles with 2 warps, 507 with 8) or, with FP64_SKIP threads or
+// more, branch around the level in warps that have no rows (SKIP: 350 cycles
+// with 8 warps, and a level of many rows takes fewer passes).
+constexpr int FP64_SKIP = 256;
+template <int W, bool BACK, class TS, class TF, bool EXACT, int R, bool SKIP>
 __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecRing& ring,
                                            uint32_t t_s, int NC) {
     using Row = RowRec<W, BACK, TF>;
@@ -654,10 +680,18 @@ __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecR
         Row row;
         if (on) row.load(a);
         for (; e < e1; ++e) {
+            if (SKIP && !on && !(wid < (mn.x & 0xffff))) {  // nothing here, nothing to load
+                const int f = sync;
+                md = mn;
+                sync = md.x >> 16;
+                mn = ent[e + 2];
+                if (f) level_sync(NC);
+                continue;
+            }
             const bool cur = on;
             const int f = sync;
             uint32_t ar = 0;
-            TS xk[W][R], acc[R], vk[W], rd = (TS)1;
+            TS xk[W][R], acc[R], vk[W], rd = (TS)1, dg = (TS)1;
             if (cur) {
                 ar = t_s + ST * row.slot(0);
 #pragma unroll
@@ -665,7 +699,8 @@ __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecR
                 slot_ld<TS, R>(ar, acc);
 #pragma unroll
                 for (int k = 0; k < W; ++k) vk[k] = row.template value<TS>(k);
-                if (BACK) rd = row.template recip<TS>(EXACT ? 1 : 0);
+                if (BACK) rd = row.template recip<TS>(0);
+                if (BACK && EXACT) dg = row.template recip<TS>(1);
             }
             md = mn;
             c = md.x & 0xffff;
@@ -682,8 +717,10 @@ __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecR
                         acc[i] = sub_mul<TS, EXACT>(acc[i], vk[k], xk[k][i]);
                 if (BACK) {
 #pragma unroll
-                    for (int i = 0; i < R; ++i)
-                        acc[i] = (EXACT && sizeof(TS) == 8) ? acc[i] / rd : acc[i] * rd;
+                    for (int i = 0; i < R; ++i) {
+                        if constexpr (EXACT && sizeof(TS) == 8) acc[i] = div_recip(acc[i], dg, rd);
+                        else acc[i] = acc[i] * rd;
+                    }
                 }
                 slot_st<TS, R>(ar, acc);
             }
@@ -697,10 +734,18 @@ template <bool BACK, class TS, class TF, bool EXACT, int R>
 __device__ __forceinline__ void level_loop_w(const int2* ent, int j0, int j1, int w, bool rows,
                                              RecRing& ring, TS* t, uint32_t t_s,
                                              unsigned char* ring_g, int NC) {
+    if constexpr (sizeof(TS) == 8) {
+        if (rows && rec_is_rows(w) && NC >= FP64_SKIP) {
+            if (w == 2) level_loop<2, BACK, TS, TF, EXACT, R, true>(ent, j0, j1, ring, t_s, NC);
+            else if (w == 3) level_loop<3, BACK, TS, TF, EXACT, R, true>(ent, j0, j1, ring, t_s, NC);
+            else level_loop<4, BACK, TS, TF, EXACT, R, true>(ent, j0, j1, ring, t_s, NC);
+            return;
+        }
+    }
     switch (rows ? w : 0) {
-    case 2: return level_loop<2, BACK, TS, TF, EXACT, R>(ent, j0, j1, ring, t_s, NC);
-    case 3: return level_loop<3, BACK, TS, TF, EXACT, R>(ent, j0, j1, ring, t_s, NC);
-    case 4: return level_loop<4, BACK, TS, TF, EXACT, R>(ent, j0, j1, ring, t_s, NC);
+    case 2: return level_loop<2, BACK, TS, TF, EXACT, R, false>(ent, j0, j1, ring, t_s, NC);
+    case 3: return level_loop<3, BACK, TS, TF, EXACT, R, false>(ent, j0, j1, ring, t_s, NC);
+    case 4: return level_loop<4, BACK, TS, TF, EXACT, R, false>(ent, j0, j1, ring, t_s, NC);
     default:
         return level_loop_any<BACK, TS, TF, EXACT, R>(ent, j0, j1, w, ring, t, t_s, ring_g, NC);
     }

@@ -137,7 +137,7 @@ struct SolveState {
     double hsum[SG_MMAX + 1];           // h1 + h2 of the current column
     double vscale[SG_MMAX + 1];         // basis vector k is stored as raw_k; v_k = vscale[k]*raw_k
     double y[SG_MMAX];
-    // lagged CGS2 (left-preconditioned GMRES, restart < SG_LAGM): the
+    // lagged CGS2 (restart < SG_LAGM): the
     // stored basis vectors raw_l relate to the orthonormal ones through an
     // upper triangular T, v_i = sum_{l<=i} T(l,i) raw_l; the newest stored
     // vector still lacks its second projection, held in lagc

@@ -98,11 +98,14 @@ void apply_pc(sg_ctx* ctx, sg_precond* pc, const TI* x, TO* y, int n, const int*
     }
 }
 
-// The lagged two-pass CGS2 serves the left-preconditioned cycle (FP32 or
-// FP64 basis) with a restart below SG_LAGM unless the caller asks for the
-// classic three passes: it relies on the operator being linear (B v_k =
-// V H(:,k)), which FGMRES's possibly nonlinear preconditioner does not give.
-bool use_lagged(bool flexible, int m, int ortho) { return ortho == 0 && !flexible && m < SG_LAGM; }
+// The lagged two-pass CGS2 serves every cycle with a restart below SG_LAGM
+// unless the caller asks for the classic three passes.  Left-preconditioned
+// GMRES relies on the operator being linear (B v_k = V H(:,k)).  FGMRES does
+// not need a linear preconditioner: with the stored directions z_l = M raw_l
+// it is FGMRES with the directions Z T (the update takes them, x += Z T y),
+// for which A (Z T) = V H holds whatever M is; they differ from M v_j by the
+// second projection, a rounding-level change of M's argument.
+bool use_lagged(int m, int ortho) { return ortho == 0 && m < SG_LAGM; }
 
 // One restart cycle as a launch sequence on ctx->stream.
 template <class TV>
@@ -186,7 +189,7 @@ void solve_device(sg_ctx* ctx, int solver, const sg_csr* A, sg_precond* pc, cons
     SG_CHECK_ARG(prm.ortho == 0 || prm.ortho == 1, "ortho must be 0 or 1 (got %d)", prm.ortho);
     const bool flexible = solver == SG_FGMRES;
     const bool fp32 = prm.precision == SG_FP32;
-    const bool lagged = use_lagged(flexible, m, prm.ortho);
+    const bool lagged = use_lagged(m, prm.ortho);
     if (!ctx->work) ctx->work = new SolveWork();
     SolveWork* w = ctx->work;
     // basis stride: a multiple of 32 elements plus 32, so consecutive basis

@@ -415,6 +415,8 @@ struct sg_precond {
     // ---- coarse space
     int nc = 0;
     sg::DBuf<double> a0, a0inv, lu0, r0, cscale_d;
+    sg::DBuf<double> a0_own;  // scratch of its build: the owned rows' terms,
+    sg::DBuf<int> a0_rows;    // and the rows that touch other parts
     sg::DBuf<int> piv0, status_d;
     // ---- host-API staging
     sg::DBuf<double> io_x, io_y;

@@ -95,89 +95,6 @@ static void use_device(const sg_ctx* ctx) { SG_CUDA(cudaSetDevice(ctx->device));
 
 using namespace sg;
 
-void sg_csr::ensure_fp32() {
-    if (val32.p) return;
-    std::vector<float> v32(h_val.size() + 16, 0.0f);
-    for (size_t i = 0; i < h_val.size(); ++i) v32[i] = (float)h_val[i];
-    val32.upload(v32, ctx->stream);
-    if (sell_ok) {
-        // FP32 copy of the SELL values (same slice layout)
-        std::vector<double> sv(sell_entries);
-        SG_CUDA(cudaMemcpyAsync(sv.data(), sl_val.p, sizeof(double) * sell_entries,
-                                cudaMemcpyDeviceToHost, ctx->stream));
-        SG_CUDA(cudaStreamSynchronize(ctx->stream));
-        std::vector<float> s32(sell_entries);
-        for (long long i = 0; i < sell_entries; ++i) s32[i] = (float)sv[i];
-        sl_val32.upload(s32, ctx->stream);
-    }
-    SG_CUDA(cudaStreamSynchronize(ctx->stream));
-}
-
-// SELL-32 copy (slices of 32 rows, slice-major, padded per slice).  Kept only
-// when the padding stays under 25% of the nonzeros.
-void sg_csr::build_sell() {
-    sell_ok = false;
-    if (nrows <= 0 || nrows != ncols) return;
-    nslices = (nrows + 31) / 32;
-    std::vector<long long> ptr(nslices + 1, 0);
-    std::vector<int> w(nslices, 0);
-    for (int s = 0; s < nslices; ++s) {
-        int mw = 0;
-        for (int r = s * 32; r < std::min(nrows, s * 32 + 32); ++r)
-            mw = std::max(mw, h_rp[r + 1] - h_rp[r]);
-        w[s] = mw;
-        ptr[s + 1] = ptr[s] + 32ll * mw;
-    }
-    sell_entries = ptr[nslices];
-    sell_maxw = 0;
-    for (int s = 0; s < nslices; ++s) sell_maxw = std::max(sell_maxw, w[s]);
-    if (sell_entries > (long long)nnz + nnz / 4 + 64 || sell_entries >= (1ll << 31)) return;
-    std::vector<int> col(sell_entries > 0 ? sell_entries : 1, 0);
-    std::vector<double> val(sell_entries > 0 ? sell_entries : 1, 0.0);
-    for (int s = 0; s < nslices; ++s)
-        for (int lane = 0; lane < 32; ++lane) {
-            const int r = s * 32 + lane;
-            int k = 0;
-            if (r < nrows)
-                for (int e = h_rp[r]; e < h_rp[r + 1]; ++e, ++k) {
-                    col[ptr[s] + 32ll * k + lane] = h_ci[e];
-                    val[ptr[s] + 32ll * k + lane] = h_val[e];
-                }
-            for (; k < w[s]; ++k) {
-                col[ptr[s] + 32ll * k + lane] = r < nrows ? r : 0;
-                val[ptr[s] + 32ll * k + lane] = 0.0;
-            }
-        }
-    sl_ptr.upload(ptr, ctx->stream);
-    sl_w.upload(w, ctx->stream);
-    sl_col.upload(col, ctx->stream);
-    sl_val.upload(val, ctx->stream);
-    // 16-bit column offsets when every |column - row| fits (banded matrices)
-    sl_dcol.release();
-    {
-        bool fits = true;
-        std::vector<int16_t> dcol(col.size());
-        for (int s = 0; s < nslices && fits; ++s)
-            for (long long e = ptr[s]; e < ptr[s + 1]; ++e) {
-                const int r = s * 32 + (int)((e - ptr[s]) % 32);
-                const long long d = (long long)col[e] - (r < nrows ? r : 0);
-                if (r >= nrows) {
-                    // lanes past the last row: result never stored; point the
-                    // load at row n-1 (offset >= -31)
-                    dcol[e] = (int16_t)((nrows - 1) - r);
-                    continue;
-                }
-                if (d < -32768 || d > 32767) {
-                    fits = false;
-                    break;
-                }
-                dcol[e] = (int16_t)d;
-            }
-        if (fits) sl_dcol.upload(dcol, ctx->stream);
-    }
-    sell_ok = true;
-}
-
 extern "C" {
 
 int sg_abi_version(void) { return SG_ABI_VERSION; }
@@ -330,43 +247,49 @@ sg_status sg_csr_create(sg_ctx* ctx, int nrows, int ncols, int nnz, const int* r
             A->ncols = ncols;
             A->nnz = nnz;
             A->h_rp.resize((size_t)nrows + 1);
-            A->h_ci.resize((size_t)nnz + 16, 0);
-            A->h_val.resize((size_t)nnz);
+            A->h_ci.resize((size_t)nnz);
+            const cudaMemcpyKind kind =
+                mem == SG_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
             if (mem == SG_MEM_DEVICE) {
                 SG_CUDA(cudaMemcpy(A->h_rp.data(), row_ptr, sizeof(int) * (nrows + 1),
                                    cudaMemcpyDeviceToHost));
-                if (nnz) {
+                if (nnz)
                     SG_CUDA(cudaMemcpy(A->h_ci.data(), col_idx, sizeof(int) * nnz,
                                        cudaMemcpyDeviceToHost));
-                    SG_CUDA(cudaMemcpy(A->h_val.data(), vals, sizeof(double) * nnz,
-                                       cudaMemcpyDeviceToHost));
-                }
             } else {
                 std::memcpy(A->h_rp.data(), row_ptr, sizeof(int) * (nrows + 1));
-                if (nnz) {
-                    std::memcpy(A->h_ci.data(), col_idx, sizeof(int) * nnz);
-                    std::memcpy(A->h_val.data(), vals, sizeof(double) * nnz);
-                }
+                if (nnz) std::memcpy(A->h_ci.data(), col_idx, sizeof(int) * nnz);
             }
             SG_CHECK_ARG(A->h_rp[0] == 0, "row_ptr[0] must be 0");
             SG_CHECK_ARG(A->h_rp[nrows] == nnz, "row_ptr[nrows] (%d) != nnz (%d)", A->h_rp[nrows],
                          nnz);
-            for (int i = 0; i < nrows; ++i) {
-                SG_CHECK_ARG(A->h_rp[i + 1] >= A->h_rp[i], "row_ptr decreases at row %d", i);
-                for (int e = A->h_rp[i]; e < A->h_rp[i + 1]; ++e) {
-                    const int c = A->h_ci[e];
-                    SG_CHECK_ARG(c >= 0 && c < ncols, "col_idx[%d] = %d outside [0,%d)", e, c, ncols);
-                    if (e > A->h_rp[i] && c < A->h_ci[e - 1]) A->sorted = false;
+            bool ok = true;
+            for (int i = 0; i < nrows; ++i) ok = ok && A->h_rp[i + 1] >= A->h_rp[i];
+            if (ok) {
+                // the arrays padded with 16 zero entries, so that 16-byte
+                // vector loads never leave them
+                cudaStream_t st = ctx->stream;
+                A->rp.upload(A->h_rp, st);
+                A->ci.alloc((size_t)nnz + 16);
+                A->val.alloc((size_t)nnz + 16);
+                if (nnz) {
+                    SG_CUDA(cudaMemcpyAsync(A->ci.p, col_idx, sizeof(int) * nnz, kind, st));
+                    SG_CUDA(cudaMemcpyAsync(A->val.p, vals, sizeof(double) * nnz, kind, st));
                 }
+                SG_CUDA(cudaMemsetAsync(A->ci.p + nnz, 0, sizeof(int) * 16, st));
+                SG_CUDA(cudaMemsetAsync(A->val.p + nnz, 0, sizeof(double) * 16, st));
+                // columns checked and the SELL copy made on the device
+                ok = csr_check_and_build(A);
             }
-            std::vector<double> vpad(A->h_val);
-            vpad.resize((size_t)nnz + 16, 0.0);
-            A->rp.upload(A->h_rp, ctx->stream);
-            A->ci.upload(A->h_ci, ctx->stream);
-            A->val.upload(vpad, ctx->stream);
-            A->h_ci.resize(nnz);
-            if (A->sorted) A->build_sell();
-            SG_CUDA(cudaStreamSynchronize(ctx->stream));
+            if (!ok) {  // say where
+                for (int i = 0; i < nrows; ++i) {
+                    SG_CHECK_ARG(A->h_rp[i + 1] >= A->h_rp[i], "row_ptr decreases at row %d", i);
+                    for (int e = A->h_rp[i]; e < A->h_rp[i + 1]; ++e)
+                        SG_CHECK_ARG(A->h_ci[e] >= 0 && A->h_ci[e] < ncols,
+                                     "col_idx[%d] = %d outside [0,%d)", e, A->h_ci[e], ncols);
+                }
+                fail(SG_ERR_INTERNAL, "the column check failed on the device only");
+            }
         } catch (...) {
             delete A;
             throw;

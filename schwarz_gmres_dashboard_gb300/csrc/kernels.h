@@ -17,6 +17,10 @@ void launch_spmv(sg_ctx* ctx, int n, const int* rp, const int* ci, const TV* val
 template <class TV, class TX, class TY>
 void launch_spmv_a(sg_ctx* ctx, const sg_csr* A, const TX* x, TY* y, const double* scale,
                    const int* active);
+// Checks the column indices of the uploaded CSR arrays (false: one is out of
+// range), notes whether every row is sorted, and makes the SELL-32 copy.
+// Waits for the stream.
+bool csr_check_and_build(sg_csr* A);
 // Times both formats on A and keeps the faster one (autotuner).
 void spmv_autotune(sg_ctx* ctx, sg_csr* A);
 // r = b - A x in FP64 with ||r||; the last block updates the solve state

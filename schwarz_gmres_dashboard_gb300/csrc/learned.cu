@@ -1352,11 +1352,15 @@ sg_status sg_learned_set_matrix(sg_learned* L, const sg_csr* A) {
                      "matrix of %d rows does not match the %dx%dx%d grid", A->nrows, L->nx, L->ny,
                      L->nz);
         // coefficient feature: log A_ii restricted to the coarse cells, standardised
-        std::vector<double> ld(A->nrows, 0.0);
+        std::vector<double> ld(A->nrows, 0.0), val((size_t)A->nnz);
+        if (A->nnz)
+            SG_CUDA(cudaMemcpyAsync(val.data(), A->val.p, sizeof(double) * A->nnz,
+                                    cudaMemcpyDeviceToHost, L->ctx->stream));
+        SG_CUDA(cudaStreamSynchronize(L->ctx->stream));
         for (int i = 0; i < A->nrows; ++i) {
             double d = 0.0;
             for (int q = A->h_rp[i]; q < A->h_rp[i + 1]; ++q)
-                if (A->h_ci[q] == i) d += A->h_val[q];
+                if (A->h_ci[q] == i) d += val[q];
             if (!(d > 0.0)) fail(SG_ERR_INVALID_ARG, "row %d has a non-positive diagonal", i);
             ld[i] = std::log(d);
         }

@@ -249,7 +249,6 @@ struct sg_csr {
     int nrows = 0, ncols = 0, nnz = 0;
     bool sorted = true;  // column indices nondecreasing within each row
     std::vector<int> h_rp, h_ci;
-    std::vector<double> h_val;
     sg::DBuf<int> rp, ci;
     sg::DBuf<double> val;
     sg::DBuf<float> val32;  // FP32 copy for the FP32 inner Krylov (made on demand)
@@ -271,7 +270,6 @@ struct sg_csr {
     sg::DBuf<double> sl_val;
     sg::DBuf<float> sl_val32;
     void ensure_fp32();
-    void build_sell();
 };
 
 namespace sg {

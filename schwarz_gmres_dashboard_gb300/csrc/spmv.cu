@@ -9,6 +9,8 @@
 // lane then sums its own row from the window (a warp-segmented reduction
 // whose per-row order is the entry order).  In FP64 the products and sums are
 // rounded one by one, so y matches the reference's serial loop bit for bit.
+#include <algorithm>
+
 #include "dev_common.cuh"
 #include "kernels.h"
 
@@ -408,7 +410,122 @@ int spmv_grid(sg_ctx* ctx, int n) {
     return (int)blocks;
 }
 
+// ------------------------------------------------------- the matrix's formats
+// flags: [0] columns out of range, [1] a row whose columns decrease, [2] an
+// entry more than 16 bits away from its row
+__global__ void __launch_bounds__(256)
+k_csr_check(int nrows, int ncols, const int* __restrict__ rp, const int* __restrict__ ci,
+            int* flags) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x) {
+        int prev = 0;
+        bool bad = false, down = false;
+        for (int e = rp[r]; e < rp[r + 1]; ++e) {
+            const int c = ci[e];
+            bad |= c < 0 || c >= ncols;
+            down |= e > rp[r] && c < prev;
+            prev = c;
+        }
+        if (bad) flags[0] = 1;
+        if (down) flags[1] = 1;
+    }
+}
+
+// SELL-32 copy from CSR: a warp per slice, a lane per row (see sg_csr).  The
+// entries of 32 consecutive rows are one range of the CSR arrays, so the
+// strided reads of a step hit the lines of the steps before; the writes are
+// coalesced.
+__global__ void __launch_bounds__(256)
+k_sell_fill(int nrows, int nslices, const int* __restrict__ rp, const int* __restrict__ ci,
+            const double* __restrict__ val, const long long* __restrict__ sptr,
+            const int* __restrict__ sw, int* col, double* sval, int16_t* dcol, int* flags) {
+    const int lane = threadIdx.x & 31;
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    for (int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < nslices; s += nwarps) {
+        const int r = s * 32 + lane, w = sw[s];
+        const bool in = r < nrows;
+        const int e0 = in ? rp[r] : 0, n = in ? rp[r + 1] - e0 : 0;
+        const long long base = sptr[s] + lane;
+        bool far = false;
+        for (int k = 0; k < w; ++k) {
+            const int c = k < n ? ci[e0 + k] : (in ? r : 0);
+            // lanes past the last row: their results are never stored, their
+            // loads go to the last row
+            const int d = in ? c - r : nrows - 1 - r;
+            far |= d < -32768 || d > 32767;
+            col[base + 32ll * k] = c;
+            sval[base + 32ll * k] = k < n ? val[e0 + k] : 0.0;
+            dcol[base + 32ll * k] = (int16_t)d;
+        }
+        if (far) flags[2] = 1;
+    }
+}
+
+__global__ void k_to_float(const double* __restrict__ x, float* __restrict__ y, size_t n) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+         i += (size_t)gridDim.x * blockDim.x)
+        y[i] = (float)x[i];
+}
+
 }  // namespace
+
+// The formats were made by host loops and uploaded (64^3: 10 ms an upload of a
+// matrix, 128^3: 100 ms; the FP32 copy another 25 ms on the first mixed
+// solve); on the device they take the copies' time.  The SELL copy is kept
+// only when the padding stays under 25% of the nonzeros.
+bool csr_check_and_build(sg_csr* A) {
+    sg_ctx* ctx = A->ctx;
+    cudaStream_t st = ctx->stream;
+    DBuf<int> flags;
+    flags.alloc(4);
+    flags.zero(st);
+    const int grid = ctx->num_sms * 8;
+    k_csr_check<<<grid, 256, 0, st>>>(A->nrows, A->ncols, A->rp.p, A->ci.p, flags.p);
+    SG_CUDA(cudaGetLastError());
+    bool sell = A->nrows > 0 && A->nrows == A->ncols;
+    std::vector<long long> ptr;
+    std::vector<int> w;
+    if (sell) {
+        A->nslices = (A->nrows + 31) / 32;
+        ptr.assign((size_t)A->nslices + 1, 0);
+        w.assign((size_t)A->nslices, 0);
+        A->sell_maxw = 0;
+        for (int s = 0; s < A->nslices; ++s) {
+            int mw = 0;
+            for (int r = s * 32; r < std::min(A->nrows, s * 32 + 32); ++r)
+                mw = std::max(mw, A->h_rp[r + 1] - A->h_rp[r]);
+            w[s] = mw;
+            ptr[s + 1] = ptr[s] + 32ll * mw;
+            A->sell_maxw = std::max(A->sell_maxw, mw);
+        }
+        A->sell_entries = ptr[A->nslices];
+        sell = A->sell_entries <= (long long)A->nnz + A->nnz / 4 + 64 &&
+               A->sell_entries < (1ll << 31);
+    }
+    if (sell) {
+        A->sl_ptr.upload(ptr, st);
+        A->sl_w.upload(w, st);
+        A->sl_col.alloc((size_t)A->sell_entries);
+        A->sl_val.alloc((size_t)A->sell_entries);
+        A->sl_dcol.alloc((size_t)A->sell_entries);
+        k_sell_fill<<<grid, 256, 0, st>>>(A->nrows, A->nslices, A->rp.p, A->ci.p, A->val.p,
+                                          A->sl_ptr.p, A->sl_w.p, A->sl_col.p, A->sl_val.p,
+                                          A->sl_dcol.p, flags.p);
+        SG_CUDA(cudaGetLastError());
+    }
+    int h[4] = {0, 0, 0, 0};
+    SG_CUDA(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    SG_CUDA(cudaStreamSynchronize(st));
+    A->sorted = h[1] == 0;
+    A->sell_ok = sell && A->sorted;
+    if (!A->sell_ok) {
+        A->sl_ptr.release();
+        A->sl_w.release();
+        A->sl_col.release();
+        A->sl_val.release();
+    }
+    if (!A->sell_ok || h[2]) A->sl_dcol.release();
+    return h[0] == 0;
+}
 
 template <class TV, class TX, class TY>
 void launch_spmv(sg_ctx* ctx, int n, const int* rp, const int* ci, const TV* val, const TX* x,
@@ -586,3 +703,16 @@ template void launch_spmv_a<float, double, float>(sg_ctx*, const sg_csr*, const 
                                                   const double*, const int*);
 
 }  // namespace sg
+
+void sg_csr::ensure_fp32() {
+    if (val32.p) return;
+    const int grid = ctx->num_sms * 8;
+    val32.alloc((size_t)nnz + 16);
+    sg::k_to_float<<<grid, 256, 0, ctx->stream>>>(val.p, val32.p, (size_t)nnz + 16);
+    SG_CUDA(cudaGetLastError());
+    if (sell_ok) {  // FP32 copy of the SELL values (same slice layout)
+        sl_val32.alloc((size_t)sell_entries);
+        sg::k_to_float<<<grid, 256, 0, ctx->stream>>>(sl_val.p, sl_val32.p, (size_t)sell_entries);
+        SG_CUDA(cudaGetLastError());
+    }
+}

@@ -66,6 +66,7 @@ struct BatchDev {
     double* sn;
     double* H;       // [I][(m+1) m], column-major, ld m+1
     double* vscale;  // [I][m+1]
+    float2* vsp;     // [I][m+1] the same as a pair of floats (vs_put)
     double* y;       // [I][m]
     float* yf;       // [I][m] y_k * vscale_k in FP32 (update of an FP32 basis)
     double* yd;      // [I][m] y_k * vscale_k in FP64
@@ -97,26 +98,22 @@ __device__ __forceinline__ int chunk_of(const BatchDev& B) {
     return B.clist ? B.clist[blockIdx.x] : (int)blockIdx.x;
 }
 
-__device__ void b_rot_compute(double& c, double& s, double a, double b) {
-    // src/core/gmres.cpp:9-30
-    if (fabs(b) < 1e-30) {
-        c = 1.0;
-        s = 0.0;
-    } else if (fabs(b) > fabs(a)) {
-        const double t = -a / b;
-        s = 1.0 / sqrt(1.0 + t * t);
-        c = s * t;
-    } else {
-        const double t = -b / a;
-        c = 1.0 / sqrt(1.0 + t * t);
-        s = c * t;
-    }
+// vscale of one basis vector, and the pair of floats whose sum it is to 2^-48
+__device__ __forceinline__ void vs_put(const BatchDev& B, size_t i, double vs) {
+    B.vscale[i] = vs;
+    const float h = (float)vs;
+    B.vsp[i] = make_float2(h, (float)(vs - (double)h));
 }
-__device__ void b_rot_apply(double c, double s, double& h1, double& h2) {
-    const double t1 = c * h1 - s * h2;
-    const double t2 = s * h1 + c * h2;
-    h1 = t1;
-    h2 = t2;
+// a * vscale rounded to the basis precision.  FP32: with the pair, within
+// 2^-23 of half a unit of the FP64 product's rounding, and no instruction on
+// the FP64 pipe (two conversions and a product there cost the SM 48 cycles a
+// warp)
+__device__ __forceinline__ float vs_mul(const BatchDev& B, size_t i, float a) {
+    const float2 p = B.vsp[i];
+    return fmaf(a, p.x, a * p.y);
+}
+__device__ __forceinline__ double vs_mul(const BatchDev& B, size_t i, double a) {
+    return a * B.vscale[i];
 }
 
 // Block sums of nv per-thread values (warp shuffles, then one pass over the
@@ -251,7 +248,7 @@ k_b_cycle_init(BatchDev B, const TV* __restrict__ raw0) {
         B.active[inst] = 0;
         return;
     }
-    B.vscale[(size_t)inst * ld] = 1.0 / beta;
+    vs_put(B, (size_t)inst * ld, 1.0 / beta);
     if (B.lagged) B.lagT[(size_t)inst * BLD * BLD] = 1.0 / beta;  // v_0 = raw_0 / beta
     B.g[(size_t)inst * ld] = beta;
     B.est[inst] = B.rnorm[inst] / beta;
@@ -274,7 +271,7 @@ k_b_spmv(BatchDev B, const int* __restrict__ rp, const int* __restrict__ ci,
         const TV* xb = x + (long long)rr * B.N;
         TV acc = (TV)0;
         for (int k = rp[mr]; k < rp[mr + 1]; ++k) acc += val[k] * xb[ci[k]];
-        y[q] = (TV)((double)acc * B.vscale[(size_t)inst * ld + j]);
+        y[q] = vs_mul(B, (size_t)inst * ld + j, acc);
     }
 }
 
@@ -324,46 +321,110 @@ k_b_spmv_sell(BatchDev B, const long long* __restrict__ sl_ptr, const int* __res
             for (int u = 0; u < BSR; ++u)
                 if (act[u])
                     y[(long long)(r0 + u) * B.N + row] =
-                        (TV)((double)acc[u] * B.vscale[(size_t)((r0 + u) * B.S + sys) * ld + j]);
+                        vs_mul(B, (size_t)((r0 + u) * B.S + sys) * ld + j, acc[u]);
         }
     }
 }
 
-// red[warp][k] = warp sums of raw_k . wv (k <= j) for a chunk: four
-// vectors' loads in flight at a time; per vector the products are summed
-// over the thread's rows in row order, then across the warp
-constexpr int BKG = 4;
+// The sums over a warp of four per-thread values at once, to FP64 accuracy:
+// each of the first two exchanges halves the values a lane holds, and the sum
+// of value (lane >> 3) ends in every lane of that eighth.  FP32 values are
+// added as unevaluated pairs (the first sum of two floats is exact, D. Knuth's
+// two-sum; pairs then lose less than 2^-44 of their sum, far below the FP32
+// products they add): ten FP32 instructions an addition, where an FP64
+// addition or conversion takes the SM 16 cycles a warp -- as FP64 shuffles
+// these sums took 2.5 times the vectors' load time.
+struct F2 {
+    float h, l;
+};
+__device__ __forceinline__ F2 two_sum(float a, float b) {
+    const float s = a + b, t = s - a;
+    return {s, (a - (s - t)) + (b - t)};
+}
+__device__ __forceinline__ F2 pair_add(F2 a, F2 b) {
+    const F2 s = two_sum(a.h, b.h);
+    const float l = s.l + (a.l + b.l);
+    const float h = s.h + l;
+    return {h, l - (h - s.h)};
+}
+__device__ __forceinline__ F2 pair_xor(F2 v, int o) {
+    return {__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)};
+}
+__device__ __forceinline__ double warp_sum4(const float* v) {
+    const int lane = threadIdx.x & 31;
+    const bool h1 = lane & 16, h2 = lane & 8;
+    const F2 a = two_sum(h1 ? v[2] : v[0], __shfl_xor_sync(0xffffffffu, h1 ? v[0] : v[2], 16));
+    const F2 b = two_sum(h1 ? v[3] : v[1], __shfl_xor_sync(0xffffffffu, h1 ? v[1] : v[3], 16));
+    const F2 give = h2 ? a : b;
+    F2 r = pair_add(h2 ? b : a, pair_xor(give, 8));
+    r = pair_add(r, pair_xor(r, 4));
+    r = pair_add(r, pair_xor(r, 2));
+    r = pair_add(r, pair_xor(r, 1));
+    return (lane & 7) == 0 ? (double)r.h + (double)r.l : 0.0;
+}
+__device__ __forceinline__ double warp_sum4(const double* v) {
+    const int lane = threadIdx.x & 31;
+    const bool h1 = lane & 16, h2 = lane & 8;
+    double a = h1 ? v[2] : v[0], b = h1 ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, h1 ? v[0] : v[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, h1 ? v[1] : v[3], 16);
+    double r = h2 ? b : a;
+    r += __shfl_xor_sync(0xffffffffu, h2 ? a : b, 8);
+    r += __shfl_xor_sync(0xffffffffu, r, 4);
+    r += __shfl_xor_sync(0xffffffffu, r, 2);
+    r += __shfl_xor_sync(0xffffffffu, r, 1);
+    return r;
+}
+// red[warp][k0 + k] = the warp's sums of v[k], k < 4
 template <class TV>
-__device__ __forceinline__ void chunk_dots(const TV* V, size_t ldv, long long off, int len, int j,
-                                           const TV (&wv)[BRPT], double (*red)[BLD]) {
-    for (int k0 = 0; k0 <= j; k0 += BKG) {
-        TV a[BKG][BRPT];
+__device__ __forceinline__ void warp_red4(const TV* v, int k0, double (*red)[BLD]) {
+    const double s = warp_sum4(v);
+    const int lane = threadIdx.x & 31;
+    if ((lane & 7) == 0 && k0 + (lane >> 3) < BLD) red[threadIdx.x >> 5][k0 + (lane >> 3)] = s;
+}
+
+// The vectors of a pass, at most NV of them (NV - 4 < j + 1 <= NV): a thread
+// takes a row at a time and holds its NV vector elements in registers, so
+// pass B reads every element once for the update and the dots.  The loads of
+// a row are unconditional (places past j load vector j again; its
+// coefficient there is 0 and its dot is not read), and in pass A w, which every
+// multiply-add needs, is loaded last, so that they are in flight together:
+// with w first the compiler follows each load by its multiply-add to save
+// registers, and a vector of 28 MB took 16 us instead of 4.4.  UPD: w -= sum_k
+// cf[k] raw_k in vector order, written back, and acc[NV] = its squares.
+template <class TV, int NV, bool UPD>
+__device__ __forceinline__ void chunk_pass(const TV* __restrict__ V, size_t ldv, long long off,
+                                           int len, int j, const TV* cf, TV* w, TV* acc) {
 #pragma unroll
-        for (int kk = 0; kk < BKG; ++kk) {
-            const TV* vk = V + (size_t)(k0 + kk) * ldv + off;
+    for (int k = 0; k < NV + (UPD ? 1 : 0); ++k) acc[k] = (TV)0;
+    const TV* Vr = V + off;
+    for (int row = threadIdx.x; row < len; row += BT) {
+        TV a[NV], x = (TV)0;
+        if (UPD) x = w[row];
 #pragma unroll
-            for (int q = 0; q < BRPT; ++q) {
-                const int row = threadIdx.x + q * BT;
-                a[kk][q] = (k0 + kk <= j && row < len) ? ld_stream(&vk[row]) : (TV)0;
-            }
+        for (int k = 0; k < NV; ++k)
+            a[k] = ld_stream(&Vr[(size_t)(k < NV - 4 ? k : min(k, j)) * ldv + row]);
+        if (!UPD) x = ld_stream(&w[row]);
+        if (UPD) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) x -= cf[k] * a[k];
+            w[row] = x;
+            acc[NV] += x * x;
         }
 #pragma unroll
-        for (int kk = 0; kk < BKG; ++kk) {
-            if (k0 + kk > j) break;
-            TV acc = (TV)0;
-#pragma unroll
-            for (int q = 0; q < BRPT; ++q) {
-                const int row = threadIdx.x + q * BT;
-                if (row < len) acc += a[kk][q] * wv[q];
-            }
-            const double v = warp_sum((double)acc);
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k0 + kk] = v;
-        }
+        for (int k = 0; k < NV; ++k) acc[k] += a[k] * x;
     }
+}
+// the warp sums of a pass's dots
+template <class TV, int NV>
+__device__ __forceinline__ void pass_sums(const TV* acc, double (*red)[BLD]) {
+#pragma unroll
+    for (int k = 0; k < NV; k += 4) warp_red4<TV>(acc + k, k, red);
 }
 
 // wv -= sum_{k <= j} cf[k] raw_k over a chunk, k in order, four vectors'
 // loads in flight at a time
+constexpr int BKG = 4;
 template <class TV>
 __device__ __forceinline__ void chunk_update(const TV* V, size_t ldv, long long off, int len, int j,
                                              const TV* cf, TV (&wv)[BRPT]) {
@@ -392,27 +453,18 @@ __device__ __forceinline__ void chunk_update(const TV* V, size_t ldv, long long 
 }
 
 // ---- CGS2 pass A: h1_k = vscale_k (raw_k . w), k <= j
-template <class TV>
-__global__ void __launch_bounds__(BT)
-k_b_dots(BatchDev B, const TV* __restrict__ V, size_t ldv, int j) {
+template <class TV, int NV>
+__global__ void __launch_bounds__(BT, NV * sizeof(TV) > 64 ? 2 : 3)
+k_b_dots(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     const int c = chunk_of(B);
     const int inst = B.cinst[c];
     if (!B.active[inst]) return;
     __shared__ double red[BT / 32][BLD];
     __shared__ double bsum[BLD], tot[BLD];
     const long long off = B.coff[c];
-    const int len = B.clen[c];
-    const TV* w = V + (size_t)(j + 1) * ldv + off;
-    // per-thread products and sums in the basis precision (FP64 arithmetic
-    // is scarce on this GPU), warp and block sums in FP64; the vectors are
-    // streamed (256-byte L2 fetches)
-    TV wv[BRPT];
-#pragma unroll
-    for (int q = 0; q < BRPT; ++q) {
-        const int row = threadIdx.x + q * BT;
-        wv[q] = row < len ? ld_stream(&w[row]) : (TV)0;
-    }
-    chunk_dots<TV>(V, ldv, off, len, j, wv, red);
+    TV acc[NV];
+    chunk_pass<TV, NV, false>(V, ldv, off, B.clen[c], j, nullptr, V + (size_t)(j + 1) * ldv + off, acc);
+    pass_sums<TV, NV>(acc, red);
     __syncthreads();
     if (!seg_reduce(B, c, inst, red, j + 1, bsum, tot)) return;
     const int ld = B.m + 1;
@@ -422,7 +474,7 @@ k_b_dots(BatchDev B, const TV* __restrict__ V, size_t ldv, int j) {
 
 // ---- CGS2 pass B: w' = w - sum_k h1_k v_k ; h2_k = vscale_k (raw_k . w');
 // hs = h1 + h2, h = h2
-template <class TV>
+template <class TV, int NV>
 __global__ void __launch_bounds__(BT)
 k_b_upd_dots(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     const int c = chunk_of(B);
@@ -432,25 +484,13 @@ k_b_upd_dots(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     __shared__ double bsum[BLD], tot[BLD];
     __shared__ TV cf[BLD];
     const int ld = B.m + 1;
-    for (int k = threadIdx.x; k <= j; k += BT)
-        cf[k] = (TV)(B.h[(size_t)inst * ld + k] * B.vscale[(size_t)inst * ld + k]);
+    for (int k = threadIdx.x; k < NV; k += BT)
+        cf[k] = k <= j ? (TV)(B.h[(size_t)inst * ld + k] * B.vscale[(size_t)inst * ld + k]) : (TV)0;
     __syncthreads();
     const long long off = B.coff[c];
-    const int len = B.clen[c];
-    TV* w = V + (size_t)(j + 1) * ldv + off;
-    TV wv[BRPT];
-#pragma unroll
-    for (int q = 0; q < BRPT; ++q) {
-        const int row = threadIdx.x + q * BT;
-        wv[q] = row < len ? ld_stream(&w[row]) : (TV)0;
-    }
-    chunk_update<TV>(V, ldv, off, len, j, cf, wv);
-#pragma unroll
-    for (int q = 0; q < BRPT; ++q) {
-        const int row = threadIdx.x + q * BT;
-        if (row < len) w[row] = wv[q];
-    }
-    chunk_dots<TV>(V, ldv, off, len, j, wv, red);
+    TV acc[NV + 1];
+    chunk_pass<TV, NV, true>(V, ldv, off, B.clen[c], j, cf, V + (size_t)(j + 1) * ldv + off, acc);
+    pass_sums<TV, NV>(acc, red);
     __syncthreads();
     if (!seg_reduce(B, c, inst, red, j + 1, bsum, tot)) return;
     for (int k = threadIdx.x; k <= j; k += BT) {
@@ -460,55 +500,65 @@ k_b_upd_dots(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     }
 }
 
-// End of Arnoldi step j of one instance (one thread), as the single-system
-// solver: the Hessenberg column (h_{0..j} from hs, h_{j+1} = nrm), the
-// Givens rotations, the residual estimate and the stopping tests.  Returns
-// true while the instance continues with step j + 1 (vscale_{j+1} = 1/nrm).
-__device__ bool b_arnoldi_end(const BatchDev& B, int inst, int j, double nrm) {
-    const int m = B.m, ld = m + 1;
+// End of Arnoldi step j of one instance (one warp), as the single-system
+// solver: hc the Hessenberg column h_0..h_j, a its last entry after the
+// earlier rotations (rotate_column), ss = ||w''||^2; the new rotation, the
+// residual estimate and the stopping tests.  Returns vscale_{j+1} while the
+// instance continues with step j + 1, 0 when it stops; nrm = ||w''||.
+__device__ double b_arnoldi_end(const BatchDev& B, int inst, int j, const double* hc, double a,
+                                double ss, double& nrm) {
+    const int m = B.m, ld = m + 1, lane = threadIdx.x & 31;
     double* Hc = B.H + (size_t)inst * ld * m + (size_t)j * ld;
     double* g = B.g + (size_t)inst * ld;
-    double* cs = B.cs + (size_t)inst * m;
-    double* sn = B.sn + (size_t)inst * m;
-    for (int i = 0; i <= j; ++i) Hc[i] = B.hs[(size_t)inst * ld + i];
-    Hc[j + 1] = nrm;
-    if (!(nrm >= 1e-30)) {
-        if (!isfinite(nrm)) {
+    if (!(ss >= 1e-60)) {  // ||w''|| < 1e-30: breakdown
+        nrm = sqrt(ss);
+        __syncwarp();
+        for (int i = lane; i <= j + 1; i += 32) Hc[i] = i <= j ? hc[i] : nrm;
+        if (lane == 0) {
+            if (!isfinite(nrm)) {
+                B.flags[inst] |= 1;
+                B.done[inst] = 1;
+            }
+            B.flags[inst] |= 2;
+            B.kcount[inst] = j + 1;
+            B.active[inst] = 0;
+        }
+        return 0.0;
+    }
+    const double vs = rsqrt(ss);
+    nrm = ss * vs;
+    const double g0 = g[j], g1 = g[j + 1], est = B.est[inst], bnorm = B.bnorm[inst];
+    double c, s;
+    rot_compute(c, s, a, nrm);
+    const double gj = c * g0 - s * g1, gn = s * g0 + c * g1;
+    const double res = fabs(gn);
+    const bool conv = B.tol_kind == SG_TOL_REF_ABS && res < B.tol;
+    const bool bad = !isfinite(res);
+    const bool stop = conv || bad || j + 1 >= m ||
+                      (B.tol_kind == SG_TOL_TRUE_REL && res * est <= 0.5 * B.tol * bnorm);
+    __syncwarp();
+    if (lane == 0) {
+        Hc[j] = c * a - s * nrm;
+        Hc[j + 1] = s * a + c * nrm;
+        B.cs[(size_t)inst * m + j] = c;
+        B.sn[(size_t)inst * m + j] = s;
+        g[j] = gj;
+        g[j + 1] = gn;
+        vs_put(B, (size_t)inst * ld + j + 1, vs);
+        B.lastres[inst] = res;
+        B.iters[inst] += 1;
+        B.kcount[inst] = j + 1;
+        if (conv) {
+            B.conv[inst] = 1;
+            B.done[inst] = 1;
+        }
+        if (bad) {
             B.flags[inst] |= 1;
             B.done[inst] = 1;
         }
-        B.flags[inst] |= 2;
-        B.kcount[inst] = j + 1;
-        B.active[inst] = 0;
-        return false;
+        if (stop) B.active[inst] = 0;
     }
-    B.vscale[(size_t)inst * ld + j + 1] = 1.0 / nrm;
-    for (int i = 0; i < j; ++i) b_rot_apply(cs[i], sn[i], Hc[i], Hc[i + 1]);
-    b_rot_compute(cs[j], sn[j], Hc[j], Hc[j + 1]);
-    b_rot_apply(cs[j], sn[j], Hc[j], Hc[j + 1]);
-    b_rot_apply(cs[j], sn[j], g[j], g[j + 1]);
-    const double res = fabs(g[j + 1]);
-    B.lastres[inst] = res;
-    B.iters[inst] += 1;
-    B.kcount[inst] = j + 1;
-    bool stop = false;
-    if (B.tol_kind == SG_TOL_REF_ABS) {
-        if (res < B.tol) {
-            B.conv[inst] = 1;
-            B.done[inst] = 1;
-            stop = true;
-        }
-    } else if (B.tol_kind == SG_TOL_TRUE_REL) {
-        if (res * B.est[inst] <= 0.5 * B.tol * B.bnorm[inst]) stop = true;
-    }
-    if (!isfinite(res)) {
-        B.flags[inst] |= 1;
-        B.done[inst] = 1;
-        stop = true;
-    }
-    if (j + 1 >= m) stop = true;
-    if (stop) B.active[inst] = 0;
-    return !stop;
+    return stop ? 0.0 : vs;
 }
 
 // ---- CGS2 pass C: w'' = w' - sum_k h2_k v_k, ||w''||, then the instance's
@@ -548,8 +598,15 @@ k_b_upd_norm(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     double ss = warp_sum((double)ssv);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][0] = ss;
     __syncthreads();
-    if (!seg_reduce(B, c, inst, red, 1, bsum, tot) || threadIdx.x != 0) return;
-    b_arnoldi_end(B, inst, j, sqrt(tot[0]));
+    if (!seg_reduce(B, c, inst, red, 1, bsum, tot)) return;
+    __shared__ double hc[BLD];
+    for (int i = threadIdx.x; i <= j; i += BT) hc[i] = B.hs[(size_t)inst * ld + i];
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const double a = rotate_column(hc, B.cs + (size_t)inst * m, B.sn + (size_t)inst * m,
+                                   B.H + (size_t)inst * ld * m + (size_t)j * ld, j);
+    double nrm;
+    b_arnoldi_end(B, inst, j, hc, a, tot[0], nrm);
 }
 
 // ---- lagged CGS2 (ortho 0, restart < 32), as the single-system solver.
@@ -561,54 +618,54 @@ k_b_upd_norm(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
 //   B  w' = z - S u; r = S^T w'; ||w'||^2; h2 = T^T r; the column is hs +
 //      h2, ||w''||^2 = ||w'||^2 - ||h2||^2, and w' is stored as raw_{j+1}
 //      with its pending correction c = h2 / ||w''||.
-template <class TV>
-__global__ void __launch_bounds__(BT)
-k_b_lag_a(BatchDev B, const TV* __restrict__ V, size_t ldv, int j) {
+// the instance's T (columns and transposed), rows and columns 0..j
+__device__ __forceinline__ void load_T(const double* T, int j, double (*Tm)[BLD], double (*Tt)[BLD]) {
+    const int lane = threadIdx.x & 31;
+    for (int i = threadIdx.x >> 5; i <= j; i += BT / 32)
+        if (lane <= j) {
+            const double v = lane <= i ? T[lane + i * BLD] : 0.0;
+            if (Tm) Tm[i][lane] = v;
+            Tt[lane][i] = v;
+        }
+}
+
+template <class TV, int NV>
+__global__ void __launch_bounds__(BT, NV * sizeof(TV) > 64 ? 2 : 3)
+k_b_lag_a(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     const int c = chunk_of(B);
     const int inst = B.cinst[c];
     if (!B.active[inst]) return;
     __shared__ double red[BT / 32][BLD];
     __shared__ double bsum[BLD], tot[BLD];
-    __shared__ double Ts[BLD][BLD + 1];
+    __shared__ double Tm[BMMAX][BLD], Tt[BMMAX][BLD], Hm[BMMAX][BLD];
     __shared__ double ps[BLD], csh[BLD];
     const long long off = B.coff[c];
-    const int len = B.clen[c];
-    const TV* w = V + (size_t)(j + 1) * ldv + off;
-    TV wv[BRPT];
-#pragma unroll
-    for (int q = 0; q < BRPT; ++q) {
-        const int row = threadIdx.x + q * BT;
-        wv[q] = row < len ? ld_stream(&w[row]) : (TV)0;
-    }
-    chunk_dots<TV>(V, ldv, off, len, j, wv, red);
+    TV acc[NV];
+    chunk_pass<TV, NV, false>(V, ldv, off, B.clen[c], j, nullptr, V + (size_t)(j + 1) * ldv + off, acc);
+    pass_sums<TV, NV>(acc, red);
     __syncthreads();
     if (!seg_reduce(B, c, inst, red, j + 1, bsum, tot)) return;
-    const int ld = B.m + 1, n1 = j + 1;
-    const double* T = B.lagT + (size_t)inst * BLD * BLD;
+    const int ld = B.m + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double* Hn = B.lagH + (size_t)inst * BLD * BMMAX;
-    for (int idx = threadIdx.x; idx < n1 * n1; idx += BT) {
-        const int l = idx % n1, i = idx / n1;
-        Ts[l][i] = l <= i ? T[l + i * BLD] : 0.0;
-    }
+    load_T(B.lagT + (size_t)inst * BLD * BLD, j, Tm, Tt);
+    for (int k = warp; k < j; k += BT / 32)
+        if (lane <= j) Hm[k][lane] = lane <= k + 1 ? Hn[lane + k * BLD] : 0.0;
     for (int k = threadIdx.x; k < j; k += BT) csh[k] = B.lagc[(size_t)inst * BLD + k];
     __syncthreads();
-    for (int i = threadIdx.x; i <= j; i += BT) {
-        double sp = 0.0;
-        for (int l = 0; l <= i; ++l) sp += Ts[l][i] * tot[l];
-        ps[i] = sp;
+    double g = 0.0;
+    if (warp == 0) {
+        const double p = lane <= j ? lag_rows(Tt, tot, j + 1) : 0.0;
+        if (lane <= j) ps[lane] = p;
+    } else if (warp == 1) {
+        if (lane <= j) g = lag_rows(Hm, csh, j);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i <= j; i += BT) {
-        double g = 0.0;
-        for (int k = (i > 0 ? i - 1 : 0); k < j; ++k) g += Hn[i + k * BLD] * csh[k];
-        B.hs[(size_t)inst * ld + i] = ps[i] - g;
-        double u = 0.0;
-        for (int k = i; k <= j; ++k) u += Ts[i][k] * ps[k];
-        B.cfu[(size_t)inst * BLD + i] = u;
-    }
+    if (lane > j) return;
+    if (warp == 0) B.cfu[(size_t)inst * BLD + lane] = lag_rows(Tm, ps, j + 1);
+    if (warp == 1) B.hs[(size_t)inst * ld + lane] = ps[lane] - g;
 }
 
-template <class TV>
+template <class TV, int NV>
 __global__ void __launch_bounds__(BT)
 k_b_lag_b(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     const int c = chunk_of(B);
@@ -617,106 +674,110 @@ k_b_lag_b(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     __shared__ double red[BT / 32][BLD];
     __shared__ double bsum[BLD], tot[BLD];
     __shared__ TV cf[BLD];
-    __shared__ double Ts[BLD][BLD + 1];
-    __shared__ double h2s[BLD], csn[BLD];
-    __shared__ double s_vs;
-    for (int k = threadIdx.x; k <= j; k += BT) cf[k] = (TV)B.cfu[(size_t)inst * BLD + k];
+    __shared__ double Tm[BMMAX][BLD], Tt[BMMAX][BLD];
+    __shared__ double h2s[BLD], hc[BLD];
+    __shared__ double s_vs, s_n2;
+    for (int k = threadIdx.x; k < NV; k += BT)
+        cf[k] = k <= j ? (TV)B.cfu[(size_t)inst * BLD + k] : (TV)0;
     __syncthreads();
     const long long off = B.coff[c];
-    const int len = B.clen[c];
-    TV* w = V + (size_t)(j + 1) * ldv + off;
-    TV wv[BRPT];
-#pragma unroll
-    for (int q = 0; q < BRPT; ++q) {
-        const int row = threadIdx.x + q * BT;
-        wv[q] = row < len ? ld_stream(&w[row]) : (TV)0;
+    TV acc[NV + 1];
+    chunk_pass<TV, NV, true>(V, ldv, off, B.clen[c], j, cf, V + (size_t)(j + 1) * ldv + off, acc);
+    pass_sums<TV, NV>(acc, red);
+    __syncwarp();
+    {  // ||w'||^2 next to the dots (j + 1 < BLD)
+        const TV sq[4] = {acc[NV], (TV)0, (TV)0, (TV)0};
+        const double s = warp_sum4(sq);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][j + 1] = s;
     }
-    chunk_update<TV>(V, ldv, off, len, j, cf, wv);
-    TV ssv = (TV)0;
-#pragma unroll
-    for (int q = 0; q < BRPT; ++q) {
-        const int row = threadIdx.x + q * BT;
-        if (row < len) {
-            w[row] = wv[q];
-            ssv += wv[q] * wv[q];
-        }
-    }
-    chunk_dots<TV>(V, ldv, off, len, j, wv, red);
-    const double ss = warp_sum((double)ssv);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][j + 1] = ss;
     __syncthreads();
     if (!seg_reduce(B, c, inst, red, j + 2, bsum, tot)) return;
-    const int ld = B.m + 1, n1 = j + 1;
+    const int m = B.m, ld = m + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double* T = B.lagT + (size_t)inst * BLD * BLD;
     double* Hn = B.lagH + (size_t)inst * BLD * BMMAX;
-    for (int idx = threadIdx.x; idx < n1 * n1; idx += BT) {
-        const int l = idx % n1, i = idx / n1;
-        Ts[l][i] = l <= i ? T[l + i * BLD] : 0.0;
+    load_T(T, j, Tm, Tt);
+    for (int i = threadIdx.x; i <= j; i += BT) hc[i] = B.hs[(size_t)inst * ld + i];
+    __syncthreads();
+    if (warp == 0 && lane <= j) {
+        const double h2 = lag_rows(Tt, tot, j + 1);
+        h2s[lane] = h2;
+        const double h = hc[lane] + h2;  // the Hessenberg column
+        hc[lane] = h;
+        B.hs[(size_t)inst * ld + lane] = h;
+        Hn[lane + j * BLD] = h;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i <= j; i += BT) {
-        double h2 = 0.0;
-        for (int l = 0; l <= i; ++l) h2 += Ts[l][i] * tot[l];
-        h2s[i] = h2;
-        const double hc = B.hs[(size_t)inst * ld + i] + h2;  // the Hessenberg column
-        B.hs[(size_t)inst * ld + i] = hc;
-        Hn[i + j * BLD] = hc;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double nrm2 = tot[j + 1];
-        for (int i = 0; i <= j; ++i) nrm2 -= h2s[i] * h2s[i];
+    double a = 0.0, tc = 0.0;
+    if (warp == 0) {
+        a = rotate_column(hc, B.cs + (size_t)inst * m, B.sn + (size_t)inst * m,
+                          B.H + (size_t)inst * ld * m + (size_t)j * ld, j);
+    } else if (warp == 1) {
+        if (lane <= j) tc = lag_rows(Tm, h2s, j + 1);
+    } else if (warp == 2) {
+        const double h2 = lane <= j ? h2s[lane] : 0.0;
+        double nrm2 = tot[j + 1] - warp_sum(h2 * h2);
         if (!(nrm2 > 0.0)) nrm2 = isfinite(nrm2) ? 0.0 : nrm2;
-        const double nrm = sqrt(nrm2);
-        Hn[j + 1 + j * BLD] = nrm;
-        s_vs = b_arnoldi_end(B, inst, j, nrm) ? 1.0 / nrm : 0.0;
+        if (lane == 0) s_n2 = nrm2;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double nrm;
+        const double vs = b_arnoldi_end(B, inst, j, hc, a, s_n2, nrm);
+        if (lane == 0) {
+            Hn[j + 1 + j * BLD] = nrm;
+            s_vs = vs;
+        }
     }
     __syncthreads();
     const double vs = s_vs;
-    if (vs == 0.0) return;
+    if (vs == 0.0 || warp != 1) return;
     // the pending correction of the new stored vector and its column of T:
-    // T(:, j+1) = T(j+1, j+1) e_{j+1} - T(:, 0..j) c
-    for (int k = threadIdx.x; k <= j; k += BT) {
-        csn[k] = h2s[k] * vs;
-        B.lagc[(size_t)inst * BLD + k] = csn[k];
-    }
-    if (threadIdx.x == 0) T[(j + 1) + (j + 1) * BLD] = vs;
-    __syncthreads();
-    for (int l = threadIdx.x; l <= j; l += BT) {
-        double sc = 0.0;
-        for (int k = l; k <= j; ++k) sc += Ts[l][k] * csn[k];
-        T[l + (j + 1) * BLD] = -sc;
+    // T(:, j+1) = T(j+1, j+1) e_{j+1} - T(:, 0..j) c with c = h2 vs
+    if (lane <= j) {
+        B.lagc[(size_t)inst * BLD + lane] = h2s[lane] * vs;
+        T[lane + (j + 1) * BLD] = -tc * vs;
+    } else if (lane == j + 1) {
+        T[lane + (j + 1) * BLD] = vs;
     }
 }
 
-// ---- y = H^{-1} g per instance (src/core/gmres.cpp:131-137)
-__global__ void k_b_backsolve(BatchDev B) {
-    const int inst = blockIdx.x * blockDim.x + threadIdx.x;
+// ---- y = H^{-1} g per instance (src/core/gmres.cpp:131-137), a warp each: a
+// lane per row, column by column from the right, the next column's entries
+// loaded ahead
+__global__ void __launch_bounds__(128) k_b_backsolve(BatchDev B) {
+    __shared__ double ys[4][BMMAX];
+    const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
+    const int inst = blockIdx.x * 4 + wrp;
     if (inst >= B.I || !B.ran[inst]) return;
     const int k = B.kcount[inst];
     const int m = B.m, ld = m + 1;
     const double* H = B.H + (size_t)inst * ld * m;
-    const double* g = B.g + (size_t)inst * ld;
-    double* y = B.y + (size_t)inst * m;
+    double gl = lane < k ? B.g[(size_t)inst * ld + lane] : 0.0;
+    double hn = k > 0 && lane < k ? H[lane + (k - 1) * ld] : 0.0;
+    double y = 0.0;
     for (int i = k - 1; i >= 0; --i) {
-        double yi = g[i];
-        for (int l = i + 1; l < k; ++l) yi -= H[i + l * ld] * y[l];
-        y[i] = yi / H[i + i * ld];
+        const double h = hn;
+        if (i > 0) hn = lane < i ? H[lane + (i - 1) * ld] : 0.0;
+        const double q = gl / h;  // lane i: y_i
+        const double yi = __shfl_sync(0xffffffffu, q, i);
+        if (lane == i) y = yi;
+        if (lane < i) gl -= h * yi;
     }
+    if (lane < BMMAX) ys[wrp][lane] = y;
+    __syncwarp();
+    if (lane >= k) return;
+    B.y[(size_t)inst * m + lane] = y;
     // coefficients of the update x += sum_k (y_k vscale_k) raw_k; lagged
     // CGS2: V y = S (T y)
-    const double* vs = B.vscale + (size_t)inst * ld;
-    const double* T = B.lagged ? B.lagT + (size_t)inst * BLD * BLD : nullptr;
-    for (int i = 0; i < k; ++i) {
-        double c = 0.0;
-        if (T) {
-            for (int l = i; l < k; ++l) c += T[i + l * BLD] * y[l];
-        } else {
-            c = y[i] * vs[i];
-        }
-        B.yd[(size_t)inst * m + i] = c;
-        B.yf[(size_t)inst * m + i] = (float)c;
+    double c = 0.0;
+    if (B.lagged) {
+        const double* T = B.lagT + (size_t)inst * BLD * BLD;
+        for (int l = lane; l < k; ++l) c += T[lane + l * BLD] * ys[wrp][l];
+    } else {
+        c = y * B.vscale[(size_t)inst * ld + lane];
     }
+    B.yd[(size_t)inst * m + lane] = c;
+    B.yf[(size_t)inst * m + lane] = (float)c;
 }
 
 template <class TV>
@@ -792,6 +853,7 @@ struct BatchWork {
     DBuf<int> clist, slist;
     std::vector<int> h_ich0, h_inch;
     DBuf<float> yf;
+    DBuf<float2> vsp;
     DBuf<unsigned> ticket;
     DBuf<double> b64, x64, r64;
     DBuf<float> V32, t32;
@@ -883,6 +945,22 @@ void apply_pc_batched(sg_ctx* ctx, sg_precond* pc, const BatchDev& B, BatchWork*
     }
 }
 
+// the instance of a pass kernel for the step's j + 1 vectors
+#define SG_B_NV(K)                                                                  \
+    do {                                                                            \
+        switch (j / 4) {                                                            \
+        case 0: K<TV, 4><<<nchunks, BT, 0, st>>>(B, V, ldv, j); break;              \
+        case 1: K<TV, 8><<<nchunks, BT, 0, st>>>(B, V, ldv, j); break;              \
+        case 2: K<TV, 12><<<nchunks, BT, 0, st>>>(B, V, ldv, j); break;             \
+        case 3: K<TV, 16><<<nchunks, BT, 0, st>>>(B, V, ldv, j); break;             \
+        case 4: K<TV, 20><<<nchunks, BT, 0, st>>>(B, V, ldv, j); break;             \
+        case 5: K<TV, 24><<<nchunks, BT, 0, st>>>(B, V, ldv, j); break;             \
+        case 6: K<TV, 28><<<nchunks, BT, 0, st>>>(B, V, ldv, j); break;             \
+        default: K<TV, 32><<<nchunks, BT, 0, st>>>(B, V, ldv, j); break;            \
+        }                                                                           \
+        SG_CUDA(cudaGetLastError());                                                \
+    } while (0)
+
 template <class TV>
 void enqueue_batch_cycle(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, const BatchDev& B,
                          BatchWork* w, int nchunks, size_t ldv) {
@@ -924,18 +1002,14 @@ void enqueue_batch_cycle(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, const Bat
         }
         ClassTimer tm(ctx, TK_ORTHO);
         if (B.lagged) {
-            k_b_lag_a<TV><<<nchunks, BT, 0, st>>>(B, V, ldv, j);
-            SG_CUDA(cudaGetLastError());
-            k_b_lag_b<TV><<<nchunks, BT, 0, st>>>(B, V, ldv, j);
-            SG_CUDA(cudaGetLastError());
+            SG_B_NV(k_b_lag_a);
+            SG_B_NV(k_b_lag_b);
             count_launch(ctx);
             count_launch(ctx);
             continue;
         }
-        k_b_dots<TV><<<nchunks, BT, 0, st>>>(B, V, ldv, j);
-        SG_CUDA(cudaGetLastError());
-        k_b_upd_dots<TV><<<nchunks, BT, 0, st>>>(B, V, ldv, j);
-        SG_CUDA(cudaGetLastError());
+        SG_B_NV(k_b_dots);
+        SG_B_NV(k_b_upd_dots);
         k_b_upd_norm<TV><<<nchunks, BT, 0, st>>>(B, V, ldv, j);
         SG_CUDA(cudaGetLastError());
         count_launch(ctx);
@@ -944,7 +1018,7 @@ void enqueue_batch_cycle(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, const Bat
     }
     {
         ClassTimer tm(ctx, TK_UPDATE);
-        k_b_backsolve<<<(B.I + 127) / 128, 128, 0, st>>>(B);
+        k_b_backsolve<<<(B.I + 3) / 4, 128, 0, st>>>(B);
         SG_CUDA(cudaGetLastError());
         k_b_update_x<TV><<<bgrid(ctx, total), BT, 0, st>>>(B, V, ldv, w->row_sys.p, w->x64.p);
         SG_CUDA(cudaGetLastError());
@@ -1064,6 +1138,7 @@ void solve_batched_device(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, int nsys
     dalloc(w->sn, (size_t)I * m);
     dalloc(w->H, I * ld * m);
     dalloc(w->vscale, I * ld);
+    dalloc(w->vsp, I * ld);
     dalloc(w->y, (size_t)I * m);
     dalloc(w->yd, (size_t)I * m);
     dalloc(w->yf, (size_t)I * m);
@@ -1109,7 +1184,7 @@ void solve_batched_device(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, int nsys
     B.active = w->active.p; B.done = w->done.p; B.conv = w->conv.p; B.iters = w->iters.p;
     B.cycles = w->cycles.p; B.kcount = w->kcount.p; B.ran = w->ran.p; B.flags = w->flags.p;
     B.bnorm = w->bnorm.p; B.rnorm = w->rnorm.p; B.est = w->est.p; B.lastres = w->lastres.p;
-    B.g = w->g.p; B.cs = w->cs.p; B.sn = w->sn.p; B.H = w->H.p; B.vscale = w->vscale.p;
+    B.g = w->g.p; B.cs = w->cs.p; B.sn = w->sn.p; B.H = w->H.p; B.vscale = w->vscale.p; B.vsp = w->vsp.p;
     B.y = w->y.p; B.yd = w->yd.p; B.yf = w->yf.p; B.h = w->h.p; B.hs = w->hs.p; B.ticket = w->ticket.p; B.part = w->part.p;
     B.notdone = w->notdone.p;
     B.lagT = w->lagT.p; B.lagH = w->lagH.p; B.lagc = w->lagc.p; B.cfu = w->cfu.p;

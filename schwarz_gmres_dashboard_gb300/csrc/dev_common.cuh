@@ -480,4 +480,71 @@ __device__ __forceinline__ bool cluster_reduce(double* partials, unsigned* count
     return true;
 }
 
+// ----------------------------------------------------- least-squares update
+// Givens rotation of src/core/gmres.cpp:9-30 (1 / sqrt(1 + t^2) as one rsqrt:
+// one rounding less)
+__device__ __forceinline__ void rot_compute(double& c, double& s, double a, double b) {
+    if (fabs(b) < 1e-30) {
+        c = 1.0;
+        s = 0.0;
+        return;
+    }
+    const bool big = fabs(b) > fabs(a);
+    const double t = -(big ? a : b) / (big ? b : a);
+    const double r = rsqrt(1.0 + t * t);
+    c = big ? r * t : r;
+    s = big ? r : r * t;
+}
+
+// One warp: the earlier rotations (cs, sn)(0..j-1) of a Hessenberg column
+// hc(0..j).  Rotation i maps the carried entry a_i (a_0 = h_0) to a_{i+1} =
+// s_i a_i + c_i h_{i+1} and leaves r_i = c_i a_i - s_i h_{i+1}: the carried
+// entries are a prefix of affine maps, formed in five steps for 32 rotations
+// instead of one after another (a dependent FP64 operation takes ~75 cycles
+// on this chip).  Writes r_0..r_{j-1} to Hc and returns a_j.
+__device__ __forceinline__ double rotate_column(const double* hc, const double* cs,
+                                                const double* sns, double* Hc, int j) {
+    const int lane = threadIdx.x & 31;
+    double a = hc[0];
+    for (int i0 = 0; i0 < j; i0 += 32) {
+        const int i = i0 + lane;
+        const bool in = i < j;
+        const double c = in ? cs[i] : 1.0, sn = in ? sns[i] : 0.0, hn = in ? hc[i + 1] : 0.0;
+        double A = in ? sn : 1.0, B = in ? c * hn : 0.0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double pA = __shfl_up_sync(0xffffffffu, A, o);
+            const double pB = __shfl_up_sync(0xffffffffu, B, o);
+            if (lane >= o) {
+                B = fma(A, pB, B);
+                A *= pA;
+            }
+        }
+        const double next = fma(A, a, B);
+        double cur = __shfl_up_sync(0xffffffffu, next, 1);
+        if (lane == 0) cur = a;
+        if (in) Hc[i] = fma(c, cur, -(sn * hn));
+        a = __shfl_sync(0xffffffffu, next, 31);
+    }
+    return a;
+}
+
+// sum_k M[k][lane] x[k] over k < n (one warp; a lane per row, four sums each)
+template <int LD>
+__device__ __forceinline__ double lag_rows(const double (*M)[LD], const double* x, int n) {
+    const int lane = threadIdx.x & 31;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    int k = 0;
+    for (; k + 4 <= n; k += 4) {
+        s0 = fma(M[k][lane], x[k], s0);
+        s1 = fma(M[k + 1][lane], x[k + 1], s1);
+        s2 = fma(M[k + 2][lane], x[k + 2], s2);
+        s3 = fma(M[k + 3][lane], x[k + 3], s3);
+    }
+    if (k < n) s0 = fma(M[k][lane], x[k], s0);
+    if (k + 1 < n) s1 = fma(M[k + 1][lane], x[k + 1], s1);
+    if (k + 2 < n) s2 = fma(M[k + 2][lane], x[k + 2], s2);
+    return (s0 + s1) + (s2 + s3);
+}
+
 }  // namespace sg

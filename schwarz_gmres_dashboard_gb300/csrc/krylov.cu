@@ -31,21 +31,6 @@ namespace {
 constexpr int KT = 256;    // threads of the Krylov kernels
 constexpr int BS_T = 256;  // threads of the back substitution (loads; one warp solves)
 
-// Givens rotation of src/core/gmres.cpp:9-30 (1 / sqrt(1 + t^2) as one rsqrt:
-// one rounding less)
-__device__ __forceinline__ void rot_compute(double& c, double& s, double a, double b) {
-    if (fabs(b) < 1e-30) {
-        c = 1.0;
-        s = 0.0;
-        return;
-    }
-    const bool big = fabs(b) > fabs(a);
-    const double t = -(big ? a : b) / (big ? b : a);
-    const double r = rsqrt(1.0 + t * t);
-    c = big ? r * t : r;
-    s = big ? r : r * t;
-}
-
 // State the end of an Arnoldi step reads, brought to shared memory in one round
 // of loads: the column h(0..j),
 // the earlier rotations, g(j..j+1) and the stopping-test scalars.
@@ -85,40 +70,7 @@ __device__ __forceinline__ void finalize_load(FinalizeIn& f, const SolveState* s
     }
 }
 
-// One warp: the column's earlier rotations.  Rotation i maps the carried entry
-// a_i (a_0 = h_0) to a_{i+1} = s_i a_i + c_i h_{i+1} and leaves r_i = c_i a_i -
-// s_i h_{i+1}: the carried entries are a prefix of affine maps, formed in five
-// steps for 32 rotations instead of one after another.  Writes r_0..r_{j-1}
-// to H's column j and returns a_j.
-__device__ double rotate_column(SolveState* st, const FinalizeIn& f, int j, int m) {
-    const int lane = threadIdx.x & 31;
-    const double* hc = f.hc;
-    double* Hc = st->H + (size_t)j * (m + 1);
-    double a = hc[0];
-    for (int i0 = 0; i0 < j; i0 += 32) {
-        const int i = i0 + lane;
-        const bool in = i < j;
-        const double c = in ? f.csv[i] : 1.0, sn = in ? f.snv[i] : 0.0, hn = in ? hc[i + 1] : 0.0;
-        double A = in ? sn : 1.0, B = in ? c * hn : 0.0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double pA = __shfl_up_sync(0xffffffffu, A, o);
-            const double pB = __shfl_up_sync(0xffffffffu, B, o);
-            if (lane >= o) {
-                B = fma(A, pB, B);
-                A *= pA;
-            }
-        }
-        const double next = fma(A, a, B);
-        double cur = __shfl_up_sync(0xffffffffu, next, 1);
-        if (lane == 0) cur = a;
-        if (in) Hc[i] = fma(c, cur, -(sn * hn));
-        a = __shfl_sync(0xffffffffu, next, 31);
-    }
-    return a;
-}
-
-// The same warp: completes Arnoldi step j from a = rotate_column and ss =
+// One warp: completes Arnoldi step j from a = rotate_column and ss =
 // ||w''||^2: normalisation, the new rotation, residual estimate and stopping
 // test.  Returns the new vector's scale 1/||w''|| when the cycle goes on, 0
 // when it stops here (breakdown, convergence, last step); nrm = ||w''||.
@@ -193,7 +145,7 @@ __device__ void arnoldi_finalize(SolveState* st, int j, int m, double ss, double
     __syncthreads();
     if (threadIdx.x < 32) {
         double nrm;
-        const double a = rotate_column(st, f, j, m);
+        const double a = rotate_column(f.hc, f.csv, f.snv, st->H + (size_t)j * (m + 1), j);
         finalize_warp(st, f, j, m, a, ss, hist, hist_cap, nrm);
     }
 }
@@ -350,23 +302,6 @@ __device__ __forceinline__ void lag_prefetch(LagIn& in, const SolveState* st, in
     }
 }
 
-// sum_k M[k][lane] x[k] over k < n (one warp; a lane per row, four sums each)
-__device__ __forceinline__ double lag_rows(const double (*M)[SG_LAGM + 1], const double* x,
-                                           int n) {
-    const int lane = threadIdx.x & 31;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int k = 0;
-    for (; k + 4 <= n; k += 4) {
-        s0 = fma(M[k][lane], x[k], s0);
-        s1 = fma(M[k + 1][lane], x[k + 1], s1);
-        s2 = fma(M[k + 2][lane], x[k + 2], s2);
-        s3 = fma(M[k + 3][lane], x[k + 3], s3);
-    }
-    if (k < n) s0 = fma(M[k][lane], x[k], s0);
-    if (k + 1 < n) s1 = fma(M[k + 1][lane], x[k + 1], s1);
-    if (k + 2 < n) s2 = fma(M[k + 2][lane], x[k + 2], s2);
-    return (s0 + s1) + (s2 + s3);
-}
 // pass A's end (all threads of the last block; d = tot[0..j]): p = T^T d,
 // hsum = p - g with g = H c, update coefficients u = T p
 __device__ void lagged_pass_a(SolveState* st, int j, const double* d, const LagIn& in) {
@@ -407,7 +342,7 @@ __device__ void lagged_pass_b(SolveState* st, int j, int m, const double* r, dou
     }
     __syncthreads();
     if (warp == 0) {
-        a = rotate_column(st, in.f, j, m);
+        a = rotate_column(in.f.hc, in.f.csv, in.f.snv, st->H + (size_t)j * (m + 1), j);
     } else if (warp == 1) {
         if (lane <= j) tc = lag_rows(in.T, h2_s, j + 1);
     } else if (warp == 2) {

@@ -230,15 +230,6 @@ k_pack_rec(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
 template <int R>
 struct FVec;
 template <>
-struct FVec<2> {
-    __device__ __forceinline__ static void ld(uint32_t a, float (&v)[2]) {
-        asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "r"(a) : "memory");
-    }
-    __device__ __forceinline__ static void st(uint32_t a, const float (&v)[2]) {
-        asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(a), "f"(v[0]), "f"(v[1]) : "memory");
-    }
-};
-template <>
 struct FVec<4> {
     __device__ __forceinline__ static void ld(uint32_t a, float (&v)[4]) {
         asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
@@ -364,18 +355,6 @@ __device__ __forceinline__ double div_recip(double a, double d, double y) {
     return q;
 }
 
-// R vector elements of one slot
-template <class TS, int R>
-__device__ __forceinline__ void slot_ld(uint32_t a, TS (&v)[R]) {
-    if constexpr (R > 1) FVec<R>::ld(a, v);
-    else v[0] = lds<TS>(a);
-}
-template <class TS, int R>
-__device__ __forceinline__ void slot_st(uint32_t a, const TS (&v)[R]) {
-    if constexpr (R > 1) FVec<R>::st(a, v);
-    else sts(a, v[0]);
-}
-
 // ---- the gather and the restricted scatter of the TMA-fed sweep.  Rows are
 // spread over the threads (consecutive rows on consecutive lanes, so index
 // loads, element copies and stores stay coalesced) and each thread keeps
@@ -480,8 +459,8 @@ __device__ __forceinline__ void scatter_ilp(const TS* t, TO* __restrict__ y, lon
 // mbarrier (group % RING_NBAR).  Per group (int4): x = stream offset, y =
 // bytes / 16 | ring position / 16 << 16, z = its first entry, w = the groups
 // that may have been issued once it is done.  Per entry (int2), one pass over
-// at most the level threads' number of rows (component records: one entry a
-// level): x = rows left of the level | 0x10000 when a barrier follows, y = the
+// at most as many rows as the level threads take (component records: one entry
+// a level): x = rows left of the level | 0x10000 when a barrier follows, y = the
 // record's byte offset in the ring.  An entry of no rows ends a group.
 struct RingSub {
     long long base;
@@ -652,7 +631,12 @@ __device__ __forceinline__ void level_loop_any(const int2* ent, int j0, int j1, 
 //    quotient correctly with it, div_recip);
 //  * the lanes past a level's end take the row that computes 0 in the unused
 //    slot, so no store is conditional within a warp;
-//  * a level of more than NC rows is several entries of the schedule.
+//  * a level of more rows than the threads take is several entries of the
+//    schedule;
+//  * of R interleaved right-hand sides a thread takes one, R neighbouring lanes
+//    a row (their struct loads are one broadcast): a level of the small
+//    subdomains that are solved in batches has ~20 rows, and a thread with all
+//    four spent ~350 cycles a level issuing their multiply-adds.
 // Cycles per level in isolation, component records with the row's loads after
 // the barrier -> this loop: 51 x 51 FP32 223 -> 104, 15^3 FP32 288 -> 165;
 // 51 x 51 FP64 354 forward, 995 backward -> 214, 270; 14^3 FP64 481, 1159 ->
@@ -667,15 +651,17 @@ __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecR
                                            uint32_t t_s, int NC) {
     using Row = RowRec<W, BACK, TF>;
     constexpr uint32_t ST = (uint32_t)(sizeof(TS) * R);
-    const int tid = threadIdx.x;
+    const int q = threadIdx.x / R;  // this thread's row of a pass
+    t_s += (uint32_t)sizeof(TS) * (threadIdx.x % R);
     for (int j = j0; j < j1; ++j) {
         ring.open(j);
-        const int wid = ring.bad ? 1 << 30 : (tid & ~31);  // first row of this warp
+        // first row of this warp
+        const int wid = ring.bad ? 1 << 30 : ((int)threadIdx.x & ~31) / R;
         int e = ring.grp[j].z;
         const int e1 = ring.grp[j + 1].z - 1;
         int2 md = ent[e], mn = ent[e + 1];
         int c = md.x & 0xffff, sync = md.x >> 16;
-        uint32_t a = ring.ring_s + (uint32_t)(md.y + Row::RB * min(tid, c));
+        uint32_t a = ring.ring_s + (uint32_t)(md.y + Row::RB * min(q, c));
         bool on = wid < c;
         Row row;
         if (on) row.load(a);
@@ -691,12 +677,12 @@ __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecR
             const bool cur = on;
             const int f = sync;
             uint32_t ar = 0;
-            TS xk[W][R], acc[R], vk[W], rd = (TS)1, dg = (TS)1;
+            TS xk[W], acc, vk[W], rd = (TS)1, dg = (TS)1;
             if (cur) {
                 ar = t_s + ST * row.slot(0);
 #pragma unroll
-                for (int k = 0; k < W; ++k) slot_ld<TS, R>(t_s + ST * row.slot(k + 1), xk[k]);
-                slot_ld<TS, R>(ar, acc);
+                for (int k = 0; k < W; ++k) xk[k] = lds<TS>(t_s + ST * row.slot(k + 1));
+                acc = lds<TS>(ar);
 #pragma unroll
                 for (int k = 0; k < W; ++k) vk[k] = row.template value<TS>(k);
                 if (BACK) rd = row.template recip<TS>(0);
@@ -705,24 +691,18 @@ __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecR
             md = mn;
             c = md.x & 0xffff;
             sync = md.x >> 16;
-            a = ring.ring_s + (uint32_t)(md.y + Row::RB * min(tid, c));
+            a = ring.ring_s + (uint32_t)(md.y + Row::RB * min(q, c));
             on = wid < c;
             mn = ent[e + 2];
             if (on) row.load(a);
             if (cur) {
 #pragma unroll
-                for (int k = 0; k < W; ++k)
-#pragma unroll
-                    for (int i = 0; i < R; ++i)
-                        acc[i] = sub_mul<TS, EXACT>(acc[i], vk[k], xk[k][i]);
+                for (int k = 0; k < W; ++k) acc = sub_mul<TS, EXACT>(acc, vk[k], xk[k]);
                 if (BACK) {
-#pragma unroll
-                    for (int i = 0; i < R; ++i) {
-                        if constexpr (EXACT && sizeof(TS) == 8) acc[i] = div_recip(acc[i], dg, rd);
-                        else acc[i] = acc[i] * rd;
-                    }
+                    if constexpr (EXACT && sizeof(TS) == 8) acc = div_recip(acc, dg, rd);
+                    else acc = acc * rd;
                 }
-                slot_st<TS, R>(ar, acc);
+                sts(ar, acc);
             }
             if (f) level_sync(NC);
         }
@@ -1091,6 +1071,7 @@ void launch_tma(sg_precond* pc, const RingPlan& plan, const TI* x, TO* y, int mo
 static bool ring_schedule(const sg_precond* pc, RingPlan& plan, long long budget, long long gmax,
                           int nlt) {
     const int sf = rec_value_bytes(pc);
+    const int pass = std::max(1, nlt / plan.R);  // rows the level threads take at once
     std::vector<RingSub> subs((size_t)pc->nparts);
     std::vector<int> ent, grp;  // int2 / int4 entries as ints
     struct Group {
@@ -1123,7 +1104,7 @@ static bool ring_schedule(const sg_precond* pc, RingPlan& plan, long long budget
                 groups.back().last = g;
                 groups.back().bytes = rel + B - groups.back().start;
             }
-            nent += pc->rec_rows && rec_is_rows(w) ? (c + nlt - 1) / nlt : 1;
+            nent += pc->rec_rows && rec_is_rows(w) ? (c + pass - 1) / pass : 1;
         }
         r.ngrp = (int)(groups.size() - g0);
         r.nent = nent + 1;  // the loop reads one entry past the last
@@ -1182,7 +1163,7 @@ static bool ring_schedule(const sg_precond* pc, RingPlan& plan, long long budget
                 const long long rel = (back ? pc->h_rec_off_b[i] : pc->h_rec_off_f[i]) - r.base;
                 const int at = (int)(gr[j].pos + rel - gr[j].start);
                 const bool rows = pc->rec_rows && rec_is_rows(w);
-                const int step = rows ? nlt : c, rb = rec_row_bytes(w, back, sf);
+                const int step = rows ? pass : c, rb = rec_row_bytes(w, back, sf);
                 for (int q = 0; q < c; q += step, ++ne) {
                     ent.push_back((c - q) | (q + step >= c ? 0x10000 : 0));
                     ent.push_back(at + (rows ? q * rb : 0));
@@ -1683,7 +1664,8 @@ static long long plan_check(sg_precond* pc, const RingPlan& plan, int plant) {
                 const long long B = rec_level_bytes(pc, w, back, c);
                 const long long rel = (back ? pc->h_rec_off_b[i] : pc->h_rec_off_f[i]) - r.base;
                 const bool rows = pc->rec_rows && rec_is_rows(w);
-                const int step = rows ? plan.level_threads : c, rb = rec_row_bytes(w, back, sf);
+                const int step = rows ? std::max(1, plan.level_threads / plan.R) : c;
+                const int rb = rec_row_bytes(w, back, sf);
                 // the ring copy holds the whole record, in this group's bytes
                 const long long at = gpos + rel - gstart;
                 if (rel < gstart || rel + B > gstart + gbytes) ++bad;

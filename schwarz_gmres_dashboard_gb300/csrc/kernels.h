@@ -99,7 +99,11 @@ void rec_setup_device(sg_precond* pc);
 template <class TI, class TO>
 bool sweep_tma(sg_precond* pc, const TI* x, TO* y, int mode, bool coarse, bool exact,
                const int* active);
-// reads the sweeps' error word (0: none) and clears it
+// reads the sweeps' error word (0: none) and clears it: the copy to the host
+// queued behind the work (fetch) and read after the caller's own
+// synchronisation (fetched), or both with a synchronisation between
+void sweep_error_fetch(sg_precond* pc);
+int sweep_error_fetched(sg_precond* pc);
 int sweep_error(sg_precond* pc);
 // four right-hand sides ld apart at once (RAS, FP32 sweeps); false: use four
 // single applies
@@ -121,7 +125,10 @@ void learned_begin(sg_learned* L, SolveState* st);
 void learned_monitor(sg_learned* L, SolveState* st);
 void learned_detach(sg_learned* L);
 uint64_t learned_gen(const sg_learned* L);  // changes when the stage's matrix changes
-int learned_error(sg_learned* L);  // a convolution's bounded wait ran out (read and cleared)
+// a convolution's bounded wait ran out (read and cleared; as for the sweeps)
+void learned_error_fetch(sg_learned* L);
+int learned_error_fetched(sg_learned* L);
+int learned_error(sg_learned* L);
 
 // ---------------------------------------------------------------- batched.cu
 // nsys independent systems (block-diagonal A, rows of system s at

@@ -652,6 +652,17 @@ __global__ void k_pack_batch(const float* __restrict__ in, const float* __restri
     }
 }
 
+// packed inputs of a batch given as (input, feature) pairs
+__global__ void k_pack_pairs(const float2* __restrict__ in, size_t total, uint32_t* __restrict__ X) {
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total;
+         q += (size_t)gridDim.x * blockDim.x) {
+        const float2 v = in[q];
+        uint4* x4 = reinterpret_cast<uint4*>(X + q * 8);
+        x4[0] = make_uint4(pack_bf16(v.x, v.y), 0u, 0u, 0u);
+        x4[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
 // cell-centred trilinear stencil along one axis: fine index fc -> coarse
 // cells c = fc/2 (weight 3/4) and its neighbour towards fc (weight 1/4,
 // clamped to the grid)
@@ -881,7 +892,8 @@ struct LearnedImpl {
     DBuf<float> feat;                        // coefficient feature of A
     DBuf<double> partials;
     DBuf<unsigned> counter;
-    DBuf<int> cerr;  // set by a convolution whose bounded wait ran out
+    DBuf<int> cerr;         // set by a convolution whose bounded wait ran out
+    PinnedBuf<int> cerr_h;  // its copy on the host
     int wait_test = 0;  // testing: 1 / 2 make the convolutions' copy / MMA waits give up
     DBuf<float> az32;   // A z of the stage's residual (FP32 values)
     DBuf<double> az64;  // the same for the FP64 training pairs
@@ -905,6 +917,7 @@ struct LearnedImpl {
     int tb = 0;
     DBuf<uint32_t> tact[4], tg[2];
     DBuf<float> ty, tt, tpart, tloss, tu, tw;
+    DBuf<float2> tx;  // the caller's input pairs
     DBuf<int> tidx;
     long long adam_t = 0;
     float out_scale = 1.f;
@@ -1012,6 +1025,7 @@ void ensure_train(sg_learned* L, int batch) {
     for (int i = 0; i < 2; ++i) L->tg[i].alloc(V * 8 * batch);
     L->ty.alloc(V * batch);
     L->tt.alloc(V * batch);
+    L->tx.alloc(V * batch);
     const int t = L->cx / TB;  // a smaller batch may have more blocks, up to the cap
     L->tpart.alloc((size_t)std::min(t * t * t * batch, L->ctx->num_sms * WGRAD_BLOCKS) * NLAYERS *
                    LAYER_P);
@@ -1202,19 +1216,34 @@ void check_ready(const sg_learned* L) {
     if (!L->A) fail(SG_ERR_NOT_SETUP, "learned stage has no matrix (sg_learned_set_matrix)");
 }
 
-void check_conv(sg_learned* L) {
-    if (learned_error(L))
+void check_fetched(sg_learned* L) {
+    if (learned_error_fetched(L))
         fail(SG_ERR_DEVICE_TIMEOUT, "a learned-stage convolution gave up waiting for its tile");
+}
+void check_conv(sg_learned* L) {
+    learned_error_fetch(L);
+    SG_CUDA(cudaStreamSynchronize(L->ctx->stream));
+    check_fetched(L);
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------- hooks
+void learned_error_fetch(sg_learned* L) {
+    if (!L || !L->cerr.p) return;
+    SG_CUDA(cudaMemcpyAsync(L->cerr_h.p, L->cerr.p, sizeof(int), cudaMemcpyDeviceToHost,
+                            L->ctx->stream));
+}
+
 int learned_error(sg_learned* L) {
+    learned_error_fetch(L);
+    if (L) SG_CUDA(cudaStreamSynchronize(L->ctx->stream));
+    return learned_error_fetched(L);
+}
+
+int learned_error_fetched(sg_learned* L) {
     if (!L || !L->cerr.p) return 0;
-    int e = 0;
-    SG_CUDA(cudaMemcpyAsync(&e, L->cerr.p, sizeof(int), cudaMemcpyDeviceToHost, L->ctx->stream));
-    SG_CUDA(cudaStreamSynchronize(L->ctx->stream));
+    const int e = *L->cerr_h.p;
     if (e) {  // reported once
         L->cerr.zero(L->ctx->stream);
         SG_CUDA(cudaStreamSynchronize(L->ctx->stream));
@@ -1307,13 +1336,14 @@ uint64_t splitmix(uint64_t& s) {
 }
 double unit(uint64_t& s) { return (double)(splitmix(s) >> 11) * (1.0 / 9007199254740992.0); }
 
-void split_pairs(const float* x, size_t V, std::vector<float>& in, std::vector<float>& ft) {
-    in.resize(V);
-    ft.resize(V);
-    for (size_t q = 0; q < V; ++q) {
-        in[q] = x[2 * q];
-        ft[q] = x[2 * q + 1];
-    }
+// the caller's (input, feature) pairs, unpacked on the device
+void upload_pairs(sg_learned* L, const float* x, int batch) {
+    sg_ctx* ctx = L->ctx;
+    const size_t V = (size_t)L->nc * batch;
+    SG_CUDA(cudaMemcpyAsync(L->tx.p, x, sizeof(float2) * V, cudaMemcpyHostToDevice, ctx->stream));
+    k_pack_pairs<<<kblocks(ctx, V), 256, 0, ctx->stream>>>(L->tx.p, V, L->tact[0].p);
+    SG_CUDA(cudaGetLastError());
+    count_launch(ctx);
 }
 }  // namespace
 
@@ -1374,6 +1404,7 @@ sg_status sg_learned_create(sg_ctx* ctx, int nx, int ny, int nz, sg_learned** ou
             L->counter.alloc(1);
             L->counter.zero(ctx->stream);
             L->cerr.alloc(1);
+            L->cerr_h.alloc(1);
             L->cerr.zero(ctx->stream);
             SG_CUDA(cudaFuncSetAttribute(k_conv3d_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          TC_SMEM));
@@ -1765,20 +1796,13 @@ sg_status sg_learned_forward(sg_learned* L, const float* x, int batch, float* y)
         SG_CUDA(cudaSetDevice(ctx->device));
         ensure_train(L, batch);
         const size_t V = (size_t)L->nc * batch;
-        std::vector<float> in, ft;
-        split_pairs(x, V, in, ft);
-        DBuf<float> din, dft;
-        din.upload(in, ctx->stream);
-        dft.upload(ft, ctx->stream);
-        k_pack_batch<<<kblocks(ctx, V), 256, 0, ctx->stream>>>(din.p, dft.p, nullptr, nullptr, batch,
-                                                              L->nc, 1.f, L->tact[0].p, nullptr);
-        SG_CUDA(cudaGetLastError());
-        count_launch(ctx);
+        upload_pairs(L, x, batch);
         forward(L, L->tact[0].p, L->tact[1].p, L->tact[2].p, L->tact[3].p, L->ty.p, batch, nullptr,
                 nullptr);
         SG_CUDA(cudaMemcpyAsync(y, L->ty.p, sizeof(float) * V, cudaMemcpyDeviceToHost, ctx->stream));
+        learned_error_fetch(L);
         SG_CUDA(cudaStreamSynchronize(ctx->stream));
-        check_conv(L);
+        check_fetched(L);
     });
 }
 
@@ -1791,24 +1815,17 @@ sg_status sg_learned_gradient(sg_learned* L, const float* x, const float* t, int
         SG_CUDA(cudaSetDevice(ctx->device));
         ensure_train(L, batch);
         const size_t V = (size_t)L->nc * batch;
-        std::vector<float> in, ft;
-        split_pairs(x, V, in, ft);
-        DBuf<float> din, dft, dt;
-        din.upload(in, ctx->stream);
-        dft.upload(ft, ctx->stream);
-        dt.upload(t, V, ctx->stream);
-        k_pack_batch<<<kblocks(ctx, V), 256, 0, ctx->stream>>>(din.p, dft.p, dt.p, nullptr, batch,
-                                                              L->nc, 1.f, L->tact[0].p, L->tt.p);
-        SG_CUDA(cudaGetLastError());
-        count_launch(ctx);
+        upload_pairs(L, x, batch);
+        SG_CUDA(cudaMemcpyAsync(L->tt.p, t, sizeof(float) * V, cudaMemcpyHostToDevice, ctx->stream));
         L->tloss.zero(ctx->stream);
         loss_grad(L, batch, true, false, nullptr);
         float l = 0.f;
         SG_CUDA(cudaMemcpyAsync(&l, L->tloss.p, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
         SG_CUDA(cudaMemcpyAsync(grad, L->grad.p, sizeof(float) * NET_PARAMS, cudaMemcpyDeviceToHost,
                                 ctx->stream));
+        learned_error_fetch(L);
         SG_CUDA(cudaStreamSynchronize(ctx->stream));
-        check_conv(L);
+        check_fetched(L);
         *loss = l;
     });
 }

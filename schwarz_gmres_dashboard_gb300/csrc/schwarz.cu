@@ -866,6 +866,7 @@ void factor_and_pack(sg_precond* pc) {
     }
     if (!pc->err_d.p) {
         pc->err_d.alloc(1);
+        if (!pc->err_h.p) pc->err_h.alloc(1);
         pc->err_d.zero(ctx->stream);
     }
     if (pc->wide_cols) {

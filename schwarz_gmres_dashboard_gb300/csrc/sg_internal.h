@@ -406,7 +406,8 @@ struct sg_precond {
     sg::DBuf<long long> rec_off_f_d, rec_off_b_d;
     sg::DBuf<int> rec_rows_f_d, rec_rows_b_d;
     sg::DBuf<unsigned char> rec_d;
-    sg::DBuf<int> err_d;  // device error word of the sweeps (bounded waits)
+    sg::DBuf<int> err_d;      // device error word of the sweeps (bounded waits)
+    sg::PinnedBuf<int> err_h; // its copy on the host
     int wait_test = 0;     // sg_precond_set_wait_test mode (0: normal)
     sg::DBuf<double> gscratch64;
     sg::DBuf<float> gscratch32;

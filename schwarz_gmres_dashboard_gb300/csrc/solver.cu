@@ -330,7 +330,10 @@ void solve_device(sg_ctx* ctx, int solver, const sg_csr* A, sg_precond* pc, cons
         w->graph = nullptr;
         throw;
     }
-    // the state now holds the FP64 true residual of the returned x
+    // the state now holds the FP64 true residual of the returned x; the error
+    // words are read with it
+    if (pc) sweep_error_fetch(pc);
+    if (pc && pc->learned) learned_error_fetch(pc->learned);
     SG_CUDA(cudaMemcpyAsync(hs, w->st.p, ctl_bytes, cudaMemcpyDeviceToHost, ctx->stream));
     SG_CUDA(cudaStreamSynchronize(ctx->stream));
     const auto t1 = std::chrono::high_resolution_clock::now();
@@ -350,9 +353,9 @@ void solve_device(sg_ctx* ctx, int solver, const sg_csr* A, sg_precond* pc, cons
             SG_CUDA(cudaMemcpy(prm.history, ctx->hist.p, sizeof(double) * cnt,
                                cudaMemcpyDeviceToHost));
     }
-    if (pc && sweep_error(pc))
+    if (pc && sweep_error_fetched(pc))
         fail(SG_ERR_DEVICE_TIMEOUT, "a subdomain sweep gave up waiting for its factor records");
-    if (pc && pc->learned && learned_error(pc->learned))
+    if (pc && pc->learned && learned_error_fetched(pc->learned))
         fail(SG_ERR_DEVICE_TIMEOUT, "a learned-stage convolution gave up waiting for its tile");
     if (pc) {
         const int hst = host_precond_status(pc);

@@ -1303,6 +1303,7 @@ void rec_setup_device(sg_precond* pc) {
     pc->rec_rows_b_d.upload(pc->h_rec_rows_b, st);
     pc->rec_d.alloc((size_t)pc->rec_total);
     pc->err_d.alloc(1);
+    if (!pc->err_h.p) pc->err_h.alloc(1);
     pc->err_d.zero(st);
     const uint16_t* pf = pc->perm_f.p;
     const uint16_t* pb = pc->perm_b.p;
@@ -1506,11 +1507,22 @@ bool sweep_tma4(sg_precond* pc, const TI* x, TO* y, long long ld, const int* sub
     return true;
 }
 
+void sweep_error_fetch(sg_precond* pc) {
+    if (pc->err_d.p)
+        SG_CUDA(cudaMemcpyAsync(pc->err_h.p, pc->err_d.p, sizeof(int), cudaMemcpyDeviceToHost,
+                                pc->ctx->stream));
+}
+
 int sweep_error(sg_precond* pc) {
     if (!pc->err_d.p) return 0;
-    int e = 0;
-    SG_CUDA(cudaMemcpyAsync(&e, pc->err_d.p, sizeof(int), cudaMemcpyDeviceToHost, pc->ctx->stream));
+    sweep_error_fetch(pc);
     SG_CUDA(cudaStreamSynchronize(pc->ctx->stream));
+    return sweep_error_fetched(pc);
+}
+
+int sweep_error_fetched(sg_precond* pc) {
+    if (!pc->err_d.p) return 0;
+    const int e = *pc->err_h.p;
     // reported once: clear the error word, the fused restriction's counters
     // and the persistent launches' work counters, which a sweep that gave up
     // may have left mid-count, so the next apply starts clean

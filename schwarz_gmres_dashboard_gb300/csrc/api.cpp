@@ -520,7 +520,7 @@ sg_status sg_precond_setup(sg_precond* pc, const sg_csr* A) {
         // it and only redoes the device factorisation.
         const uint64_t key = structure_key(pc, A, part.data(), nparts, overlap);
         if (!(pc->has_structure && pc->structure_key == key)) {
-            pc->has_structure = false;
+            pc->has_structure = pc->on_device = false;
             // the integer set-up on the device (opts.reserved[5] = 0), unless
             // its bitmaps would not fit; else, or when asked (1), on host threads
             pc->setup_on_device = pc->opts.reserved[5] == 0 &&

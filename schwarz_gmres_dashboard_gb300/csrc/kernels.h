@@ -95,7 +95,7 @@ void precond_apply_device(sg_precond* pc, const TI* x, TO* y, const int* active,
                           bool exact = true);
 
 // ---------------------------------------------------------------- sweep.cu
-void rec_setup_device(sg_precond* pc);
+void rec_setup_device(sg_precond* pc, bool kept);
 template <class TI, class TO>
 bool sweep_tma(sg_precond* pc, const TI* x, TO* y, int mode, bool coarse, bool exact,
                const int* active);

@@ -844,8 +844,34 @@ void pack_launch(sg_precond* pc, TF* lval, TF* uval, TF* udiag) {
     SG_CUDA(cudaGetLastError());
 }
 
+// the integer set-up's arrays -> device
+void upload_structure(sg_precond* pc) {
+    cudaStream_t st = pc->ctx->stream;
+    pc->info.upload(pc->h_info, st);
+    pc->order.upload(pc->h_order, st);
+    pc->dofs.upload(pc->sub, st);
+    pc->lev_ptr_f.upload(pc->h_lev_ptr_f, st);
+    pc->lev_ptr_b.upload(pc->h_lev_ptr_b, st);
+    pc->lrp_d.upload(pc->lrp, st);
+    pc->lci_d.upload(pc->lci, st);
+    pc->ldiag_d.upload(pc->ldiag, st);
+    pc->lmap_d.upload(pc->lmap, st);
+    pc->ownloc_d.upload(pc->ownloc, st);
+    pc->owned_ptr_d.upload(pc->owned_ptr, st);
+    pc->owned_d.upload(pc->owned, st);
+    if (pc->wide_cols) {
+        pc->perm_f.upload(reinterpret_cast<const uint16_t*>(pc->h_perm_f32.data()),
+                          pc->h_perm_f32.size() * 2, st);
+        pc->perm_b.upload(reinterpret_cast<const uint16_t*>(pc->h_perm_b32.data()),
+                          pc->h_perm_b32.size() * 2, st);
+    } else {
+        pc->perm_f.upload(pc->h_perm_f16, st);
+        pc->perm_b.upload(pc->h_perm_b16, st);
+    }
+}
+
 template <class TC>
-void factor_and_pack(sg_precond* pc) {
+void factor_and_pack(sg_precond* pc, bool kept) {
     sg_ctx* ctx = pc->ctx;
     k_factor<TC><<<pc->nparts, SWEEP_T, 0, ctx->stream>>>(
         pc->info.p, pc->lrp_d.p, pc->lci_d.p, pc->ldiag_d.p,
@@ -856,7 +882,7 @@ void factor_and_pack(sg_precond* pc) {
     // with per-row ready flags (reserved[0] = 4)
     const int variant = pc->opts.reserved[0];  // 0 TMA records, 1 level, 4 sync-free
     if (variant != 0) pc->use_rec = false;
-    rec_setup_device(pc);
+    rec_setup_device(pc, kept);
     if (pc->use_rec) return;
     {
         int max_smem = 0;
@@ -905,35 +931,20 @@ void precond_setup_device(sg_precond* pc, const sg_csr* A) {
         SG_CUDA(cudaGetLastError());
         return;
     }
-    // ---- batched ILU(0): host structures -> device
-    pc->info.upload(pc->h_info, st);
-    pc->order.upload(pc->h_order, st);
-    pc->dofs.upload(pc->sub, st);
-    pc->lev_ptr_f.upload(pc->h_lev_ptr_f, st);
-    pc->lev_ptr_b.upload(pc->h_lev_ptr_b, st);
-    pc->lrp_d.upload(pc->lrp, st);
-    pc->lci_d.upload(pc->lci, st);
-    pc->ldiag_d.upload(pc->ldiag, st);
-    pc->lmap_d.upload(pc->lmap, st);
-    pc->ownloc_d.upload(pc->ownloc, st);
-    pc->owned_ptr_d.upload(pc->owned_ptr, st);
-    pc->owned_d.upload(pc->owned, st);
-    
-    if (pc->wide_cols) {
-        pc->perm_f.upload(reinterpret_cast<const uint16_t*>(pc->h_perm_f32.data()),
-                          pc->h_perm_f32.size() * 2, st);
-        pc->perm_b.upload(reinterpret_cast<const uint16_t*>(pc->h_perm_b32.data()),
-                          pc->h_perm_b32.size() * 2, st);
-    } else {
-        pc->perm_f.upload(pc->h_perm_f16, st);
-        pc->perm_b.upload(pc->h_perm_b16, st);
-    }
+    // ---- batched ILU(0): host structures -> device.  After a set-up of the
+    // same structure they are there already, and every buffer has its size.
+    const bool kept = pc->on_device;
+    pc->on_device = false;
+    auto reserve = [&](auto& b, size_t count) {
+        if (!kept) b.alloc(count);
+    };
+    if (!kept) upload_structure(pc);
     const long long nz = (long long)pc->lci.size();
-    pc->lu_d.alloc((size_t)nz);
+    reserve(pc->lu_d, (size_t)nz);
     k_gather_vals<<<ctx->num_sms * 4, 256, 0, st>>>(nz, pc->lmap_d.p, A->val.p, pc->lu_d.p);
     SG_CUDA(cudaGetLastError());
-    if (pc->wide_cols) factor_and_pack<int>(pc);
-    else factor_and_pack<uint16_t>(pc);
+    if (pc->wide_cols) factor_and_pack<int>(pc, kept);
+    else factor_and_pack<uint16_t>(pc, kept);
     if (!pc->use_smem && !pc->use_rec) {
         const size_t cnt = (size_t)pc->total_rows + (size_t)pc->nparts;
         if (pc->opts.sweep_dtype == SG_FP64) pc->gscratch64.alloc(cnt);
@@ -943,20 +954,22 @@ void precond_setup_device(sg_precond* pc, const sg_csr* A) {
     if (pc->kind == SG_PC_TWOLEVEL_ASM || pc->kind == SG_PC_TWOLEVEL_RAS) {
         const int nc = pc->nparts;
         pc->nc = nc;
-        pc->part_d.upload(pc->part, st);
-        pc->cscale_d.upload(pc->h_cscale, st);
-        pc->a0.alloc((size_t)nc * nc);
-        pc->lu0.alloc((size_t)nc * nc);
-        pc->a0inv.alloc((size_t)nc * nc);
-        pc->piv0.alloc(nc);
-        pc->r0.alloc(nc);
-        pc->status_d.alloc(1);
+        if (!kept) {
+            pc->part_d.upload(pc->part, st);
+            pc->cscale_d.upload(pc->h_cscale, st);
+        }
+        reserve(pc->a0, (size_t)nc * nc);
+        reserve(pc->lu0, (size_t)nc * nc);
+        reserve(pc->a0inv, (size_t)nc * nc);
+        reserve(pc->piv0, nc);
+        reserve(pc->r0, nc);
+        reserve(pc->status_d, 1);
         pc->status_d.zero(st);
         const size_t smem = (size_t)nc * (4 + 4);
         SG_CUDA(cudaFuncSetAttribute(k_a0_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
-        pc->a0_own.alloc((size_t)n);
-        pc->a0_rows.alloc((size_t)n);
+        reserve(pc->a0_own, (size_t)n);
+        reserve(pc->a0_rows, (size_t)n);
         k_a0_build<<<nc, A0_T, smem, st>>>(nc, pc->owned_ptr_d.p, pc->owned_d.p, A->rp.p, A->ci.p,
                                            A->val.p, pc->part_d.p, pc->cscale_d.p, pc->a0_own.p,
                                            pc->a0_rows.p, pc->a0.p);
@@ -976,6 +989,7 @@ void precond_setup_device(sg_precond* pc, const sg_csr* A) {
         SG_CUDA(cudaGetLastError());
     }
     SG_CUDA(cudaStreamSynchronize(st));
+    pc->on_device = true;
 }
 
 // ---------------------------------------------------------------- apply

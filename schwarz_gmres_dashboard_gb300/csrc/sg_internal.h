@@ -351,6 +351,7 @@ struct sg_precond {
     sg_precond_opts opts{};
     bool is_setup = false;
     bool has_structure = false;   // integer set-up done for structure_key
+    bool on_device = false;       // ... and its arrays and plans are on the device
     bool setup_on_device = false; // ... by the device kernels (false: host threads)
     uint64_t structure_key = 0;
     int n = 0;

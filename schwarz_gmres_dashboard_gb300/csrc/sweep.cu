@@ -1270,14 +1270,39 @@ static RingFit ring_size(sg_precond* pc, RingPlan& plan) {
 
 void tune_plan(sg_precond* pc, RingPlan& plan, const RingFit& fit);
 
+static void pack_records(sg_precond* pc) {
+    cudaStream_t st = pc->ctx->stream;
+    const uint16_t* pf = pc->perm_f.p;
+    const uint16_t* pb = pc->perm_b.p;
+#define SG_PACK(TF)                                                                        \
+    k_pack_rec<TF><<<pc->nparts, 256, 0, st>>>(                                            \
+        pc->info.p, pc->lrp_d.p, pc->lci_d.p, pc->ldiag_d.p, pc->lu_d.p, pf, pb,            \
+        pc->lev_ptr_f.p, pc->lev_ptr_b.p, pc->rec_off_f_d.p, pc->rec_off_b_d.p,             \
+        pc->rec_rows_f_d.p, pc->rec_rows_b_d.p, pc->rec_rows ? 1 : 0, pc->rec_d.p)
+    if (pc->opts.sweep_dtype == SG_FP64) SG_PACK(double);
+    else if (pc->opts.factor_dtype == SG_BF16) SG_PACK(uint16_t);
+    else SG_PACK(float);
+#undef SG_PACK
+    SG_CUDA(cudaGetLastError());
+}
+
 // Packs the level records in the configured factor type, plans the
 // one-vector ring and times its block size, record-group size and launch
-// shape.
-void rec_setup_device(sg_precond* pc) {
+// shape.  All but the records depends on the structure alone: a set-up with
+// new values of the same structure (kept) packs them again and leaves the
+// rest (the plan's 56 timed sweeps took 3 of the 6.2 ms of a re-set-up at
+// 64^3).
+void rec_setup_device(sg_precond* pc, bool kept) {
     if (!pc->use_rec) return;
     sg_ctx* ctx = pc->ctx;
     cudaStream_t st = ctx->stream;
     RingPlan& plan = pc->ring1;
+    if (kept) {
+        pc->err_d.zero(st);
+        if (pc->coarse_sync.p) pc->coarse_sync.zero(st);
+        pack_records(pc);
+        return;
+    }
     plan.R = 1;
     plan.ready = false;
     pc->ring4.ready = false;  // a new set-up plans the four-vector ring again when asked
@@ -1305,18 +1330,7 @@ void rec_setup_device(sg_precond* pc) {
     pc->err_d.alloc(1);
     if (!pc->err_h.p) pc->err_h.alloc(1);
     pc->err_d.zero(st);
-    const uint16_t* pf = pc->perm_f.p;
-    const uint16_t* pb = pc->perm_b.p;
-#define SG_PACK(TF)                                                                        \
-    k_pack_rec<TF><<<pc->nparts, 256, 0, st>>>(                                            \
-        pc->info.p, pc->lrp_d.p, pc->lci_d.p, pc->ldiag_d.p, pc->lu_d.p, pf, pb,            \
-        pc->lev_ptr_f.p, pc->lev_ptr_b.p, pc->rec_off_f_d.p, pc->rec_off_b_d.p,             \
-        pc->rec_rows_f_d.p, pc->rec_rows_b_d.p, pc->rec_rows ? 1 : 0, pc->rec_d.p)
-    if (pc->opts.sweep_dtype == SG_FP64) SG_PACK(double);
-    else if (pc->opts.factor_dtype == SG_BF16) SG_PACK(uint16_t);
-    else SG_PACK(float);
-#undef SG_PACK
-    SG_CUDA(cudaGetLastError());
+    pack_records(pc);
     // block size (forced by opts.reserved[1], else timed), record-group size
     // and launch shape.  Levels of a 3D subdomain hold ~100+ rows, those of a
     // small 2D one ~20: a 512-thread block then idles at every level

@@ -630,69 +630,154 @@ k_a0_build(int nc, const int* __restrict__ owned_ptr, const int* __restrict__ ow
     }
 }
 
-// Dense LU with partial pivoting, one CTA (src/precond/coarse_solve.h:15-47:
-// first strictly larger magnitude, full row swaps, rounded ops in order).
-__global__ void __launch_bounds__(1024) k_lu(int n, double* L, int* piv, int* status) {
-    __shared__ double s_val[1024];
-    __shared__ int s_idx[1024];
-    __shared__ int s_bad;
-    if (threadIdx.x == 0) s_bad = 0;
-    for (int k = 0; k < n; ++k) {
-        double bv = -1.0;
-        int bi = n;
-        for (int i = k + threadIdx.x; i < n; i += blockDim.x) {
-            const double a = fabs(L[(size_t)i * n + k]);
-            if (a > bv) {
-                bv = a;
-                bi = i;
-            }
-        }
-        s_val[threadIdx.x] = bv;
-        s_idx[threadIdx.x] = bi;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) {
-                const double a = s_val[threadIdx.x + o];
-                const int ai = s_idx[threadIdx.x + o];
-                if (a > s_val[threadIdx.x] || (a == s_val[threadIdx.x] && ai < s_idx[threadIdx.x])) {
-                    s_val[threadIdx.x] = a;
-                    s_idx[threadIdx.x] = ai;
-                }
-            }
-            __syncthreads();
-        }
-        const int mr = s_idx[0];
-        const double mv = s_val[0];
-        if (threadIdx.x == 0) {
-            piv[k] = mr;
-            if (!(mv >= 1e-30)) {
-                s_bad = 1;
-                *status = 1;
-            }
-        }
-        __syncthreads();
-        if (s_bad) return;
-        if (mr != k)
-            for (int j = threadIdx.x; j < n; j += blockDim.x) {
-                const double tmp = L[(size_t)k * n + j];
-                L[(size_t)k * n + j] = L[(size_t)mr * n + j];
-                L[(size_t)mr * n + j] = tmp;
-            }
-        __syncthreads();
-        const double piv_v = L[(size_t)k * n + k];
-        for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x)
-            L[(size_t)i * n + k] = L[(size_t)i * n + k] / piv_v;
-        __syncthreads();
-        const int rows = n - k - 1;
-        const long long cnt = (long long)rows * rows;
-        for (long long q = threadIdx.x; q < cnt; q += blockDim.x) {
-            const int i = k + 1 + (int)(q / rows);
-            const int j = k + 1 + (int)(q % rows);
-            L[(size_t)i * n + j] =
-                __dsub_rn(L[(size_t)i * n + j], __dmul_rn(L[(size_t)i * n + k], L[(size_t)k * n + j]));
+// Dense LU with partial pivoting (src/precond/coarse_solve.h:15-47: first
+// strictly larger magnitude, full row swaps, rounded ops in order), LU_NB
+// columns at a time.  Every entry is updated by the same columns in the same
+// order with the same two roundings wherever it is computed, so the factors do
+// not depend on the blocking, bit for bit.
+//
+// The n^3 / 3 multiplications and subtractions bound it, on FP64 pipes of two
+// lanes a cycle and SM: in one CTA they alone are 2.9 ms at n = 256.  Only a
+// panel's columns need the pivots one by one and stay in one CTA (a thread a
+// row, the panel in shared memory, magnitudes compared as integers, which
+// leave the FP64 pipe alone); the rest is spread over the GPU.  One CTA
+// for all: 0.29 ms at n = 64, 4.28 at 256; now 0.23 and 1.13.
+constexpr int LU_NB = 16;
+constexpr int LU_T = 512;
+constexpr int LU_LD = LU_NB + 1;  // row stride of a panel in shared memory
+__global__ void __launch_bounds__(LU_T)
+k_lu_panel(int n, int k0, int in_smem, double* A, int* piv, int* status) {
+    extern __shared__ __align__(16) unsigned char lu_raw[];
+    __shared__ unsigned long long s_val[LU_T / 32];
+    __shared__ int s_idx[LU_T / 32];
+    if (*status) return;
+    const int rows = n - k0, nb = min(LU_NB, rows), T = blockDim.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double* P = in_smem ? reinterpret_cast<double*>(lu_raw) : A + (size_t)k0 * n + k0;
+    const size_t ld = in_smem ? LU_LD : n;
+    if (in_smem) {
+        for (int t = tid; t < rows * LU_NB; t += T) {
+            const int r = t / LU_NB, c = t % LU_NB;
+            if (c < nb) P[r * ld + c] = A[(size_t)(k0 + r) * n + k0 + c];
         }
         __syncthreads();
     }
+    for (int k = 0; k < nb; ++k) {
+        unsigned long long bv = 0;  // 1 + the bits of |a|, ordered as |a|; 0 for NaN
+        int bi = n;
+        auto better = [&](unsigned long long a, int i) {
+            if (a > bv || (a == bv && i < bi)) {
+                bv = a;
+                bi = i;
+            }
+        };
+        for (int r = k + tid; r < rows; r += T) {
+            const unsigned long long a =
+                (unsigned long long)__double_as_longlong(P[r * ld + k]) & 0x7fffffffffffffffull;
+            if (a <= 0x7ff0000000000000ull) better(a + 1, r);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            better(__shfl_xor_sync(0xffffffffu, bv, o), __shfl_xor_sync(0xffffffffu, bi, o));
+        if (lane == 0) {
+            s_val[warp] = bv;
+            s_idx[warp] = bi;
+        }
+        __syncthreads();
+        for (int w = 0; w < T / 32; ++w) better(s_val[w], s_idx[w]);
+        if (bv < 1 + (unsigned long long)__double_as_longlong(1e-30)) {  // in every thread alike
+            if (tid == 0) *status = 1;
+            return;
+        }
+        if (tid == 0) piv[k0 + k] = k0 + bi;
+        if (bi != k && tid < nb) {
+            const double t = P[k * ld + tid];
+            P[k * ld + tid] = P[bi * ld + tid];
+            P[bi * ld + tid] = t;
+        }
+        __syncthreads();
+        const double d = P[k * ld + k];
+        for (int r = k + 1 + tid; r < rows; r += T) {
+            const double l = P[r * ld + k] / d;
+            P[r * ld + k] = l;
+            for (int c = k + 1; c < nb; c += 4) {  // four at a time: their latencies overlap
+                double a[4], u[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    a[e] = c + e < nb ? P[r * ld + c + e] : 0.0;
+                    u[e] = c + e < nb ? P[k * ld + c + e] : 0.0;
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) a[e] = __dsub_rn(a[e], __dmul_rn(l, u[e]));
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (c + e < nb) P[r * ld + c + e] = a[e];
+            }
+        }
+        __syncthreads();
+    }
+    if (in_smem)
+        for (int t = tid; t < rows * LU_NB; t += T) {
+            const int r = t / LU_NB, c = t % LU_NB;
+            if (c < nb) A[(size_t)(k0 + r) * n + k0 + c] = P[r * ld + c];
+        }
+}
+
+// The panel's row swaps in the other columns, a thread a column, and on its
+// right the panel rows of U.  A thread reads and writes its own column only.
+constexpr int LU_CT = 32;
+__global__ void __launch_bounds__(LU_CT)
+k_lu_rows(int n, int k0, double* A, const int* __restrict__ piv, const int* __restrict__ status) {
+    __shared__ double l[LU_NB][LU_NB];
+    __shared__ double u[LU_NB][LU_CT];
+    if (*status) return;
+    const int nb = min(LU_NB, n - k0), tid = threadIdx.x;
+    const int q = blockIdx.x * LU_CT + tid, j = q < k0 ? q : q + nb;  // columns outside the panel
+    for (int t = tid; t < LU_NB * LU_NB; t += LU_CT) {
+        const int r = t / LU_NB, c = t % LU_NB;
+        l[r][c] = r < nb && c < nb ? A[(size_t)(k0 + r) * n + k0 + c] : 0.0;
+    }
+    __syncthreads();
+    if (j >= n) return;
+#pragma unroll
+    for (int k = 0; k < LU_NB; ++k) u[k][tid] = k < nb ? A[(size_t)(k0 + k) * n + j] : 0.0;
+    for (int k = 0; k < nb; ++k) {
+        const int r = piv[k0 + k];
+        double* p = r < k0 + nb ? &u[r - k0][tid] : &A[(size_t)r * n + j];
+        const double t = *p;
+        *p = u[k][tid];
+        u[k][tid] = t;
+    }
+    double x[LU_NB];
+#pragma unroll
+    for (int k = 0; k < LU_NB; ++k) x[k] = u[k][tid];
+    if (j >= k0 + nb) {
+#pragma unroll
+        for (int k = 0; k < LU_NB; ++k)
+#pragma unroll
+            for (int i = k + 1; i < LU_NB; ++i) x[i] = __dsub_rn(x[i], __dmul_rn(l[i][k], x[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < LU_NB; ++k)
+        if (k < nb) A[(size_t)(k0 + k) * n + j] = x[k];
+}
+
+// The rows and columns after the panel: 16 x 16 tiles, an entry a thread.
+__global__ void __launch_bounds__(256)
+k_lu_update(int n, int k0, double* A, const int* __restrict__ status) {
+    __shared__ double l[LU_NB][LU_NB + 1];
+    __shared__ double u[LU_NB][LU_NB];
+    if (*status) return;
+    const int tx = threadIdx.x % LU_NB, ty = threadIdx.x / LU_NB;
+    const int r = k0 + LU_NB + blockIdx.y * LU_NB + ty, c = k0 + LU_NB + blockIdx.x * LU_NB + tx;
+    const bool in = r < n && c < n;
+    l[ty][tx] = r < n ? A[(size_t)r * n + k0 + tx] : 0.0;
+    u[ty][tx] = c < n ? A[(size_t)(k0 + ty) * n + c] : 0.0;
+    double a = in ? A[(size_t)r * n + c] : 0.0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < LU_NB; ++k) a = __dsub_rn(a, __dmul_rn(l[ty][k], u[k][tx]));
+    if (in) A[(size_t)r * n + c] = a;
 }
 
 // Column t of A0^{-1} from the LU factors (one CTA per column): pivots and
@@ -844,6 +929,34 @@ void pack_launch(sg_precond* pc, TF* lval, TF* uval, TF* udiag) {
     SG_CUDA(cudaGetLastError());
 }
 
+// LU of the n x n matrix A in place, a panel at a time
+void dense_lu(sg_ctx* ctx, int n, double* A, int* piv, int* status) {
+    cudaStream_t st = ctx->stream;
+    int max_smem = 0;
+    SG_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    // static scratch and the block's own kilobyte beside the panel; a panel of
+    // more rows works in global memory
+    const size_t room = (size_t)max_smem - 2048;
+    SG_CUDA(cudaFuncSetAttribute(k_lu_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)room));
+    for (int k0 = 0; k0 < n; k0 += LU_NB) {
+        const int nb = std::min(LU_NB, n - k0), rest = n - k0 - nb;
+        const size_t smem = (size_t)(n - k0) * LU_LD * sizeof(double);
+        const bool fits = smem <= room;
+        k_lu_panel<<<1, std::min(LU_T, (n - k0 + 31) & ~31), fits ? smem : 0, st>>>(n, k0, fits ? 1 : 0, A, piv, status);
+        SG_CUDA(cudaGetLastError());
+        if (n > nb) {
+            k_lu_rows<<<(n - nb + LU_CT - 1) / LU_CT, LU_CT, 0, st>>>(n, k0, A, piv, status);
+            SG_CUDA(cudaGetLastError());
+        }
+        if (rest > 0) {
+            const unsigned t = (unsigned)(rest + LU_NB - 1) / LU_NB;
+            k_lu_update<<<dim3(t, t), 256, 0, st>>>(n, k0, A, status);
+            SG_CUDA(cudaGetLastError());
+        }
+    }
+}
+
 // the integer set-up's arrays -> device
 void upload_structure(sg_precond* pc) {
     cudaStream_t st = pc->ctx->stream;
@@ -976,8 +1089,7 @@ void precond_setup_device(sg_precond* pc, const sg_csr* A) {
         SG_CUDA(cudaGetLastError());
         SG_CUDA(cudaMemcpyAsync(pc->lu0.p, pc->a0.p, sizeof(double) * nc * nc,
                                 cudaMemcpyDeviceToDevice, st));
-        k_lu<<<1, 1024, 0, st>>>(nc, pc->lu0.p, pc->piv0.p, pc->status_d.p);
-        SG_CUDA(cudaGetLastError());
+        dense_lu(ctx, nc, pc->lu0.p, pc->piv0.p, pc->status_d.p);
         int bad = 0;
         SG_CUDA(cudaMemcpyAsync(&bad, pc->status_d.p, sizeof(int), cudaMemcpyDeviceToHost, st));
         SG_CUDA(cudaStreamSynchronize(st));

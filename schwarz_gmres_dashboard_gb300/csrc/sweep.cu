@@ -197,6 +197,9 @@ __device__ __forceinline__ void pack_level(const SubInfo& inf, const int* rp, co
     }
 }
 
+// Block (s, y) packs every gridDim.y-th level of subdomain s: a row is a few
+// dependent loads, so one block a subdomain waits most of its time (64
+// subdomains of 64^3: 0.35 ms, with 16 blocks each 0.057).
 template <class TF>
 __global__ void __launch_bounds__(256)
 k_pack_rec(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
@@ -212,12 +215,12 @@ k_pack_rec(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
     const double* v = lu + inf.csr_nz_off;
     const int* dg = ldiag + inf.row_off;
     const bool sf = row_structs && rec_is_rows(inf.wl), sb = row_structs && rec_is_rows(inf.wu);
-    for (int l = 0; l < inf.nlev_f; ++l) {
+    for (int l = blockIdx.y; l < inf.nlev_f; l += gridDim.y) {
         const int i = inf.lev_off_f + l, p0 = lev_f[i];
         pack_level<TF, false>(inf, rp, ci, dg, v, perm_f + inf.row_off + p0, lev_f[i + 1] - p0,
                               rows_f[i], inf.wl, sf, rec + off_f[i]);
     }
-    for (int l = 0; l < inf.nlev_b; ++l) {
+    for (int l = blockIdx.y; l < inf.nlev_b; l += gridDim.y) {
         const int i = inf.lev_off_b + l, p0 = lev_b[i];
         pack_level<TF, true>(inf, rp, ci, dg, v, perm_b + inf.row_off + p0, lev_b[i + 1] - p0,
                              rows_b[i], inf.wu, sb, rec + off_b[i]);
@@ -1274,8 +1277,9 @@ static void pack_records(sg_precond* pc) {
     cudaStream_t st = pc->ctx->stream;
     const uint16_t* pf = pc->perm_f.p;
     const uint16_t* pb = pc->perm_b.p;
+    const int per = std::min(16, std::max(1, 8 * pc->ctx->num_sms / pc->nparts));
 #define SG_PACK(TF)                                                                        \
-    k_pack_rec<TF><<<pc->nparts, 256, 0, st>>>(                                            \
+    k_pack_rec<TF><<<dim3(pc->nparts, per), 256, 0, st>>>(                                 \
         pc->info.p, pc->lrp_d.p, pc->lci_d.p, pc->ldiag_d.p, pc->lu_d.p, pf, pb,            \
         pc->lev_ptr_f.p, pc->lev_ptr_b.p, pc->rec_off_f_d.p, pc->rec_off_b_d.p,             \
         pc->rec_rows_f_d.p, pc->rec_rows_b_d.p, pc->rec_rows ? 1 : 0, pc->rec_d.p)

@@ -340,6 +340,7 @@ struct RingPlan {
     DBuf<unsigned char> sub_d;
     DBuf<int> ent_d, grp_d;
     DBuf<unsigned> work;       // persistent launches: next subdomain, CTAs done
+    std::map<const void*, int> resident;  // CTAs of a kernel that the GPU holds at once
 };
 
 }  // namespace sg

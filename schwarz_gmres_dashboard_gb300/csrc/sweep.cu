@@ -502,8 +502,9 @@ struct RecArgs {
     int persist;
     unsigned* work;
     // coarse restriction fused into the sweep (cooperative launch, all blocks
-    // resident): each block writes r0[s] and counts itself in sync[0]; sync[1]
-    // counts the blocks done with r0 (the last one resets both)
+    // resident): each restriction is written to r0[s] and counted in sync[0];
+    // sync[1] counts the subdomains done with r0 (the last one resets both).
+    // Blocks from nparts on compute restrictions only.
     int fuse;
     double* r0w;
     unsigned* sync;
@@ -744,6 +745,19 @@ struct SweepSmem {
     double* a0row;        // nc (a0pre)
 };
 
+// The coarse restriction of subdomain s (the order of k_restrict), published
+// for the blocks that add the coarse term.
+template <class TI>
+__device__ __forceinline__ void publish_restriction(const RecArgs& a, int s, const SubInfo& inf,
+                                                    const TI* __restrict__ x, double* red) {
+    const double z = restrict_chunks<TI>(a.owned + inf.own_off, x, inf.n_own, red);
+    if (threadIdx.x == 0) {
+        a.r0w[s] = inf.cscale * z;
+        __threadfence();
+        if (a.wait_test != 2) atomicAdd(&a.sync[0], 1u);
+    }
+}
+
 // One subdomain: stage its schedule, start its record stream, gather its
 // right-hand side(s) (and, in the fused two-level mode, the coarse
 // restrictions this block owes), run both sweeps, add the coarse term and
@@ -809,22 +823,15 @@ __device__ __forceinline__ bool sweep_one(const RecArgs& a, int s, const TI* __r
     }
     cp_async_wait_all();
     if (threadIdx.x < R) t[(size_t)R * tslot(n, tp) + threadIdx.x] = (TS)0;
-    if (coarse && a.fuse && (int)blockIdx.x >= (int)gridDim.x / 2) {
-        // coarse restrictions (the order of k_restrict), published for the
-        // other blocks before the level loop.  Blocks run largest subdomain
-        // first, so the second half -- the smaller subdomains, with slack --
-        // computes its own and its mirror block's, and the critical first
-        // half computes none.
-        const int mirror = (int)gridDim.x - 1 - (int)blockIdx.x;
+    if (coarse && a.fuse && (int)gridDim.x == a.nparts && (int)blockIdx.x >= a.nparts / 2) {
+        // no blocks to spare for the restrictions.  Blocks run largest
+        // subdomain first, so the second half -- the smaller subdomains, with
+        // slack -- computes its own and its mirror block's before the level
+        // loop, and the critical first half computes none.
+        const int mirror = a.nparts - 1 - (int)blockIdx.x;
         for (int pass = 0; pass < (mirror == (int)blockIdx.x ? 1 : 2); ++pass) {
             const int sr = pass == 0 ? s : a.order[mirror];
-            const SubInfo ir = pass == 0 ? inf : a.info[sr];
-            const double z = restrict_chunks<TI>(a.owned + ir.own_off, x, ir.n_own, s_red);
-            if (threadIdx.x == 0) {
-                a.r0w[sr] = ir.cscale * z;
-                __threadfence();
-                if (a.wait_test != 2) atomicAdd(&a.sync[0], 1u);
-            }
+            publish_restriction<TI>(a, sr, pass == 0 ? inf : a.info[sr], x, s_red);
         }
     }
     __syncthreads();
@@ -852,7 +859,7 @@ __device__ __forceinline__ bool sweep_one(const RecArgs& a, int s, const TI* __r
             if (threadIdx.x == 0) {
                 const long long t0 = clock64();
                 int ok = 1;
-                while (ld_acquire(&a.sync[0]) < gridDim.x) {
+                while (ld_acquire(&a.sync[0]) < (unsigned)a.nparts) {
                     if (clock64() - t0 > a.wait_budget) {
                         ok = 0;
                         break;
@@ -874,7 +881,7 @@ __device__ __forceinline__ bool sweep_one(const RecArgs& a, int s, const TI* __r
             if (threadIdx.x == 0) {
                 s_zc = inf.cscale * z;
                 // the last block done with r0 resets the counters
-                if (a.fuse && atomicAdd(&a.sync[1], 1u) == gridDim.x - 1) {
+                if (a.fuse && atomicAdd(&a.sync[1], 1u) == (unsigned)a.nparts - 1) {
                     a.sync[0] = 0u;
                     a.sync[1] = 0u;
                 }
@@ -936,6 +943,15 @@ k_sweep_tma(const __grid_constant__ RecArgs a, const TI* __restrict__ x, TO* __r
     };
     int gbase = 0;  // record groups this CTA has streamed (mbarrier phases)
     if constexpr (!PERSIST) {
+        if (a.fuse && (int)blockIdx.x >= a.nparts) {
+            double* red = reinterpret_cast<double*>(sm.ring);  // the ring and vector are unused
+            for (int q = (int)blockIdx.x - a.nparts; q < a.nparts; q += (int)gridDim.x - a.nparts) {
+                const int sr = a.order[q];
+                publish_restriction<TI>(a, sr, a.info[sr], x, red);
+                __syncthreads();
+            }
+            return;
+        }
         const int s = a.order[blockIdx.x];
         if (!on(s)) return;  // subdomain not needed by this apply
         sweep_one<TI, TO, TS, TF, EXACT, R>(a, s, x, y, mode, coarse, sm, gbase, true);
@@ -1021,6 +1037,16 @@ size_t sweep_smem(const sg_precond* pc, const RingPlan& plan) {
     return sweep_smem_for(pc, plan, plan.ring_bytes);
 }
 
+// Blocks of the fused sweep that compute restrictions only: one a subdomain,
+// or as many as still fit when that leaves each at most four.  32 subdomains
+// of a 201 x 187 grid: sweep 35.7 -> 31.4 us; 108 of 96^3 (44 blocks): apply
+// 167 -> 164; with 48 blocks for 256 subdomains of 128^3 66.4 -> 66.6, so not
+// there (the second half of the sweeping blocks has the time).
+int restrict_blocks(int nparts, int cap) {
+    const int room = std::min(nparts, cap - nparts);
+    return room > 0 && 4LL * room >= nparts ? room : 0;
+}
+
 template <class TI, class TO, class TS, class TF, bool EXACT, int R>
 void launch_tma(sg_precond* pc, const RingPlan& plan, const TI* x, TO* y, int mode, bool coarse,
                 const int* active, bool fuse = false, long long ldx = 0, long long ldy = 0) {
@@ -1040,9 +1066,17 @@ void launch_tma(sg_precond* pc, const RingPlan& plan, const TI* x, TO* y, int mo
     const int coarse_i = coarse ? 1 : 0;
     if (fuse) {
         // the blocks wait for one another's restriction: co-residency is
-        // guaranteed by the cooperative launch (checked at set-up)
+        // guaranteed by the cooperative launch (checked at set-up).  Where the
+        // GPU holds more blocks than subdomains, the others take the
+        // restrictions off the sweeping ones.
+        auto& cap = const_cast<RingPlan&>(plan).resident[reinterpret_cast<const void*>(kern)];
+        if (cap == 0) {
+            int per_sm = 0;
+            SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem));
+            cap = per_sm * pc->ctx->num_sms;
+        }
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(pc->nparts);
+        cfg.gridDim = dim3(pc->nparts + restrict_blocks(pc->nparts, cap));
         cfg.blockDim = dim3(nt);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = pc->ctx->stream;
@@ -1406,6 +1440,7 @@ void tune_plan(sg_precond* pc, RingPlan& plan, const RingFit& fit) {
         if (bf16) return sweep_occupancy(pc, plan, k_sweep_tma<float, float, float, uint16_t, false, 1, false>);
         return sweep_occupancy(pc, plan, k_sweep_tma<float, float, float, float, false, 1, false>);
     };
+    plan.resident.clear();
     cudaEvent_t e0, e1;
     SG_CUDA(cudaEventCreate(&e0));
     SG_CUDA(cudaEventCreate(&e1));

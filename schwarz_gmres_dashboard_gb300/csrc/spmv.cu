@@ -165,6 +165,77 @@ __device__ __forceinline__ int sell_col(const int16_t* col, long long e, int r, 
     return r + (int)ldg_stream(&col[e], pol);
 }
 
+// CSR SpMV for rows of uneven lengths (those SELL refuses): a block takes 256
+// rows, forms their products together as in k_spmv_csr, and deals the rows to
+// its threads by length, so a warp adds rows of about one length.  With a
+// lane's own row each, every addition of the longest row of 32 takes the FP64
+// pipe the time of a full warp's: 720,000 rows of 2 to ~50 entries, 10
+// million in all, 185 us in k_spmv_csr, 76 here (8,192 rows 17 and 9).  Per row the order and the
+// rounding are the same.
+template <class TV, class TX, class TY>
+__global__ void __launch_bounds__(SPMV_THREADS, 4)
+k_spmv_uneven(int n, const int* __restrict__ rp, const int* __restrict__ ci,
+              const TV* __restrict__ val, const TX* __restrict__ x, TY* __restrict__ y,
+              const double* __restrict__ scale, const int* __restrict__ active) {
+    if (active && *active == 0) return;
+    constexpr int VN = VecT<TV>::N, CAP = 4096, BINS = 64;
+    using VV = typename VecT<TV>::V;
+    using VI = typename VecT<TV>::I;
+    __shared__ TV w[CAP];
+    __shared__ int start[SPMV_THREADS + 1];
+    __shared__ int bin[BINS];
+    __shared__ unsigned char row_of[SPMV_THREADS];
+    const int tid = threadIdx.x;
+    const TV sc = scale ? (TV)(*scale) : (TV)1;
+    for (int r0 = blockIdx.x * SPMV_THREADS; r0 < n; r0 += gridDim.x * SPMV_THREADS) {
+        __syncthreads();  // the previous rows are done with
+        start[tid] = __ldg(&rp[min(r0 + tid, n)]);
+        if (tid == 0) start[SPMV_THREADS] = __ldg(&rp[min(r0 + SPMV_THREADS, n)]);
+        if (tid < BINS) bin[tid] = 0;
+        __syncthreads();
+        const int len = min(start[tid + 1] - start[tid], BINS - 1);
+        const int at = atomicAdd(&bin[len], 1);
+        __syncthreads();
+        if (tid < 32) {  // bins -> their first positions
+            const int a = bin[2 * tid], b = bin[2 * tid + 1];
+            int s = a + b;
+#pragma unroll
+            for (int o = 1; o < 32; o *= 2) {
+                const int t = __shfl_up_sync(0xffffffffu, s, o);
+                if (tid >= o) s += t;
+            }
+            bin[2 * tid] = s - a - b;
+            bin[2 * tid + 1] = s - b;
+        }
+        __syncthreads();
+        row_of[bin[len] + at] = (unsigned char)tid;
+        __syncthreads();
+        const int q = row_of[tid];
+        const int rs = start[q], re = start[q + 1], end = start[SPMV_THREADS];
+        TV sum = (TV)0;
+        for (int ws = start[0]; ws < end; ws += CAP) {
+            const int we = min(ws + CAP, end);
+#pragma unroll 2
+            for (int e0 = (ws & ~(VN - 1)) + tid * VN; e0 < we; e0 += SPMV_THREADS * VN) {
+                TV v[VN];
+                int c[VN];
+                unpack<TV, VV>(__ldg(reinterpret_cast<const VV*>(val + e0)), v);
+                unpacki(__ldg(reinterpret_cast<const VI*>(ci + e0)), c);
+#pragma unroll
+                for (int u = 0; u < VN; ++u) {
+                    const int e = e0 + u;
+                    if (e >= ws && e < we) w[e - ws] = pmul(v[u], (TV)__ldg(&x[c[u]]));
+                }
+            }
+            __syncthreads();
+            const int lo = max(rs, ws), hi = min(re, we);
+            for (int e = lo; e < hi; ++e) sum = padd(sum, w[e - ws]);
+            __syncthreads();
+        }
+        if (r0 + q < n) y[r0 + q] = (TY)(scale ? pmul(sum, sc) : sum);
+    }
+}
+
 // SELL-32 SpMV: a warp per slice of 32 rows, a lane per row; every load of
 // a step k is one contiguous 32-element segment.  MODE 0: same per-row order
 // and rounding as the CSR kernel (padding adds exact zeros at the end of a
@@ -590,6 +661,13 @@ void launch_spmv_a(sg_ctx* ctx, const sg_csr* A, const TX* x, TY* y, const doubl
         int cfg = sell_cfg_of<TV>(A);
         if (cfg < 0 || kSellCfgs[cfg].dcol != (fmt == 3)) cfg = fmt == 3 ? 3 : 0;
         launch_sell<TV, TX, TY>(ctx, A, cfg, x, y, scale, active);
+    } else if (!A->sell_ok) {
+        const int blocks = (A->nrows + SPMV_THREADS - 1) / SPMV_THREADS;
+        k_spmv_uneven<TV, TX, TY>
+            <<<std::min(blocks, ctx->num_sms * 8), SPMV_THREADS, 0, ctx->stream>>>(
+                A->nrows, A->rp.p, A->ci.p, csr_vals<TV>(A), x, y, scale, active);
+        SG_CUDA(cudaGetLastError());
+        count_launch(ctx);
     } else {
         launch_spmv<TV, TX, TY>(ctx, A->nrows, A->rp.p, A->ci.p, csr_vals<TV>(A), x, y, scale,
                                 active);

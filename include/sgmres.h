@@ -290,7 +290,7 @@ typedef struct sg_solve_params {
     /* orthogonalisation of the Arnoldi step (the reference uses modified
      * Gram-Schmidt, src/core/gmres.cpp:288-292): 0 = CGS2 in the fewest
      * streaming passes -- two (second projection deferred by one step) when
-     * the cycle's operator is linear (GMRES, restart < 32), else three;
+     * restart < 32 (GMRES and FGMRES), else three;
      * 1 = classic CGS2, three passes per step */
     int ortho;
     int reserved[7];

@@ -666,7 +666,7 @@ class GMRESParams:
     tol_kind: int = TOL_REF_ABS
     precision: int = FP64
     use_graph: bool = True
-    # 0: CGS2 in the fewest passes (two for linear GMRES cycles, restart < 32);
+    # 0: CGS2 in the fewest passes (two with restart < 32, else three);
     # 1: classic three-pass CGS2
     ortho: int = 0
 

@@ -36,7 +36,7 @@ void launch_bnorm(sg_ctx* ctx, const double* v, int n, SolveState* st);
 template <class TV>
 void launch_cycle_init(sg_ctx* ctx, const TV* raw0, int n, SolveState* st, int m, bool flexible);
 // One CGS2 Arnoldi step on raw[j+1] against raw[0..j] (with the Givens
-// update of the least-squares problem done by the last block); lagged: the
+// update of the least-squares problem done by the last cluster); lagged: the
 // two-pass variant with the second projection carried to the next step
 // (st->lagged must be set for the whole solve, m < SG_LAGM).
 template <class TV>

@@ -302,7 +302,7 @@ __device__ __forceinline__ void lag_prefetch(LagIn& in, const SolveState* st, in
     }
 }
 
-// pass A's end (all threads of the last block; d = tot[0..j]): p = T^T d,
+// pass A's end (all threads of the block that ends the pass; d = tot[0..j]): p = T^T d,
 // hsum = p - g with g = H c, update coefficients u = T p
 __device__ void lagged_pass_a(SolveState* st, int j, const double* d, const LagIn& in) {
     __shared__ double p_s[SG_LAGM];
@@ -320,7 +320,7 @@ __device__ void lagged_pass_a(SolveState* st, int j, const double* d, const LagI
     if (warp == 1) st->hsum[lane] = p_s[lane] - g;
 }
 
-// pass B's end (all threads of the last block; r = tot[0..j], ss =
+// pass B's end (all threads of that block; r = tot[0..j], ss =
 // ||w'||^2): h2 = T^T r, the column hsum + h2, its rotations (warp 0), the new
 // norm (warp 2), the step's end (warp 0), the new vector's pending correction
 // and T column (warp 1)

@@ -541,7 +541,8 @@ k_sweep_sf(const SubInfo* __restrict__ info, const int* __restrict__ order,
 // terms while the other warps stage the listed rows, A0_CH at a time, and
 // give each other part j a thread that folds its terms.  (One thread per part
 // walking every row and entry: 8.2 ms for 64 parts of 4096 rows, a load's
-// latency per entry; now the fold of the own terms bounds it.)
+// latency per entry; folding all entries of the listed rows 0.94; now 0.50,
+// half of it the listed rows' staging.)
 constexpr int A0_T = 256;
 constexpr int A0_CH = 32;  // listed rows staged at a time
 constexpr int A0_W = 32;   // their entries; longer rows are read from global memory
@@ -557,7 +558,7 @@ k_a0_build(int nc, const int* __restrict__ owned_ptr, const int* __restrict__ ow
     int* flag = reinterpret_cast<int*>(smraw);  // nc
     int* list = flag + nc;                      // nc
     __shared__ int s_nl, s_cnt[A0_T / 32];
-    __shared__ int s_n[A0_CH], s_e[A0_CH], s_p[A0_CH][A0_W], s_q[A0_CH][A0_W];
+    __shared__ int s_n[A0_CH], s_e[A0_CH], s_c[A0_CH], s_p[A0_CH][A0_W], s_q[A0_CH][A0_W];
     __shared__ double s_v[A0_CH][A0_W], s_t[A0_CH][A0_W];
     const int i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q0 = owned_ptr[i], q1 = owned_ptr[i + 1];
@@ -662,12 +663,16 @@ k_a0_build(int nc, const int* __restrict__ owned_ptr, const int* __restrict__ ow
             }
             a0_sync();
             // the rows' terms: at the first entry of each other part, c_i
-            // times the sum of the row's entries in it
-            for (int t = ft; t < nr * 8; t += FT) {
-                const int r = t >> 3, n = s_n[r];
+            // times the sum of the row's entries in it; a row's terms are put
+            // one after another, in its order (most rows have one: a fold over
+            // all seven entries of a row was most of this kernel's time)
+            for (int t = ft; t < A0_CH * 8; t += FT) {
+                const int r = t >> 3, u = t & 7, n = r < nr ? s_n[r] : 0;
+                const unsigned group = 0xffu << (lane & 24);
                 if (n > A0_W) continue;
-                for (int e = t & 7; e < n; e += 8) {
-                    const int p = s_p[r][e];
+                int base = 0;
+                for (int e = u; e - u < n; e += 8) {
+                    const int p = e < n ? s_p[r][e] : i;
                     bool first = p != i;
                     for (int d = 0; d < e && first; ++d) first = s_p[r][d] != p;
                     double acc = 0.0;
@@ -676,27 +681,46 @@ k_a0_build(int nc, const int* __restrict__ owned_ptr, const int* __restrict__ ow
                         for (int d = e; d < n; ++d)
                             if (s_p[r][d] == p) acc = __dadd_rn(acc, __dmul_rn(s_v[r][d], c));
                     }
-                    s_t[r][e] = __dmul_rn(c_i, acc);
-                    s_q[r][e] = first ? p : -1;
+                    const unsigned m = __ballot_sync(group, first) & group;
+                    if (first) {
+                        const int at = base + __popc(m & ((1u << lane) - 1u));
+                        s_t[r][at] = __dmul_rn(c_i, acc);
+                        s_q[r][at] = p;
+                    }
+                    base += __popc(m);
                 }
+                if (u == 0) s_c[r] = base;
             }
             a0_sync();
             if (jj >= 0) {
-                for (int r = 0; r < nr; ++r) {
-                    const int n = s_n[r];
-                    if (n <= A0_W) {
-                        for (int e = 0; e < n; ++e)
-                            if (s_q[r][e] == jj) row = __dadd_rn(row, s_t[r][e]);
-                        continue;
+                for (int r0 = 0; r0 < nr; r0 += 4) {
+                    int n[4], c[4], q[4];
+                    double t[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {  // four rows' first terms in flight
+                        n[u] = r0 + u < nr ? s_n[r0 + u] : 0;
+                        c[u] = r0 + u < nr ? s_c[r0 + u] : 0;
+                        q[u] = s_q[r0 + u][0];
+                        t[u] = s_t[r0 + u][0];
                     }
-                    double acc = 0.0;
-                    bool any = false;
-                    for (int e = s_e[r]; e < s_e[r] + n; ++e) {
-                        if (part[ci[e]] != jj) continue;
-                        acc = __dadd_rn(acc, __dmul_rn(v[e], c_j));
-                        any = true;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int r = r0 + u;
+                        if (n[u] <= A0_W) {
+                            if (c[u] > 0 && q[u] == jj) row = __dadd_rn(row, t[u]);
+                            for (int e = 1; e < c[u]; ++e)
+                                if (s_q[r][e] == jj) row = __dadd_rn(row, s_t[r][e]);
+                            continue;
+                        }
+                        double acc = 0.0;
+                        bool any = false;
+                        for (int e = s_e[r]; e < s_e[r] + n[u]; ++e) {
+                            if (part[ci[e]] != jj) continue;
+                            acc = __dadd_rn(acc, __dmul_rn(v[e], c_j));
+                            any = true;
+                        }
+                        if (any) row = __dadd_rn(row, __dmul_rn(c_i, acc));
                     }
-                    if (any) row = __dadd_rn(row, __dmul_rn(c_i, acc));
                 }
             }
             a0_sync();

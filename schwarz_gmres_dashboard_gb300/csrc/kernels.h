@@ -128,7 +128,6 @@ uint64_t learned_gen(const sg_learned* L);  // changes when the stage's matrix c
 // a convolution's bounded wait ran out (read and cleared; as for the sweeps)
 void learned_error_fetch(sg_learned* L);
 int learned_error_fetched(sg_learned* L);
-int learned_error(sg_learned* L);
 
 // ---------------------------------------------------------------- batched.cu
 // nsys independent systems (block-diagonal A, rows of system s at

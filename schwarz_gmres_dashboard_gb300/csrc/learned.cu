@@ -1235,12 +1235,6 @@ void learned_error_fetch(sg_learned* L) {
                             L->ctx->stream));
 }
 
-int learned_error(sg_learned* L) {
-    learned_error_fetch(L);
-    if (L) SG_CUDA(cudaStreamSynchronize(L->ctx->stream));
-    return learned_error_fetched(L);
-}
-
 int learned_error_fetched(sg_learned* L) {
     if (!L || !L->cerr.p) return 0;
     const int e = *L->cerr_h.p;

@@ -343,12 +343,15 @@ struct RowRec {
 // in one fused multiply-add, rounds the quotient correctly -- five dependent
 // operations where the division takes the time of seven and twice the FP64
 // slots.  Outside the exponents where no residual can lose bits (and for
-// infinities and NaN) the division itself; a zero keeps the sign of a y.
+// infinities and NaN) the division itself; a zero keeps the sign of a y, but
+// not where y overflowed (|d| < 2^-1024: 0 * inf is NaN, 0 / d is 0).
 __device__ __noinline__ double div_plain(double a, double d) { return a / d; }
 __device__ __forceinline__ double div_recip(double a, double d, double y) {
     const int ha = __double2hiint(a);
     const int ea = (ha >> 20) & 0x7ff, ed = (__double2hiint(d) >> 20) & 0x7ff;
-    const bool zero = ((ha << 1) | __double2loint(a)) == 0;  // also the lanes past a level's end
+    // also the lanes past a level's end
+    const bool zero = ((ha << 1) | __double2loint(a)) == 0 &&
+                      (__double2hiint(y) & 0x7ff00000) != 0x7ff00000;
     const double q0 = a * y;
     double q = fma(fma(-q0, d, a), y, q0);
     q = fma(fma(-q, d, a), y, q);

@@ -860,8 +860,7 @@ struct BatchWork {
     DBuf<double> V64, t64;
     int* h_notdone = nullptr;
     // what the instance/chunk tables and the checks were made for
-    const sg_csr* key_A = nullptr;
-    long long key_nnz = -1;
+    uint64_t key_A = 0;  // sg_csr::gen: an address is used again
     int key_nrhs = -1;
     std::vector<int> key_rows;
     const sg_precond* key_pc = nullptr;
@@ -1058,9 +1057,9 @@ void solve_batched_device(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, int nsys
     cudaStream_t st = ctx->stream;
     const std::vector<int> rows(sys_row_ptr, sys_row_ptr + S + 1);
     const bool same_tables =
-        w->key_A == A && w->key_nnz == A->nnz && w->key_nrhs == R && w->key_rows == rows;
+        w->key_A == A->gen && w->key_nrhs == R && w->key_rows == rows;
     if (!same_tables) {
-        w->key_A = nullptr;
+        w->key_A = 0;
         w->key_pc = nullptr;
         // the matrix must be block diagonal over the systems
         for (int s = 0; s < S; ++s)
@@ -1101,8 +1100,7 @@ void solve_batched_device(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, int nsys
         w->nchunks = (int)cinst.size();
         w->h_ich0 = ich0;
         w->h_inch = inch;
-        w->key_A = A;
-        w->key_nnz = A->nnz;
+        w->key_A = A->gen;
         w->key_nrhs = R;
         w->key_rows = rows;
     }

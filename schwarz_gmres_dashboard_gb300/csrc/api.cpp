@@ -284,7 +284,9 @@ sg_status sg_csr_create(sg_ctx* ctx, int nrows, int ncols, int nnz, const int* r
             if (!ok) {  // say where
                 for (int i = 0; i < nrows; ++i) {
                     SG_CHECK_ARG(A->h_rp[i + 1] >= A->h_rp[i], "row_ptr decreases at row %d", i);
-                    for (int e = A->h_rp[i]; e < A->h_rp[i + 1]; ++e)
+                    // a row_ptr that decreases later may pass nnz before
+                    const int end = std::min(A->h_rp[i + 1], nnz);
+                    for (int e = A->h_rp[i]; e < end; ++e)
                         SG_CHECK_ARG(A->h_ci[e] >= 0 && A->h_ci[e] < ncols,
                                      "col_idx[%d] = %d outside [0,%d)", e, A->h_ci[e], ncols);
                 }

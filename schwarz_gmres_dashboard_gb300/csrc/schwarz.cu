@@ -1145,7 +1145,8 @@ void precond_setup_device(sg_precond* pc, const sg_csr* A) {
     }
     // ---- batched ILU(0): host structures -> device.  After a set-up of the
     // same structure they are there already, and every buffer has its size.
-    const bool kept = pc->on_device;
+    // (Records laid out for values that needed the division are planned again.)
+    const bool kept = pc->on_device && !pc->rec_divides;
     pc->on_device = false;
     auto reserve = [&](auto& b, size_t count) {
         if (!kept) b.alloc(count);

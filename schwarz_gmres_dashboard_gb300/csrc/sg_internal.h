@@ -298,7 +298,7 @@ __host__ __device__ __forceinline__ int tslot(int r, int p) { return p ? r + (r 
 // are stored as row structs (when the preconditioner's rec_rows is set): the
 // row's and the columns' slots (16 bits each), the values, and in the backward
 // sweep the diagonal's reciprocal (FP32, also beside BF16 values; FP64 sweeps
-// hold the reciprocal and the diagonal).  After a level's rows comes one that
+// hold the reciprocal in two parts and the diagonal).  After a level's rows comes one that
 // computes t = 0 in the unused slot: the lanes past the level's end take it.
 // The sizes are multiples of 4 (FP64:
 // 8) bytes whose strides spread a warp over the shared-memory banks, hence
@@ -306,7 +306,7 @@ __host__ __device__ __forceinline__ int tslot(int r, int p) { return p ? r + (r 
 //   bytes    W = 2     3      4
 //   BF16     12, 16  16, 20  20, 24    (forward, backward)
 //   FP32     16, 20  20, 24  28, 36
-//   FP64     24, 40  40, 48  48, 72
+//   FP64     24, 48  40, 56  48, 72
 __host__ __device__ constexpr bool rec_is_rows(int w) { return w >= 2 && w <= 4; }
 __host__ __device__ constexpr int rec_val_off(int w, int sf) {
     return (2 * (1 + w) + sf - 1) / sf * sf;
@@ -315,7 +315,7 @@ __host__ __device__ constexpr int rec_recip_off(int w, int sf) {
     return (rec_val_off(w, sf) + w * sf + 3) / 4 * 4;
 }
 __host__ __device__ constexpr int rec_row_bytes(int w, bool back, int sf) {
-    const int b = back ? rec_recip_off(w, sf) + (sf == 8 ? 16 : 4) : rec_recip_off(w, sf);
+    const int b = back ? rec_recip_off(w, sf) + (sf == 8 ? 24 : 4) : rec_recip_off(w, sf);
     return b % 32 == 0 ? b + (sf == 8 ? 8 : 4) : b;
 }
 
@@ -378,6 +378,9 @@ struct sg_precond {
     bool use_sf = false;   // sync-free sweep (per-row ready flags)
     int rec_depth = 0;               // 1 when the TMA-fed sweep is set up (0: not used)
     bool rec_rows = true;            // row structs for levels of width 2 to 4 (rec_layout)
+    bool rec_divides = false;        // ... not, for a diagonal too small or large (rec_setup_device)
+    sg::DBuf<int> far_d;             // set by the packing where one is
+    sg::PinnedBuf<int> far_h;
     // how the level records stream through the sweep's shared-memory ring,
     // for one right-hand side at a time (ring1) and for four interleaved ones
     // (ring4, planned when a batched solve first asks for it)

@@ -140,8 +140,14 @@ template <class TF>
 __device__ __forceinline__ void put_recip(unsigned char* p, double d);
 template <>
 __device__ __forceinline__ void put_recip<double>(unsigned char* p, double d) {
-    reinterpret_cast<double*>(p)[0] = 1.0 / d;
-    reinterpret_cast<double*>(p)[1] = d;
+    const double y = 1.0 / d;
+    reinterpret_cast<double*>(p)[0] = y;
+    reinterpret_cast<double*>(p)[1] = fma(-y, d, 1.0) * y;  // what rounding y left
+    reinterpret_cast<double*>(p)[2] = d;
+}
+// |d| in [2^-300, 2^301): its quotients may be formed from the reciprocal
+__device__ __forceinline__ bool recip_safe(double d) {
+    return (unsigned)(((__double2hiint(d) >> 20) & 0x7ff) - 723) <= 600u;
 }
 template <>
 __device__ __forceinline__ void put_recip<float>(unsigned char* p, double d) {
@@ -157,7 +163,8 @@ __device__ __forceinline__ void put_recip<uint16_t>(unsigned char* p, double d) 
 template <class TF, bool BACK>
 __device__ __forceinline__ void pack_level(const SubInfo& inf, const int* rp, const int* ci,
                                            const int* dg, const double* v, const uint16_t* perm,
-                                           int c, int C, int w, bool rows, unsigned char* R) {
+                                           int c, int C, int w, bool rows, unsigned char* R,
+                                           int* far) {
     constexpr int SF = (int)sizeof(TF);
     const uint16_t zero = (uint16_t)tslot(inf.n, inf.tshift);
     const int rb = rec_row_bytes(w, BACK, SF), vo = rec_val_off(w, SF);
@@ -191,6 +198,7 @@ __device__ __forceinline__ void pack_level(const SubInfo& inf, const int* rp, co
         }
         if (BACK) {
             const double d = q < c ? v[dg[r]] : 1.0;
+            if (SF == 8 && rows && !recip_safe(d)) *far = 1;
             if (rows) put_recip<TF>(P + rec_recip_off(w, SF), d);
             else (vv + (size_t)C * w)[q] = to_factor<TF>(d);
         }
@@ -208,7 +216,7 @@ k_pack_rec(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
            const uint16_t* __restrict__ perm_b, const int* __restrict__ lev_f,
            const int* __restrict__ lev_b, const long long* __restrict__ off_f,
            const long long* __restrict__ off_b, const int* __restrict__ rows_f,
-           const int* __restrict__ rows_b, int row_structs, unsigned char* rec) {
+           const int* __restrict__ rows_b, int row_structs, unsigned char* rec, int* far) {
     const SubInfo inf = info[blockIdx.x];
     const int* rp = lrp + inf.csr_row_off;
     const int* ci = lci + inf.csr_nz_off;
@@ -218,12 +226,12 @@ k_pack_rec(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
     for (int l = blockIdx.y; l < inf.nlev_f; l += gridDim.y) {
         const int i = inf.lev_off_f + l, p0 = lev_f[i];
         pack_level<TF, false>(inf, rp, ci, dg, v, perm_f + inf.row_off + p0, lev_f[i + 1] - p0,
-                              rows_f[i], inf.wl, sf, rec + off_f[i]);
+                              rows_f[i], inf.wl, sf, rec + off_f[i], far);
     }
     for (int l = blockIdx.y; l < inf.nlev_b; l += gridDim.y) {
         const int i = inf.lev_off_b + l, p0 = lev_b[i];
         pack_level<TF, true>(inf, rp, ci, dg, v, perm_b + inf.row_off + p0, lev_b[i + 1] - p0,
-                             rows_b[i], inf.wu, sb, rec + off_b[i]);
+                             rows_b[i], inf.wu, sb, rec + off_b[i], far);
     }
 }
 
@@ -287,7 +295,7 @@ struct RowRec {
     static constexpr int RB = rec_row_bytes(W, BACK, SF);
     static constexpr int VO = rec_val_off(W, SF);
     static constexpr int DO = rec_recip_off(W, SF);
-    static constexpr int NW = (BACK ? DO + (SF == 8 ? 16 : 4) : VO + W * SF + 3) / 4;  // words read
+    static constexpr int NW = (BACK ? DO + (SF == 8 ? 24 : 4) : VO + W * SF + 3) / 4;  // words read
     uint32_t w[(NW + 3) / 4 * 4];
 
     __device__ __forceinline__ void load(uint32_t a) {
@@ -326,7 +334,7 @@ struct RowRec {
             return (TS)__hiloint2double((int)w[VO / 4 + 2 * k + 1], (int)w[VO / 4 + 2 * k]);
         }
     }
-    // FP64 sweeps: i = 0 the reciprocal, 1 the diagonal itself
+    // FP64 sweeps: i = 0 the reciprocal, 1 what rounding it left, 2 the diagonal
     template <class TS>
     __device__ __forceinline__ TS recip(int i) const {
         if constexpr (SF == 8)
@@ -634,8 +642,14 @@ __device__ __forceinline__ void level_loop_any(const int2* ent, int j0, int j1, 
 // code (a divergent branch or an inner loop costs 40 to 80 cycles a level):
 //  * a thread loads the struct of its next row before the barrier, between
 //    the loads of this level's vector elements and their first use;
-//  * the diagonal comes as its reciprocal (exact FP64 sweeps round the
-//    quotient correctly with it, div_recip);
+//  * the diagonal comes as its reciprocal.  Exact FP64 sweeps round the quotient
+//    correctly with it (div_recip); the solver's take the reciprocal in two
+//    parts, a / d = fma(a, y, a y2) (N. Brisebarre, J.-M. Muller, S. K. Raina,
+//    "Accelerating correctly rounded floating-point division when the divisor
+//    is known in advance", 2004): within 2^-104 of the quotient before its one
+//    rounding (2.4 10^9 random and hard quotients all equal the division; a y
+//    alone is another number for 26% of them).  One operation deeper than a y:
+//    solves of 100 x 100 in 4 parts 12.7 -> 13.6 ms, 64^3 in 64 18.1 -> 19.2;
 //  * the lanes past a level's end take the row that computes 0 in the unused
 //    slot, so no store is conditional within a warp;
 //  * a level of more rows than the threads take is several entries of the
@@ -647,7 +661,8 @@ __device__ __forceinline__ void level_loop_any(const int2* ent, int j0, int j1, 
 // Cycles per level in isolation, component records with the row's loads after
 // the barrier -> this loop: 51 x 51 FP32 223 -> 104, 15^3 FP32 288 -> 165;
 // 51 x 51 FP64 354 forward, 995 backward -> 214, 270; 14^3 FP64 481, 1159 ->
-// 414, 519.  Warps without rows still take the predicated FP64 instructions'
+// 414, 519 (backward with a y; with its second part ~80 more, by the solves
+// above).  Warps without rows still take the predicated FP64 instructions'
 // slots of the narrow FP64 pipe, so FP64 sweeps either run their levels on few
 // warps (270 cycles with 2 warps, 507 with 8) or, with FP64_SKIP threads or
 // more, branch around the level in warps that have no rows (SKIP: 350 cycles
@@ -693,7 +708,7 @@ __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecR
 #pragma unroll
                 for (int k = 0; k < W; ++k) vk[k] = row.template value<TS>(k);
                 if (BACK) rd = row.template recip<TS>(0);
-                if (BACK && EXACT) dg = row.template recip<TS>(1);
+                if (BACK && sizeof(TS) == 8) dg = row.template recip<TS>(EXACT ? 2 : 1);
             }
             md = mn;
             c = md.x & 0xffff;
@@ -707,6 +722,7 @@ __device__ __forceinline__ void level_loop(const int2* ent, int j0, int j1, RecR
                 for (int k = 0; k < W; ++k) acc = sub_mul<TS, EXACT>(acc, vk[k], xk[k]);
                 if (BACK) {
                     if constexpr (EXACT && sizeof(TS) == 8) acc = div_recip(acc, dg, rd);
+                    else if constexpr (sizeof(TS) == 8) acc = fma(acc, rd, acc * dg);
                     else acc = acc * rd;
                 }
                 sts(ar, acc);
@@ -1310,8 +1326,17 @@ static RingFit ring_size(sg_precond* pc, RingPlan& plan) {
 
 void tune_plan(sg_precond* pc, RingPlan& plan, const RingFit& fit);
 
-static void pack_records(sg_precond* pc) {
+// Packs the level records.  Returns false where they are row structs of an
+// FP64 sweep and a diagonal is so small, large or non-finite that its quotients
+// have to be divided.
+static bool pack_records(sg_precond* pc) {
     cudaStream_t st = pc->ctx->stream;
+    const bool check = pc->opts.sweep_dtype == SG_FP64 && pc->rec_rows;
+    if (!pc->far_d.p) {
+        pc->far_d.alloc(1);
+        pc->far_h.alloc(1);
+    }
+    if (check) pc->far_d.zero(st);
     const uint16_t* pf = pc->perm_f.p;
     const uint16_t* pb = pc->perm_b.p;
     const int per = std::min(16, std::max(1, 8 * pc->ctx->num_sms / pc->nparts));
@@ -1319,12 +1344,16 @@ static void pack_records(sg_precond* pc) {
     k_pack_rec<TF><<<dim3(pc->nparts, per), 256, 0, st>>>(                                 \
         pc->info.p, pc->lrp_d.p, pc->lci_d.p, pc->ldiag_d.p, pc->lu_d.p, pf, pb,            \
         pc->lev_ptr_f.p, pc->lev_ptr_b.p, pc->rec_off_f_d.p, pc->rec_off_b_d.p,             \
-        pc->rec_rows_f_d.p, pc->rec_rows_b_d.p, pc->rec_rows ? 1 : 0, pc->rec_d.p)
+        pc->rec_rows_f_d.p, pc->rec_rows_b_d.p, pc->rec_rows ? 1 : 0, pc->rec_d.p, pc->far_d.p)
     if (pc->opts.sweep_dtype == SG_FP64) SG_PACK(double);
     else if (pc->opts.factor_dtype == SG_BF16) SG_PACK(uint16_t);
     else SG_PACK(float);
 #undef SG_PACK
     SG_CUDA(cudaGetLastError());
+    if (!check) return true;
+    SG_CUDA(cudaMemcpyAsync(pc->far_h.p, pc->far_d.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SG_CUDA(cudaStreamSynchronize(st));
+    return *pc->far_h.p == 0;
 }
 
 // Packs the level records in the configured factor type, plans the
@@ -1341,37 +1370,38 @@ void rec_setup_device(sg_precond* pc, bool kept) {
     if (kept) {
         pc->err_d.zero(st);
         if (pc->coarse_sync.p) pc->coarse_sync.zero(st);
-        pack_records(pc);
-        return;
+        if (pack_records(pc)) return;
     }
     plan.R = 1;
     plan.ready = false;
     pc->ring4.ready = false;  // a new set-up plans the four-vector ring again when asked
     // records of row structs, unless their rings do not fit beside the vector
     // of a subdomain near the shared-memory limit (component records are
-    // smaller)
-    rec_layout(pc, true);
-    RingFit fit = ring_size(pc, plan);
-    if (fit.gmax.empty()) {
-        rec_layout(pc, false);
+    // smaller) or a diagonal needs the division (their rows divide)
+    RingFit fit;
+    pc->rec_divides = false;
+    for (bool rows = true;; rows = false) {
+        rec_layout(pc, rows);
         fit = ring_size(pc, plan);
+        if (fit.gmax.empty() && rows) continue;
+        if (fit.gmax.empty() || (pc->opts.reserved[0] & 1)) {
+            pc->use_rec = false;
+            return;
+        }
+        if (pc->rec_stage_bytes % 16 != 0 || pc->rec_total % 16 != 0)
+            fail(SG_ERR_INTERNAL, "level records are not 16-byte multiples");
+        pc->rec_depth = 1;
+        pc->rec_off_f_d.upload(pc->h_rec_off_f, st);
+        pc->rec_off_b_d.upload(pc->h_rec_off_b, st);
+        pc->rec_rows_f_d.upload(pc->h_rec_rows_f, st);
+        pc->rec_rows_b_d.upload(pc->h_rec_rows_b, st);
+        pc->rec_d.alloc((size_t)pc->rec_total);
+        pc->err_d.alloc(1);
+        if (!pc->err_h.p) pc->err_h.alloc(1);
+        pc->err_d.zero(st);
+        if (pack_records(pc)) break;
+        pc->rec_divides = true;
     }
-    if (fit.gmax.empty() || (pc->opts.reserved[0] & 1)) {
-        pc->use_rec = false;
-        return;
-    }
-    if (pc->rec_stage_bytes % 16 != 0 || pc->rec_total % 16 != 0)
-        fail(SG_ERR_INTERNAL, "level records are not 16-byte multiples");
-    pc->rec_depth = 1;
-    pc->rec_off_f_d.upload(pc->h_rec_off_f, st);
-    pc->rec_off_b_d.upload(pc->h_rec_off_b, st);
-    pc->rec_rows_f_d.upload(pc->h_rec_rows_f, st);
-    pc->rec_rows_b_d.upload(pc->h_rec_rows_b, st);
-    pc->rec_d.alloc((size_t)pc->rec_total);
-    pc->err_d.alloc(1);
-    if (!pc->err_h.p) pc->err_h.alloc(1);
-    pc->err_d.zero(st);
-    pack_records(pc);
     // block size (forced by opts.reserved[1], else timed), record-group size
     // and launch shape.  Levels of a 3D subdomain hold ~100+ rows, those of a
     // small 2D one ~20: a 512-thread block then idles at every level

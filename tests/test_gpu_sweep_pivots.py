@@ -50,3 +50,60 @@ def test_zeros_over_tiny_pivots(sg, oracle, width, threads):
     ref = oracle.precond("ras", A, 2, 0, part).apply(x)
     assert np.all(np.isfinite(ref))
     assert np.array_equal(y.view(np.uint64), np.asarray(ref).view(np.uint64))
+
+
+def _matrix(sg, width):
+    if width == 2:
+        return sg.make_poisson_2d(40, 33), (40, 33, 1)
+    if width == 3:
+        return sg.make_varcoef_3d(13, 11, 9, 1.0, 3.0, 1), (13, 11, 9)
+    return sg.make_aniso_2d(31, 37, 0.3, 0.6), (31, 37, 1)
+
+
+def _solve(sg, A, M, b, precision):
+    M.setup(A)
+    x = np.zeros(A.nrows)
+    r = sg.gmres(A, b, x, M, sg.GMRESParams(restart=20, max_iter=60, tol=1e-11, precision=precision,
+                                            tol_kind=sg.TOL_TRUE_REL))
+    return x, np.array(r.residual_history), r
+
+
+@pytest.mark.parametrize("width", [2, 3, 4])
+@pytest.mark.parametrize("threads", [0, 64, 256])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_solver_sweeps_divide(sg, width, threads, precision):
+    """The FP64 sweeps of a solve against those that divide row by row (the
+    sync-free ones): the same residual history and solution, bit for bit."""
+    A, g = _matrix(sg, width)
+    part = sg.partition_boxes(*g, 4, 0.1, seed=2)
+    b = sg.uniform(A.nrows, 5) - 0.5
+    p = sg.FP64 if precision == "fp64" else sg.FP32
+    M = sg.RASPrecond(4, 1, part, sweep_threads=threads)
+    x, h, _ = _solve(sg, A, M, b, p)
+    assert M.sweep_choice()["sweep"] == "tma"
+    y, k, _ = _solve(sg, A, sg.RASPrecond(4, 1, part, sweep="syncfree"), b, p)
+    assert np.array_equal(h, k) and np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("width", [2, 3, 4])
+def test_solve_with_tiny_pivots(sg, width):
+    """Pivots whose reciprocal overflows in systems whose right-hand side is
+    zero: the solve converges as it does when the sweeps divide; a set-up with
+    ordinary values after it, and back, computes what a new one does."""
+    A, rows = _blocks(sg, width)
+    part = (np.arange(A.nrows) * 2 // A.nrows).astype(np.int32)
+    b = sg.uniform(A.nrows, 5) - 0.5
+    b[rows] = 0.0
+    M = sg.RASPrecond(2, 0, part)
+    x, h, r = _solve(sg, A, M, b, sg.FP64)
+    assert r.converged and M.check() == 0 and M.sweep_choice()["sweep"] == "tma"
+    y, k, _ = _solve(sg, A, sg.RASPrecond(2, 0, part, sweep="syncfree"), b, sg.FP64)
+    assert np.array_equal(h, k) and np.array_equal(x, y)
+    tiny, v = A.vals, A.vals.copy()
+    v[np.abs(v) < 1e-200] = 4.0
+    for vals in (v, tiny):
+        A.vals = vals
+        A.upload()
+        x, h, _ = _solve(sg, A, M, b, sg.FP64)
+        y, k, _ = _solve(sg, A, sg.RASPrecond(2, 0, part), b, sg.FP64)
+        assert M.check() == 0 and np.array_equal(h, k) and np.array_equal(x, y)

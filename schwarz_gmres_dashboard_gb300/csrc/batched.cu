@@ -510,8 +510,8 @@ __device__ double b_arnoldi_end(const BatchDev& B, int inst, int j, const double
     const int m = B.m, ld = m + 1, lane = threadIdx.x & 31;
     double* Hc = B.H + (size_t)inst * ld * m + (size_t)j * ld;
     double* g = B.g + (size_t)inst * ld;
-    if (!(ss >= 1e-60)) {  // ||w''|| < 1e-30: breakdown
-        nrm = sqrt(ss);
+    nrm = sqrt(ss);
+    if (!(nrm >= 1e-30)) {  // breakdown
         __syncwarp();
         for (int i = lane; i <= j + 1; i += 32) Hc[i] = i <= j ? hc[i] : nrm;
         if (lane == 0) {
@@ -525,8 +525,7 @@ __device__ double b_arnoldi_end(const BatchDev& B, int inst, int j, const double
         }
         return 0.0;
     }
-    const double vs = rsqrt(ss);
-    nrm = ss * vs;
+    const double vs = 1.0 / nrm;
     const double g0 = g[j], g1 = g[j + 1], est = B.est[inst], bnorm = B.bnorm[inst];
     double c, s;
     rot_compute(c, s, a, nrm);

@@ -481,8 +481,7 @@ __device__ __forceinline__ bool cluster_reduce(double* partials, unsigned* count
 }
 
 // ----------------------------------------------------- least-squares update
-// Givens rotation of src/core/gmres.cpp:9-30 (1 / sqrt(1 + t^2) as one rsqrt:
-// one rounding less)
+// Givens rotation of src/core/gmres.cpp:9-30
 __device__ __forceinline__ void rot_compute(double& c, double& s, double a, double b) {
     if (fabs(b) < 1e-30) {
         c = 1.0;
@@ -491,7 +490,7 @@ __device__ __forceinline__ void rot_compute(double& c, double& s, double a, doub
     }
     const bool big = fabs(b) > fabs(a);
     const double t = -(big ? a : b) / (big ? b : a);
-    const double r = rsqrt(1.0 + t * t);
+    const double r = 1.0 / sqrt(1.0 + t * t);
     c = big ? r * t : r;
     s = big ? r : r * t;
 }

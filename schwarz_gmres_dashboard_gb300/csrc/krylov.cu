@@ -78,9 +78,9 @@ __device__ double finalize_warp(SolveState* st, const FinalizeIn& f, int j, int 
                                 double ss, double* hist, int hist_cap, double& nrm) {
     const int lane = threadIdx.x & 31;
     double* Hc = st->H + (size_t)j * (m + 1);
-    if (!(ss >= 1e-60)) {
-        // breakdown, ||w''|| < 1e-30 (src/core/gmres.cpp:297-300): this column is used as is
-        nrm = sqrt(ss);
+    nrm = sqrt(ss);
+    if (!(nrm >= 1e-30)) {
+        // breakdown (src/core/gmres.cpp:297-300): this column is used as is
         __syncwarp();
         for (int i = lane; i <= j + 1; i += 32) Hc[i] = i <= j ? f.hc[i] : nrm;
         if (lane == 0) {
@@ -94,8 +94,7 @@ __device__ double finalize_warp(SolveState* st, const FinalizeIn& f, int j, int 
         }
         return 0.0;
     }
-    const double vs = rsqrt(ss);
-    nrm = ss * vs;
+    const double vs = 1.0 / nrm;
     double c, sn;
     rot_compute(c, sn, a, nrm);
     const double g0 = f.gv[0], g1 = f.gv[1];

@@ -326,42 +326,11 @@ k_b_spmv_sell(BatchDev B, const long long* __restrict__ sl_ptr, const int* __res
     }
 }
 
-// The sums over a warp of four per-thread values at once, to FP64 accuracy:
-// each of the first two exchanges halves the values a lane holds, and the sum
-// of value (lane >> 3) ends in every lane of that eighth.  FP32 values are
-// added as unevaluated pairs (the first sum of two floats is exact, D. Knuth's
-// two-sum; pairs then lose less than 2^-44 of their sum, far below the FP32
-// products they add): ten FP32 instructions an addition, where an FP64
-// addition or conversion takes the SM 16 cycles a warp -- as FP64 shuffles
-// these sums took 2.5 times the vectors' load time.
-struct F2 {
-    float h, l;
-};
-__device__ __forceinline__ F2 two_sum(float a, float b) {
-    const float s = a + b, t = s - a;
-    return {s, (a - (s - t)) + (b - t)};
-}
-__device__ __forceinline__ F2 pair_add(F2 a, F2 b) {
-    const F2 s = two_sum(a.h, b.h);
-    const float l = s.l + (a.l + b.l);
-    const float h = s.h + l;
-    return {h, l - (h - s.h)};
-}
-__device__ __forceinline__ F2 pair_xor(F2 v, int o) {
-    return {__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)};
-}
-__device__ __forceinline__ double warp_sum4(const float* v) {
-    const int lane = threadIdx.x & 31;
-    const bool h1 = lane & 16, h2 = lane & 8;
-    const F2 a = two_sum(h1 ? v[2] : v[0], __shfl_xor_sync(0xffffffffu, h1 ? v[0] : v[2], 16));
-    const F2 b = two_sum(h1 ? v[3] : v[1], __shfl_xor_sync(0xffffffffu, h1 ? v[1] : v[3], 16));
-    const F2 give = h2 ? a : b;
-    F2 r = pair_add(h2 ? b : a, pair_xor(give, 8));
-    r = pair_add(r, pair_xor(r, 4));
-    r = pair_add(r, pair_xor(r, 2));
-    r = pair_add(r, pair_xor(r, 1));
-    return (lane & 7) == 0 ? (double)r.h + (double)r.l : 0.0;
-}
+// The sums over a warp of four per-thread values at once, in FP64: each of the
+// first two exchanges halves the values a lane holds, and the sum of value
+// (lane >> 3) ends in every lane of that eighth.  (A step's two passes over 64
+// systems of four right-hand sides: 215 us; 169 with the sums as pairs of
+// floats, which hold 48 bits of their largest term, not 53.)
 __device__ __forceinline__ double warp_sum4(const double* v) {
     const int lane = threadIdx.x & 31;
     const bool h1 = lane & 16, h2 = lane & 8;
@@ -378,7 +347,8 @@ __device__ __forceinline__ double warp_sum4(const double* v) {
 // red[warp][k0 + k] = the warp's sums of v[k], k < 4
 template <class TV>
 __device__ __forceinline__ void warp_red4(const TV* v, int k0, double (*red)[BLD]) {
-    const double s = warp_sum4(v);
+    const double d[4] = {(double)v[0], (double)v[1], (double)v[2], (double)v[3]};
+    const double s = warp_sum4(d);
     const int lane = threadIdx.x & 31;
     if ((lane & 7) == 0 && k0 + (lane >> 3) < BLD) red[threadIdx.x >> 5][k0 + (lane >> 3)] = s;
 }
@@ -685,8 +655,7 @@ k_b_lag_b(BatchDev B, TV* __restrict__ V, size_t ldv, int j) {
     pass_sums<TV, NV>(acc, red);
     __syncwarp();
     {  // ||w'||^2 next to the dots (j + 1 < BLD)
-        const TV sq[4] = {acc[NV], (TV)0, (TV)0, (TV)0};
-        const double s = warp_sum4(sq);
+        const double s = warp_sum((double)acc[NV]);
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][j + 1] = s;
     }
     __syncthreads();

@@ -66,7 +66,6 @@ struct BatchDev {
     double* sn;
     double* H;       // [I][(m+1) m], column-major, ld m+1
     double* vscale;  // [I][m+1]
-    float2* vsp;     // [I][m+1] the same as a pair of floats (vs_put)
     double* y;       // [I][m]
     float* yf;       // [I][m] y_k * vscale_k in FP32 (update of an FP32 basis)
     double* yd;      // [I][m] y_k * vscale_k in FP64
@@ -96,24 +95,6 @@ struct BatchDev {
 // chunk of the list, otherwise chunk b
 __device__ __forceinline__ int chunk_of(const BatchDev& B) {
     return B.clist ? B.clist[blockIdx.x] : (int)blockIdx.x;
-}
-
-// vscale of one basis vector, and the pair of floats whose sum it is to 2^-48
-__device__ __forceinline__ void vs_put(const BatchDev& B, size_t i, double vs) {
-    B.vscale[i] = vs;
-    const float h = (float)vs;
-    B.vsp[i] = make_float2(h, (float)(vs - (double)h));
-}
-// a * vscale rounded to the basis precision.  FP32: with the pair, within
-// 2^-23 of half a unit of the FP64 product's rounding, and no instruction on
-// the FP64 pipe (two conversions and a product there cost the SM 48 cycles a
-// warp)
-__device__ __forceinline__ float vs_mul(const BatchDev& B, size_t i, float a) {
-    const float2 p = B.vsp[i];
-    return fmaf(a, p.x, a * p.y);
-}
-__device__ __forceinline__ double vs_mul(const BatchDev& B, size_t i, double a) {
-    return a * B.vscale[i];
 }
 
 // Block sums of nv per-thread values (warp shuffles, then one pass over the
@@ -248,7 +229,7 @@ k_b_cycle_init(BatchDev B, const TV* __restrict__ raw0) {
         B.active[inst] = 0;
         return;
     }
-    vs_put(B, (size_t)inst * ld, 1.0 / beta);
+    B.vscale[(size_t)inst * ld] = 1.0 / beta;
     if (B.lagged) B.lagT[(size_t)inst * BLD * BLD] = 1.0 / beta;  // v_0 = raw_0 / beta
     B.g[(size_t)inst * ld] = beta;
     B.est[inst] = B.rnorm[inst] / beta;
@@ -271,7 +252,7 @@ k_b_spmv(BatchDev B, const int* __restrict__ rp, const int* __restrict__ ci,
         const TV* xb = x + (long long)rr * B.N;
         TV acc = (TV)0;
         for (int k = rp[mr]; k < rp[mr + 1]; ++k) acc += val[k] * xb[ci[k]];
-        y[q] = vs_mul(B, (size_t)inst * ld + j, acc);
+        y[q] = (TV)((double)acc * B.vscale[(size_t)inst * ld + j]);
     }
 }
 
@@ -321,7 +302,7 @@ k_b_spmv_sell(BatchDev B, const long long* __restrict__ sl_ptr, const int* __res
             for (int u = 0; u < BSR; ++u)
                 if (act[u])
                     y[(long long)(r0 + u) * B.N + row] =
-                        vs_mul(B, (size_t)((r0 + u) * B.S + sys) * ld + j, acc[u]);
+                        (TV)((double)acc[u] * B.vscale[(size_t)((r0 + u) * B.S + sys) * ld + j]);
         }
     }
 }
@@ -513,7 +494,7 @@ __device__ double b_arnoldi_end(const BatchDev& B, int inst, int j, const double
         B.sn[(size_t)inst * m + j] = s;
         g[j] = gj;
         g[j + 1] = gn;
-        vs_put(B, (size_t)inst * ld + j + 1, vs);
+        B.vscale[(size_t)inst * ld + j + 1] = vs;
         B.lastres[inst] = res;
         B.iters[inst] += 1;
         B.kcount[inst] = j + 1;
@@ -821,7 +802,6 @@ struct BatchWork {
     DBuf<int> clist, slist;
     std::vector<int> h_ich0, h_inch;
     DBuf<float> yf;
-    DBuf<float2> vsp;
     DBuf<unsigned> ticket;
     DBuf<double> b64, x64, r64;
     DBuf<float> V32, t32;
@@ -1104,7 +1084,6 @@ void solve_batched_device(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, int nsys
     dalloc(w->sn, (size_t)I * m);
     dalloc(w->H, I * ld * m);
     dalloc(w->vscale, I * ld);
-    dalloc(w->vsp, I * ld);
     dalloc(w->y, (size_t)I * m);
     dalloc(w->yd, (size_t)I * m);
     dalloc(w->yf, (size_t)I * m);
@@ -1150,7 +1129,7 @@ void solve_batched_device(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, int nsys
     B.active = w->active.p; B.done = w->done.p; B.conv = w->conv.p; B.iters = w->iters.p;
     B.cycles = w->cycles.p; B.kcount = w->kcount.p; B.ran = w->ran.p; B.flags = w->flags.p;
     B.bnorm = w->bnorm.p; B.rnorm = w->rnorm.p; B.est = w->est.p; B.lastres = w->lastres.p;
-    B.g = w->g.p; B.cs = w->cs.p; B.sn = w->sn.p; B.H = w->H.p; B.vscale = w->vscale.p; B.vsp = w->vsp.p;
+    B.g = w->g.p; B.cs = w->cs.p; B.sn = w->sn.p; B.H = w->H.p; B.vscale = w->vscale.p;
     B.y = w->y.p; B.yd = w->yd.p; B.yf = w->yf.p; B.h = w->h.p; B.hs = w->hs.p; B.ticket = w->ticket.p; B.part = w->part.p;
     B.notdone = w->notdone.p;
     B.lagT = w->lagT.p; B.lagH = w->lagH.p; B.lagc = w->lagc.p; B.cfu = w->cfu.p;

@@ -180,11 +180,27 @@ __device__ __forceinline__ int sell_col(const int16_t* col, long long e, int r, 
 // pipe the time of a full warp's: 720,000 rows of 2 to ~50 entries, 10
 // million in all, 185 us in k_spmv_csr, 76 here (8,192 rows 17 and 9).  Per row the order and the
 // rounding are the same.
+//
+// Of long rows a window holds few, and only their threads add.  Then a tile of
+// 32 rows a warp, as in k_spmv_csr, adds eight rows at a time -- on eight warps,
+// which the FP64 pipe serves in turn (16 cycles each, an addition's latency is
+// ~80), so the more blocks an SM has, the longer the rows may be: a block with
+// two long rows or more changes over where the mean length of an entry's row
+// (sum of squares / entries) exceeds uneven_turn, which lies between the two
+// columns below.  us by one way, the other, k_spmv_csr: 8,192 rows of 640
+// entries 1095, 1297, 1457; 3,000 of 1,000 2557, 2179, 2334; 8,192 of 384 on
+// geometric average 1409, 977, 1099; 256 of 40,000 385000, 96800, 97300; two
+// blocks an SM, 40,000 rows of 1,500 5833, 6793, 7051; three, 100,000 of 1,000
+// on average 6469, 7683, 8177.
+constexpr int UNEVEN_LONG = 256;
+int uneven_turn(int blocks, int num_sms) {
+    return 900 * std::min((blocks + num_sms - 1) / num_sms, 4) - 200;
+}
 template <class TV, class TX, class TY>
 __global__ void __launch_bounds__(SPMV_THREADS, 4)
 k_spmv_uneven(int n, const int* __restrict__ rp, const int* __restrict__ ci,
               const TV* __restrict__ val, const TX* __restrict__ x, TY* __restrict__ y,
-              const double* __restrict__ scale, const int* __restrict__ active) {
+              const double* __restrict__ scale, const int* __restrict__ active, int turn) {
     if (active && *active == 0) return;
     constexpr int VN = VecT<TV>::N, CAP = 4096, BINS = 64;
     using VV = typename VecT<TV>::V;
@@ -192,18 +208,56 @@ k_spmv_uneven(int n, const int* __restrict__ rp, const int* __restrict__ ci,
     __shared__ TV w[CAP];
     __shared__ int start[SPMV_THREADS + 1];
     __shared__ int bin[BINS];
+    __shared__ int longs;                   // rows of UNEVEN_LONG entries or more,
+    __shared__ unsigned long long squares;  // and the sum of their lengths' squares
     __shared__ unsigned char row_of[SPMV_THREADS];
     const int tid = threadIdx.x;
     const TV sc = scale ? (TV)(*scale) : (TV)1;
+    // the products of VN entries from e0 on, those in the window [ws, we)
+    auto products = [&](TV* win, int e0, int ws, int we) {
+        TV v[VN];
+        int c[VN];
+        unpack<TV, VV>(__ldg(reinterpret_cast<const VV*>(val + e0)), v);
+        unpacki(__ldg(reinterpret_cast<const VI*>(ci + e0)), c);
+#pragma unroll
+        for (int u = 0; u < VN; ++u) {
+            const int e = e0 + u;
+            if (e >= ws && e < we) win[e - ws] = pmul(v[u], (TV)__ldg(&x[c[u]]));
+        }
+    };
     for (int r0 = blockIdx.x * SPMV_THREADS; r0 < n; r0 += gridDim.x * SPMV_THREADS) {
         __syncthreads();  // the previous rows are done with
         start[tid] = __ldg(&rp[min(r0 + tid, n)]);
         if (tid == 0) start[SPMV_THREADS] = __ldg(&rp[min(r0 + SPMV_THREADS, n)]);
         if (tid < BINS) bin[tid] = 0;
+        if (tid == 0) longs = 0, squares = 0;
         __syncthreads();
-        const int len = min(start[tid + 1] - start[tid], BINS - 1);
+        const int mine = start[tid + 1] - start[tid], len = min(mine, BINS - 1);
         const int at = atomicAdd(&bin[len], 1);
+        if (mine >= UNEVEN_LONG) {
+            atomicAdd(&longs, 1);
+            atomicAdd(&squares, (unsigned long long)mine * mine);
+        }
         __syncthreads();
+        if (longs > 1 &&
+            squares > (unsigned long long)turn * (unsigned)(start[SPMV_THREADS] - start[0])) {
+            constexpr int WCAP = CAP / SPMV_WARPS;
+            const int lane = tid & 31, warp = tid >> 5;
+            TV* ww = w + warp * WCAP;
+            const int rs = start[tid], re = start[tid + 1], end = start[32 * warp + 32];
+            TV sum = (TV)0;
+            for (int ws = start[32 * warp]; ws < end; ws += WCAP) {
+                const int we = min(ws + WCAP, end);
+                for (int e0 = (ws & ~(VN - 1)) + lane * VN; e0 < we; e0 += 32 * VN)
+                    products(ww, e0, ws, we);
+                __syncwarp();
+                const int lo = max(rs, ws), hi = min(re, we);
+                for (int e = lo; e < hi; ++e) sum = padd(sum, ww[e - ws]);
+                __syncwarp();
+            }
+            if (r0 + tid < n) y[r0 + tid] = (TY)(scale ? pmul(sum, sc) : sum);
+            continue;
+        }
         if (tid < 32) {  // bins -> their first positions
             const int a = bin[2 * tid], b = bin[2 * tid + 1];
             int s = a + b;
@@ -224,17 +278,8 @@ k_spmv_uneven(int n, const int* __restrict__ rp, const int* __restrict__ ci,
         for (int ws = start[0]; ws < end; ws += CAP) {
             const int we = min(ws + CAP, end);
 #pragma unroll 2
-            for (int e0 = (ws & ~(VN - 1)) + tid * VN; e0 < we; e0 += SPMV_THREADS * VN) {
-                TV v[VN];
-                int c[VN];
-                unpack<TV, VV>(__ldg(reinterpret_cast<const VV*>(val + e0)), v);
-                unpacki(__ldg(reinterpret_cast<const VI*>(ci + e0)), c);
-#pragma unroll
-                for (int u = 0; u < VN; ++u) {
-                    const int e = e0 + u;
-                    if (e >= ws && e < we) w[e - ws] = pmul(v[u], (TV)__ldg(&x[c[u]]));
-                }
-            }
+            for (int e0 = (ws & ~(VN - 1)) + tid * VN; e0 < we; e0 += SPMV_THREADS * VN)
+                products(w, e0, ws, we);
             __syncthreads();
             const int lo = max(rs, ws), hi = min(re, we);
             for (int e = lo; e < hi; ++e) sum = padd(sum, w[e - ws]);
@@ -673,7 +718,8 @@ void launch_spmv_a(sg_ctx* ctx, const sg_csr* A, const TX* x, TY* y, const doubl
         const int blocks = (A->nrows + SPMV_THREADS - 1) / SPMV_THREADS;
         k_spmv_uneven<TV, TX, TY>
             <<<std::min(blocks, ctx->num_sms * 8), SPMV_THREADS, 0, ctx->stream>>>(
-                A->nrows, A->rp.p, A->ci.p, csr_vals<TV>(A), x, y, scale, active);
+                A->nrows, A->rp.p, A->ci.p, csr_vals<TV>(A), x, y, scale, active,
+                uneven_turn(blocks, ctx->num_sms));
         SG_CUDA(cudaGetLastError());
         count_launch(ctx);
     } else {

@@ -19,3 +19,55 @@ def test_bad_column_before_the_decrease(sg):
     A = sg.CSRMatrix(3, 8, np.array([0, 2, 900, 5], np.int32), np.array([0, 9, 1, 2, 3], np.int32), np.ones(5))
     with pytest.raises(sg.SgError, match=r"col_idx\[1\] = 9 outside \[0,8\)"):
         A.upload()
+
+
+@pytest.mark.parametrize("n", [2, 40, 1000])
+def test_sorted_rows_are_told_by_entry(sg, n):
+    """Only a decrease inside a row makes it unsorted (no SELL copy): not the
+    one from row to row, with empty rows between or none; and a column out of
+    range is named wherever it is."""
+    i = np.arange(n)
+    ci = np.stack([i * 0, i * 0 + n // 2, i * 0 + n - 1], 1)[:, :2 if n < 3 else 3].astype(np.int32)
+    w = ci.shape[1]
+    v = np.ones(ci.size)
+    for rp in (w * np.arange(n + 1), np.append(0, w * np.arange(1, n + 1))):
+        A = sg.CSRMatrix(n, n, rp.astype(np.int32), ci.ravel().copy(), v)
+        A.upload()
+        A.format = 2
+    for k in {0, n // 2, n - 1}:
+        bad = ci.copy()
+        bad[k] = bad[k][::-1]
+        if n > 2 or k == 0:
+            A = sg.CSRMatrix(n, n, (w * np.arange(n + 1)).astype(np.int32), bad.ravel(), v)
+            A.upload()
+            with pytest.raises(sg.SgError, match="no SELL copy"):
+                A.format = 2
+        far = ci.copy()
+        far[k, w - 1] = n
+        with pytest.raises(sg.SgError, match=rf"col_idx\[{k * w + w - 1}\] = {n} outside"):
+            sg.CSRMatrix(n, n, (w * np.arange(n + 1)).astype(np.int32), far.ravel(), v).upload()
+    # rows of one and two entries with empty rows between
+    rows = np.where(i % 3 == 0, 0, 1 + i % 2)
+    rp = np.concatenate([[0], np.cumsum(rows)]).astype(np.int32)
+    cc = np.concatenate([np.arange(k, dtype=np.int32) for k in rows])
+    sg.CSRMatrix(n, n, rp, cc, np.ones(cc.size)).upload()
+
+
+def test_upload_of_a_long_row(sg):
+    """A row of 3 million entries: its columns are checked at memory speed
+    (copies of 36 MB from pageable memory are ~4 ms; one entry after another
+    was 80)."""
+    import time
+
+    n = 50000
+    w = np.full(n, 5)
+    w[n // 2] = 3_000_000
+    rp = np.concatenate([[0], np.cumsum(w)]).astype(np.int32)
+    ci = np.zeros(rp[-1], np.int32)
+    A = sg.CSRMatrix(n, n, rp, ci, np.ones(ci.size))
+    best = np.inf
+    for _ in range(4):
+        t = time.perf_counter()
+        A.upload()
+        best = min(best, time.perf_counter() - t)
+    assert best < 0.03

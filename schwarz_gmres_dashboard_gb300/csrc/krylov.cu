@@ -199,14 +199,23 @@ constexpr int DOTS_PER_SM = 4, UPD_PER_SM = 3;  // resident blocks of the two pa
 // KPW per warp
 int warps_per_tile(int kc) { return kc <= KPW ? 1 : (kc <= 2 * KPW ? 2 : (kc <= 4 * KPW ? 4 : 8)); }
 
-// acc + a . b, one multiply-add per element (FP64 ones are the scarce resource)
-__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+// acc + a . b.  FP64: one multiply-add per element (the scarce resource).  FP32:
+// the four products by themselves first, then one addition to the sum -- four
+// at the sum's size double a dot's error (128^3: 2.0e-6 of a lane's terms, not
+// 1.1e-6) and save nothing, as the loads bound the pass.
 template <class TV>
-__device__ __forceinline__ TV dotv(const TV (&a)[Vec<TV>::N], const TV (&b)[Vec<TV>::N], TV acc) {
+__device__ __forceinline__ TV dotv(const TV (&a)[Vec<TV>::N], const TV (&b)[Vec<TV>::N], TV acc);
+template <>
+__device__ __forceinline__ double dotv<double>(const double (&a)[2], const double (&b)[2],
+                                               double acc) {
+    return fma(a[1], b[1], fma(a[0], b[0], acc));
+}
+template <>
+__device__ __forceinline__ float dotv<float>(const float (&a)[4], const float (&b)[4], float acc) {
+    float s = a[0] * b[0];
 #pragma unroll
-    for (int e = 0; e < Vec<TV>::N; ++e) acc = fma_t(a[e], b[e], acc);
-    return acc;
+    for (int e = 1; e < 4; ++e) s = fmaf(a[e], b[e], s);
+    return acc + s;
 }
 
 // the warp sums of four values at once: each of the first two exchanges halves

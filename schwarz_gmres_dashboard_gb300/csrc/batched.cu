@@ -574,7 +574,7 @@ __device__ __forceinline__ void load_T(const double* T, int j, double (*Tm)[BLD]
     for (int i = threadIdx.x >> 5; i <= j; i += BT / 32)
         if (lane <= j) {
             const double v = lane <= i ? T[lane + i * BLD] : 0.0;
-            if (Tm) Tm[i][lane] = v;
+            Tm[i][lane] = v;
             Tt[lane][i] = v;
         }
 }

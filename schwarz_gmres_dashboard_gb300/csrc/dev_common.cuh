@@ -302,21 +302,14 @@ __device__ __forceinline__ void scatter_owned(const TS* t, TO* __restrict__ y,
     }
 }
 
-// Grid-level completion of a reduction: every block stores its nv block sums
+// Grid-level completion of a reduction by blocks of at least nv warps: every
+// block stores its nv block sums
 // (bsum, smem) into partials[block*nv + k]; the last block to arrive sums
 // them in block order (deterministic) into smem `out` and returns true.  The
 // arrival counter is reset by the last block, so consecutive kernels on one
 // stream can share it.  No block waits for another.
-struct NoPrefetch {
-    __device__ __forceinline__ void operator()() const {}
-};
-// prefetch: run by the last block before it loads the partials (loads of
-// what its epilogue needs, so both rounds of loads are in flight together;
-// the results are visible to the block when this returns true)
-template <class Prefetch = NoPrefetch>
 __device__ __forceinline__ bool last_block_reduce(double* partials, unsigned* counter,
-                                                  const double* bsum, int nv, double* out,
-                                                  Prefetch prefetch = Prefetch()) {
+                                                  const double* bsum, int nv, double* out) {
     __shared__ unsigned s_ticket;
     for (int k = threadIdx.x; k < nv; k += blockDim.x)
         partials[(size_t)blockIdx.x * nv + k] = bsum[k];
@@ -326,51 +319,25 @@ __device__ __forceinline__ bool last_block_reduce(double* partials, unsigned* co
     __syncthreads();
     if (s_ticket != gridDim.x - 1) return false;
     __threadfence();
-    prefetch();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = gridDim.x;
     // per lane the partials are added in block order, as a plain loop would;
-    // the loads run ahead: sixteen per lane for one value per warp, else
-    // four values k = k0 + nw * kk per warp with four partials each
-    if (nv <= nw) {
-        if (warp < nv) {
-            double s = 0.0;
-            for (int b0 = lane; b0 < nb; b0 += 32 * 16) {
-                double v[16];
+    // the loads run ahead, sixteen per lane
+    if (warp < nv) {
+        double s = 0.0;
+        for (int b0 = lane; b0 < nb; b0 += 32 * 16) {
+            double v[16];
 #pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    const int b = b0 + 32 * r;
-                    v[r] = b < nb ? __ldcg(&partials[(size_t)b * nv + warp]) : 0.0;
-                }
-#pragma unroll
-                for (int r = 0; r < 16; ++r)
-                    if (b0 + 32 * r < nb) s += v[r];
+            for (int r = 0; r < 16; ++r) {
+                const int b = b0 + 32 * r;
+                v[r] = b < nb ? __ldcg(&partials[(size_t)b * nv + warp]) : 0.0;
             }
-            s = warp_sum(s);
-            if (lane == 0) out[warp] = s;
+#pragma unroll
+            for (int r = 0; r < 16; ++r)
+                if (b0 + 32 * r < nb) s += v[r];
         }
-    } else for (int k0 = warp; k0 < nv; k0 += 4 * nw) {
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int b0 = lane; b0 < nb; b0 += 32 * 4) {
-            double v[4][4];
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int b = b0 + 32 * r, k = k0 + nw * kk;
-                    v[kk][r] = (b < nb && k < nv) ? __ldcg(&partials[(size_t)b * nv + k]) : 0.0;
-                }
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    if (b0 + 32 * r < nb) s[kk] += v[kk][r];
-        }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            const double t = warp_sum(s[kk]);
-            if (lane == 0 && k0 + nw * kk < nv) out[k0 + nw * kk] = t;
-        }
+        s = warp_sum(s);
+        if (lane == 0) out[warp] = s;
     }
     __syncthreads();
     if (threadIdx.x == 0) *counter = 0u;

@@ -103,7 +103,7 @@ struct PinnedBuf {
 // --------------------------------------------------------------- solver state
 // Restart lengths up to SG_MMAX are supported.
 constexpr int SG_MMAX = 128;
-// restart lengths below SG_LAGM use the lagged CGS2 in the GMRES cycle
+// restart lengths below SG_LAGM use the lagged CGS2 (GMRES and FGMRES)
 constexpr int SG_LAGM = 32;
 
 // Device-resident Arnoldi / Givens state of one solve (FP64 throughout).
@@ -340,7 +340,7 @@ struct RingPlan {
     DBuf<unsigned char> sub_d;
     DBuf<int> ent_d, grp_d;
     DBuf<unsigned> work;       // persistent launches: next subdomain, CTAs done
-    std::map<const void*, int> resident;  // CTAs of a kernel that the GPU holds at once
+    mutable std::map<const void*, int> resident;  // CTAs of a kernel that the GPU holds at once
 };
 
 }  // namespace sg

@@ -1088,7 +1088,7 @@ void launch_tma(sg_precond* pc, const RingPlan& plan, const TI* x, TO* y, int mo
         // guaranteed by the cooperative launch (checked at set-up).  Where the
         // GPU holds more blocks than subdomains, the others take the
         // restrictions off the sweeping ones.
-        auto& cap = const_cast<RingPlan&>(plan).resident[reinterpret_cast<const void*>(kern)];
+        auto& cap = plan.resident[reinterpret_cast<const void*>(kern)];
         if (cap == 0) {
             int per_sm = 0;
             SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem));

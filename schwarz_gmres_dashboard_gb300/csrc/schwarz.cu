@@ -71,7 +71,13 @@ __global__ void k_gather_vals(long long nz, const int* __restrict__ map,
 // pivot rows are fetched and matched before the first division, so a level
 // costs three round trips and then only arithmetic; other rows fetch as they
 // go.  64 subdomains of 64^3, 52 levels: 0.63 ms before, 0.45 now.
-constexpr int FAC_T = 256;
+//
+// A level of more rows than threads takes several rounds, so a subdomain that
+// has an SM to itself takes FAC_T threads (one subdomain of 1600 x 1600, levels
+// of up to 1,600 rows: a set-up of 102 ms with half of them, 82 so); two blocks of
+// half the threads share one otherwise (1,000 subdomains of 128^3: 6.4 ms, 7.1
+// with whole ones).
+constexpr int FAC_T = 512;
 constexpr int FAC_W = 9;
 constexpr int FAC_L = 4;
 __device__ __forceinline__ void factor_row(int i, const int* __restrict__ rp,
@@ -98,12 +104,12 @@ __device__ __forceinline__ void factor_row(int i, const int* __restrict__ rp,
     }
 }
 
-template <class TC>
-__global__ void __launch_bounds__(FAC_T, 2)
+template <class TC, int T>
+__global__ void __launch_bounds__(T, FAC_T / T)
 k_factor(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
          const int* __restrict__ lci, const int* __restrict__ ldiag,
          const TC* __restrict__ perm_f, const int* __restrict__ lev_f, double* lu) {
-    __shared__ double s_v[FAC_W][FAC_T];  // each thread's row
+    __shared__ double s_v[FAC_W][T];  // each thread's row
     const SubInfo inf = info[blockIdx.x];
     const int* rp = lrp + inf.csr_row_off;
     const int* ci = lci + inf.csr_nz_off;
@@ -114,7 +120,7 @@ k_factor(const SubInfo* __restrict__ info, const int* __restrict__ lrp,
     const int tid = threadIdx.x;
     for (int l = 0; l < inf.nlev_f; ++l) {
         const int p0 = lf[l], p1 = lf[l + 1];
-        for (int p = p0 + tid; p < p1; p += FAC_T) {
+        for (int p = p0 + tid; p < p1; p += T) {
             const int i = pf[p];
             const int rs = rp[i], w = rp[i + 1] - rs;
             bool fast = w <= FAC_W;
@@ -1085,7 +1091,9 @@ void upload_structure(sg_precond* pc) {
 template <class TC>
 void factor_and_pack(sg_precond* pc, bool kept) {
     sg_ctx* ctx = pc->ctx;
-    k_factor<TC><<<pc->nparts, FAC_T, 0, ctx->stream>>>(
+    const bool whole = pc->nparts <= ctx->num_sms;
+    auto* factor = whole ? k_factor<TC, FAC_T> : k_factor<TC, FAC_T / 2>;
+    factor<<<pc->nparts, whole ? FAC_T : FAC_T / 2, 0, ctx->stream>>>(
         pc->info.p, pc->lrp_d.p, pc->lci_d.p, pc->ldiag_d.p,
         reinterpret_cast<const TC*>(pc->perm_f.p), pc->lev_ptr_f.p, pc->lu_d.p);
     SG_CUDA(cudaGetLastError());

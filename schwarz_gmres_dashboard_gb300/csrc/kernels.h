@@ -37,11 +37,12 @@ template <class TV>
 void launch_cycle_init(sg_ctx* ctx, const TV* raw0, int n, SolveState* st, int m, bool flexible);
 // One CGS2 Arnoldi step on raw[j+1] against raw[0..j] (with the Givens
 // update of the least-squares problem done by the last cluster); lagged: the
-// two-pass variant with the second projection carried to the next step
+// two-pass variant with the second projection carried to the next step, 1 for
+// GMRES, 2 for FGMRES
 // (st->lagged must be set for the whole solve, m < SG_LAGM).
 template <class TV>
 void launch_cgs2(sg_ctx* ctx, TV* raw, size_t ldv, int n, int j, int m, SolveState* st,
-                 bool lagged);
+                 int lagged);
 // y = H^{-1} g (k x k upper triangle) by one thread.
 void launch_backsolve(sg_ctx* ctx, SolveState* st, int m);
 // x += sum_k y_k * vscale_k * basis_k  (k < st->kcount)

@@ -73,9 +73,9 @@ __device__ __forceinline__ void finalize_load(FinalizeIn& f, const SolveState* s
 // One warp: completes Arnoldi step j from a = rotate_column and ss =
 // ||w''||^2: normalisation, the new rotation, residual estimate and stopping
 // test.  Returns the new vector's scale 1/||w''|| when the cycle goes on, 0
-// when it stops here (breakdown, convergence, last step); nrm = ||w''||.
+// when it stops here (breakdown, convergence, last step or asked to); nrm = ||w''||.
 __device__ double finalize_warp(SolveState* st, const FinalizeIn& f, int j, int m, double a,
-                                double ss, double* hist, int hist_cap, double& nrm) {
+                                double ss, double* hist, int hist_cap, double& nrm, bool last) {
     const int lane = threadIdx.x & 31;
     double* Hc = st->H + (size_t)j * (m + 1);
     nrm = sqrt(ss);
@@ -104,7 +104,7 @@ __device__ double finalize_warp(SolveState* st, const FinalizeIn& f, int j, int 
     // (which the restart verifies in FP64)
     const bool conv = f.tol_kind == SG_TOL_REF_ABS && res < f.tol;
     const bool bad = !isfinite(res);
-    const bool stop = conv || bad || j + 1 >= m ||
+    const bool stop = conv || bad || last || j + 1 >= m ||
                       (f.tol_kind == SG_TOL_TRUE_REL && res * f.est_scale <= 0.5 * f.tol * f.bnorm);
     if (lane == 0) {
         st->vscale[j + 1] = vs;
@@ -145,7 +145,7 @@ __device__ void arnoldi_finalize(SolveState* st, int j, int m, double ss, double
     if (threadIdx.x < 32) {
         double nrm;
         const double a = rotate_column(f.hc, f.csv, f.snv, st->H + (size_t)j * (m + 1), j);
-        finalize_warp(st, f, j, m, a, ss, hist, hist_cap, nrm);
+        finalize_warp(st, f, j, m, a, ss, hist, hist_cap, nrm, false);
     }
 }
 
@@ -331,11 +331,22 @@ __device__ void lagged_pass_a(SolveState* st, int j, const double* d, const LagI
 // pass B's end (all threads of that block; r = tot[0..j], ss =
 // ||w'||^2): h2 = T^T r, the column hsum + h2, its rotations (warp 0), the new
 // norm (warp 2), the step's end (warp 0), the new vector's pending correction
-// and T column (warp 1)
+// and T column (warp 1).
+//
+// A remainder below a tenth of w' (Kahan's and Parlett's "twice is enough", B. N.
+// Parlett, "The symmetric eigenvalue problem", 1980, 6.9) or below four
+// roundings of w is rounding itself: w lies in the span of the vectors before.
+// Left-preconditioned GMRES has converged then.  FGMRES need not have
+// (directions that repeat, a preconditioner of low rank), and to carry on from
+// the noise multiplies it by the correction's size at every step -- residuals of
+// 1e9 to 1e50 where three passes stay at 1.  So its cycle ends here: with this
+// column where its diagonal stands above the noise (w' is all of it), else
+// without.
 __device__ void lagged_pass_b(SolveState* st, int j, int m, const double* r, double ss,
-                              double* hist, int hist_cap, LagIn& in) {
+                              double* hist, int hist_cap, LagIn& in, bool flexible, double eps) {
     __shared__ double h2_s[SG_LAGM];
     __shared__ double s_vs, s_n2;
+    __shared__ int s_noise;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double a = 0.0, tc = 0.0;
     if (warp == 0) {
@@ -358,11 +369,24 @@ __device__ void lagged_pass_b(SolveState* st, int j, int m, const double* r, dou
         double nrm2 = ss - warp_sum(h2 * h2);
         if (!(nrm2 > 0.0)) nrm2 = isfinite(nrm2) ? 0.0 : nrm2;
         if (lane == 0) s_n2 = nrm2;
+        if (flexible) {
+            const double h = lane <= j ? in.f.hc[lane] : 0.0;
+            const double col = warp_sum(h * h);
+            if (lane == 0) s_noise = nrm2 < 0.01 * ss || nrm2 < 16.0 * eps * eps * col;
+        }
     }
     __syncthreads();
     if (warp == 0) {
-        double nrm;
-        const double vs = finalize_warp(st, in.f, j, m, a, s_n2, hist, hist_cap, nrm);
+        double nrm = 0.0, vs = 0.0;
+        const bool noise = flexible && s_noise;
+        if (noise && a * a <= 1e4 * ss) {
+            if (lane == 0) {
+                st->kcount = j;
+                st->cycle_active = 0;
+            }
+        } else {
+            vs = finalize_warp(st, in.f, j, m, a, s_n2, hist, hist_cap, nrm, noise);
+        }
         if (lane == 0) {
             st->lagH[j + 1 + j * SG_LAGM] = nrm;
             s_vs = j + 1 < SG_LAGM ? vs : 0.0;
@@ -636,7 +660,8 @@ k_upd_dots(const TV* __restrict__ raw, size_t ldv, int n, int nk, TV* __restrict
         cp_async_wait();
         __syncthreads();
         if (cluster_reduce(partials, counter, bs, nk + 1, tot))
-            lagged_pass_b(st, nk - 1, m, tot, tot[nk], hist, hist_cap, lag_in);
+            lagged_pass_b(st, nk - 1, m, tot, tot[nk], hist, hist_cap, lag_in, lagged == 2,
+                          sizeof(TV) == 8 ? 0x1p-53 : 0x1p-24);
         return;
     }
     if (cluster_reduce(partials, counter, bs, nk, tot)) {
@@ -1007,7 +1032,7 @@ static void dots_any(sg_ctx* ctx, const TV* raw, size_t ldv, int n, int nk, cons
 
 template <class TV>
 void launch_cgs2(sg_ctx* ctx, TV* raw, size_t ldv, int n, int j, int m, SolveState* st,
-                 bool lagged) {
+                 int lagged) {
     const int nk = j + 1;
     TV* w = raw + (size_t)(j + 1) * ldv;
     if (lagged) {
@@ -1015,7 +1040,7 @@ void launch_cgs2(sg_ctx* ctx, TV* raw, size_t ldv, int n, int j, int m, SolveSta
         if (m >= SG_LAGM || nk > KW * KPW) fail(SG_ERR_INTERNAL, "lagged CGS2 needs m < %d", SG_LAGM);
         dots_any<TV>(ctx, raw, ldv, n, nk, w, st, 0, 1);
         launch_clusters(ctx, tile_blocks<TV>(n, nk), upd_dots_kernel<TV>(nk), raw, ldv,
-                        n, nk, w, st, ctx->partials.p, ctx->counter.p, 1, m, ctx->hist_d,
+                        n, nk, w, st, ctx->partials.p, ctx->counter.p, lagged, m, ctx->hist_d,
                         ctx->hist_cap);
         return;
     }
@@ -1098,8 +1123,8 @@ void launch_cycle_end(sg_ctx* ctx, SolveState* st) {
 
 template void launch_cycle_init<double>(sg_ctx*, const double*, int, SolveState*, int, bool);
 template void launch_cycle_init<float>(sg_ctx*, const float*, int, SolveState*, int, bool);
-template void launch_cgs2<double>(sg_ctx*, double*, size_t, int, int, int, SolveState*, bool);
-template void launch_cgs2<float>(sg_ctx*, float*, size_t, int, int, int, SolveState*, bool);
+template void launch_cgs2<double>(sg_ctx*, double*, size_t, int, int, int, SolveState*, int);
+template void launch_cgs2<float>(sg_ctx*, float*, size_t, int, int, int, SolveState*, int);
 template void launch_update_x<double>(sg_ctx*, const double*, size_t, int, double*, SolveState*);
 template void launch_update_x<float>(sg_ctx*, const float*, size_t, int, double*, SolveState*);
 template void launch_copy<double, double>(sg_ctx*, const double*, double*, int, const int*);

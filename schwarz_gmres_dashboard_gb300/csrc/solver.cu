@@ -104,7 +104,8 @@ void apply_pc(sg_ctx* ctx, sg_precond* pc, const TI* x, TO* y, int n, const int*
 // not need a linear preconditioner: with the stored directions z_l = M raw_l
 // it is FGMRES with the directions Z T (the update takes them, x += Z T y),
 // for which A (Z T) = V H holds whatever M is; they differ from M v_j by the
-// second projection, a rounding-level change of M's argument.
+// second projection, a rounding-level change of M's argument while the vectors
+// are independent -- where they are not, lagged_pass_b ends the cycle.
 bool use_lagged(int m, int ortho) { return ortho == 0 && m < SG_LAGM; }
 
 // One restart cycle as a launch sequence on ctx->stream.
@@ -152,7 +153,7 @@ void enqueue_cycle(sg_ctx* ctx, const sg_csr* A, sg_precond* pc, const double* b
             launch_spmv_a<TV, TV, TV>(ctx, A, zj, wj, &st->vscale[j], active);
         }
         ClassTimer tm(ctx, TK_ORTHO);
-        launch_cgs2<TV>(ctx, V, ldv, n, j, m, st, lagged);
+        launch_cgs2<TV>(ctx, V, ldv, n, j, m, st, lagged ? (flexible ? 2 : 1) : 0);
     }
     {
         ClassTimer tm(ctx, TK_UPDATE);

@@ -73,9 +73,9 @@ __device__ __forceinline__ void finalize_load(FinalizeIn& f, const SolveState* s
 // One warp: completes Arnoldi step j from a = rotate_column and ss =
 // ||w''||^2: normalisation, the new rotation, residual estimate and stopping
 // test.  Returns the new vector's scale 1/||w''|| when the cycle goes on, 0
-// when it stops here (breakdown, convergence, last step or asked to); nrm = ||w''||.
+// when it stops here (breakdown, convergence, last step); nrm = ||w''||.
 __device__ double finalize_warp(SolveState* st, const FinalizeIn& f, int j, int m, double a,
-                                double ss, double* hist, int hist_cap, double& nrm, bool last) {
+                                double ss, double* hist, int hist_cap, double& nrm) {
     const int lane = threadIdx.x & 31;
     double* Hc = st->H + (size_t)j * (m + 1);
     nrm = sqrt(ss);
@@ -104,7 +104,7 @@ __device__ double finalize_warp(SolveState* st, const FinalizeIn& f, int j, int 
     // (which the restart verifies in FP64)
     const bool conv = f.tol_kind == SG_TOL_REF_ABS && res < f.tol;
     const bool bad = !isfinite(res);
-    const bool stop = conv || bad || last || j + 1 >= m ||
+    const bool stop = conv || bad || j + 1 >= m ||
                       (f.tol_kind == SG_TOL_TRUE_REL && res * f.est_scale <= 0.5 * f.tol * f.bnorm);
     if (lane == 0) {
         st->vscale[j + 1] = vs;
@@ -145,7 +145,7 @@ __device__ void arnoldi_finalize(SolveState* st, int j, int m, double ss, double
     if (threadIdx.x < 32) {
         double nrm;
         const double a = rotate_column(f.hc, f.csv, f.snv, st->H + (size_t)j * (m + 1), j);
-        finalize_warp(st, f, j, m, a, ss, hist, hist_cap, nrm, false);
+        finalize_warp(st, f, j, m, a, ss, hist, hist_cap, nrm);
     }
 }
 
@@ -336,12 +336,11 @@ __device__ void lagged_pass_a(SolveState* st, int j, const double* d, const LagI
 // A remainder below a tenth of w' (Kahan's and Parlett's "twice is enough", B. N.
 // Parlett, "The symmetric eigenvalue problem", 1980, 6.9) or below four
 // roundings of w is rounding itself: w lies in the span of the vectors before.
-// Left-preconditioned GMRES has converged then.  FGMRES need not have
-// (directions that repeat, a preconditioner of low rank), and to carry on from
-// the noise multiplies it by the correction's size at every step -- residuals of
-// 1e9 to 1e50 where three passes stay at 1.  So its cycle ends here: with this
-// column where its diagonal stands above the noise (w' is all of it), else
-// without.
+// Left-preconditioned GMRES has converged then, and so has FGMRES where the
+// column's diagonal stands above the noise (w' is all of it).  Else (directions
+// that repeat, a preconditioner of low rank) the column is noise too, and to
+// carry on multiplies it by the correction's size at every step -- residuals of
+// 1e9 to 1e50 where three passes stay at 1 -- so the cycle ends without it.
 __device__ void lagged_pass_b(SolveState* st, int j, int m, const double* r, double ss,
                               double* hist, int hist_cap, LagIn& in, bool flexible, double eps) {
     __shared__ double h2_s[SG_LAGM];
@@ -378,14 +377,13 @@ __device__ void lagged_pass_b(SolveState* st, int j, int m, const double* r, dou
     __syncthreads();
     if (warp == 0) {
         double nrm = 0.0, vs = 0.0;
-        const bool noise = flexible && s_noise;
-        if (noise && a * a <= 1e4 * ss) {
+        if (flexible && s_noise && a * a <= 1e4 * ss) {
             if (lane == 0) {
                 st->kcount = j;
                 st->cycle_active = 0;
             }
         } else {
-            vs = finalize_warp(st, in.f, j, m, a, s_n2, hist, hist_cap, nrm, noise);
+            vs = finalize_warp(st, in.f, j, m, a, s_n2, hist, hist_cap, nrm);
         }
         if (lane == 0) {
             st->lagH[j + 1 + j * SG_LAGM] = nrm;

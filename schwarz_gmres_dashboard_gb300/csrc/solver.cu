@@ -105,7 +105,7 @@ void apply_pc(sg_ctx* ctx, sg_precond* pc, const TI* x, TO* y, int n, const int*
 // it is FGMRES with the directions Z T (the update takes them, x += Z T y),
 // for which A (Z T) = V H holds whatever M is; they differ from M v_j by the
 // second projection, a rounding-level change of M's argument while the vectors
-// are independent -- where they are not, lagged_pass_b ends the cycle.
+// are independent -- before a column of noise lagged_pass_b ends the cycle.
 bool use_lagged(int m, int ortho) { return ortho == 0 && m < SG_LAGM; }
 
 // One restart cycle as a launch sequence on ctx->stream.

@@ -19,6 +19,17 @@ uint64_t next_object_gen() {
     static std::atomic<uint64_t> g{0};
     return ++g;
 }
+
+void allow_smem(sg_ctx* ctx, const void* kern) {
+    if (ctx->smem_allowed.count(kern)) return;
+    cudaFuncAttributes fa;
+    SG_CUDA(cudaFuncGetAttributes(&fa, kern));
+    int most = 0;
+    SG_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    SG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 most - (int)fa.sharedSizeBytes));
+    ctx->smem_allowed.insert(kern);
+}
 }  // namespace sg
 
 namespace sg {

@@ -950,8 +950,7 @@ void sweep_launch(sg_precond* pc, const TF* lval, const TF* uval, const TF* udia
     size_t smem = 0;
     if (pc->use_smem) {
         smem = ((size_t)(pc->max_n + 1) * sizeof(TS) + 15) & ~(size_t)15;
-        SG_CUDA(cudaFuncSetAttribute(k_sweep<TI, TO, TS, TF, TC>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_smem(ctx, k_sweep<TI, TO, TS, TF, TC>);
     }
     k_sweep<TI, TO, TS, TF, TC><<<pc->nparts, SWEEP_T, smem, ctx->stream>>>(
         pc->info.p, pc->order.p, pc->dofs.p, reinterpret_cast<const TC*>(pc->perm_f.p),
@@ -978,8 +977,7 @@ void sf_launch(sg_precond* pc, const TF* lval, const TF* uval, const TF* udiag, 
         !pc->owned_d.p || !pc->err_d.p || (coarse && (!pc->a0inv.p || !pc->r0.p)))
         fail(SG_ERR_INTERNAL, "preconditioner device buffers missing for this apply");
     const size_t smem = sf_smem(pc);
-    SG_CUDA(cudaFuncSetAttribute(k_sweep_sf<TI, TO, TS, TF, TC, EXACT>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ctx, k_sweep_sf<TI, TO, TS, TF, TC, EXACT>);
     k_sweep_sf<TI, TO, TS, TF, TC, EXACT><<<pc->nparts, SWEEP_T, smem, ctx->stream>>>(
         pc->info.p, pc->order.p, pc->dofs.p, reinterpret_cast<const TC*>(pc->perm_f.p),
         reinterpret_cast<const TC*>(pc->lcol.p), lval, reinterpret_cast<const TC*>(pc->perm_b.p),
@@ -1042,8 +1040,7 @@ void dense_lu(sg_ctx* ctx, int n, double* A, int* piv, int* status) {
     // static scratch and the block's own kilobyte beside the panel; a panel of
     // more rows works in global memory
     const size_t room = (size_t)max_smem - 2048;
-    SG_CUDA(cudaFuncSetAttribute(k_lu_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)room));
+    allow_smem(ctx, k_lu_panel);
     for (int k0 = 0; k0 < n; k0 += LU_NB) {
         const int nb = std::min(LU_NB, n - k0), rest = n - k0 - nb;
         const size_t smem = (size_t)(n - k0) * LU_LD * sizeof(double);
@@ -1187,8 +1184,7 @@ void precond_setup_device(sg_precond* pc, const sg_csr* A) {
         reserve(pc->status_d, 1);
         pc->status_d.zero(st);
         const size_t smem = (size_t)nc * (4 + 4);
-        SG_CUDA(cudaFuncSetAttribute(k_a0_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
+        allow_smem(ctx, k_a0_build);
         reserve(pc->a0_own, (size_t)n);
         reserve(pc->a0_rows, (size_t)n);
         k_a0_build<<<nc, A0_T, smem, st>>>(nc, pc->owned_ptr_d.p, pc->owned_d.p, A->rp.p, A->ci.p,
@@ -1203,8 +1199,7 @@ void precond_setup_device(sg_precond* pc, const sg_csr* A) {
         SG_CUDA(cudaStreamSynchronize(st));
         if (bad) fail(SG_ERR_SINGULAR, "Coarse matrix is singular");
         const size_t smem2 = (size_t)nc * 8;
-        SG_CUDA(cudaFuncSetAttribute(k_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem2));
+        allow_smem(ctx, k_inv);
         k_inv<<<nc, 256, smem2, st>>>(nc, pc->lu0.p, pc->piv0.p, pc->a0inv.p);
         SG_CUDA(cudaGetLastError());
     }

@@ -862,7 +862,7 @@ bool build_schwarz_device(sg_precond* pc, const sg_csr* A, const int* part_in, i
     int max_ns = 0;
     for (int s = 0; s < P; ++s) max_ns = std::max(max_ns, sptr[s + 1] - sptr[s]);
     const size_t lv_smem = sizeof(int) * (size_t)std::min(max_ns, lv_smem_rows);
-    SG_CUDA(cudaFuncSetAttribute(k_levels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lv_smem));
+    allow_smem(ctx, k_levels);
     k_levels<<<P, LV_T, lv_smem, st>>>(la, lv_smem_rows);
     SG_CUDA(cudaGetLastError());
     std::vector<int> nlev;
@@ -891,8 +891,7 @@ bool build_schwarz_device(sg_precond* pc, const sg_csr* A, const int* part_in, i
     for (int t = 0; t < 2 * P; ++t) max_nl = std::max(max_nl, nlev[t]);
     const int lo_smem_levels = 16 * 1024;
     const size_t lo_smem = sizeof(int) * (size_t)std::min(max_nl, lo_smem_levels);
-    SG_CUDA(cudaFuncSetAttribute(k_level_order, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)std::max<size_t>(lo_smem, 4)));
+    allow_smem(ctx, k_level_order);
     k_level_order<<<2 * P, LV_T, std::max<size_t>(lo_smem, 4), st>>>(
         d_sptr.p, d_lev_lo.p, d_lev_up.p, d_loff_f.p, d_loff_b.p, d_nlev.p, P, d_ptr_f.p,
         d_ptr_b.p, d_perm_f.p, d_perm_b.p, lo_smem_levels);

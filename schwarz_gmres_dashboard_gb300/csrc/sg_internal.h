@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -196,6 +197,7 @@ struct sg_ctx {
     sg::DBuf<unsigned int> counter;
     // clusters of a reducing kernel that this device holds at once, by kernel
     std::map<const void*, int> max_clusters;
+    std::set<const void*> smem_allowed;  // kernels seen by allow_smem
     // residual history of the running solve (device)
     sg::DBuf<double> hist;
     double* hist_d = nullptr;
@@ -237,6 +239,13 @@ void collect_timers(sg_ctx* ctx);
 // process-wide increasing generation numbers of matrices, preconditioners and
 // learned stages (a recycled address never repeats a generation)
 uint64_t next_object_gen();
+// Lets a kernel use as much dynamic shared memory as the device gives a block
+// beside its static part.  The limit belongs to the process: set to each
+// launch's own size, a thread with another context could lower it between
+// this thread's call and its launch.
+void allow_smem(sg_ctx* ctx, const void* kern);
+template <class K>
+void allow_smem(sg_ctx* ctx, K* kern) { allow_smem(ctx, reinterpret_cast<const void*>(kern)); }
 inline void count_launch(sg_ctx* ctx) {
     if (ctx->capturing) ctx->captured++;
     else ctx->launches++;

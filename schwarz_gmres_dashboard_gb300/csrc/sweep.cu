@@ -1079,7 +1079,7 @@ void launch_tma(sg_precond* pc, const RingPlan& plan, const TI* x, TO* y, int mo
     if constexpr (sizeof(TS) == 4) {
         if (a.persist) kern = k_sweep_tma<TI, TO, TS, TF, EXACT, R, true>;
     }
-    SG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(pc->ctx, kern);
     a.ldx = ldx;
     a.ldy = ldy;
     const int coarse_i = coarse ? 1 : 0;
@@ -1256,7 +1256,7 @@ static int sweep_occupancy(sg_precond* pc, const RingPlan& plan, K kern) {
     const size_t smem = sweep_smem(pc, plan);
     const int nt = plan.threads > 0 ? plan.threads : SW_T;
     int per_sm = 0;
-    SG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(pc->ctx, kern);
     SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem));
     return per_sm;
 }
